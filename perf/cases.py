@@ -3,9 +3,9 @@ and portions of prompts, through ``LLMEngine``'s model (``runner.decoder.forward
 that the engine's benchmark and tests run: NVFP4 weights with an fp8 cache, bf16 throughout, FP8 block weights in a
 hybrid of gated delta net, gated attention and experts.
 
-Models have the layer sizes of the presets and two layers of them, behind an 8192-word vocabulary, so that the layers
-have about the share of a pass that they have in a whole model. As in the engine, a step of one or a few tokens per
-sequence is replayed from a CUDA graph over fixed buffers, and prompts run eagerly.
+Models have the layer sizes of the presets and one or two layers of them, behind a vocabulary cut as much, so that the
+layers have about the share of a pass that they have in a whole model. As in the engine, a step of one or a few tokens
+per sequence is replayed from a CUDA graph over fixed buffers, and prompts run eagerly.
 """
 from __future__ import annotations
 
@@ -13,10 +13,12 @@ import math
 
 import torch
 
-LAYERS, VOCAB, BLOCK = 2, 8192, 16
-#: standard deviation of the weights, and of those whose outputs join the residual stream: theirs is divided by the root of
-#: the number of sublayers of the whole model, as deep models are initialised, so that no layer drowns the stream
-STD, STD_OUT = 0.02, 0.02 / 128 ** 0.5
+#: one layer where activations are four bits wide: behind a second one a last-bit difference in the first has become a
+#: step of the quantisers in so many places that no two correct results are alike
+LAYERS, VOCAB, BLOCK = {"nvfp4": 1, "bf16": 2, "hybrid-fp8": 2}, 2048, 16
+#: standard deviation of the weights, of those whose outputs join the residual stream (divided by the root of the number of
+#: sublayers of the whole model, as deep models are initialised), and of the stream that the layers find
+STD, STD_OUT, STD_STREAM = 0.02, 0.02 / 128 ** 0.5, 2.0
 
 
 # ----------------------------------------------------------------------------- cases
@@ -91,10 +93,10 @@ def _lengths(c):
 def _config(model):
     from metrale_inference_alpha_b200.config.model_config import preset
     if model == "hybrid-fp8":
-        return preset("qwen-hybrid-moe-35b-fp8", num_layers=LAYERS, layer_types=["gdn", "attention"], ffn_types=["moe"] * LAYERS,
-                      vocab_size=VOCAB)
+        return preset("qwen-hybrid-moe-35b-fp8", num_layers=LAYERS[model], layer_types=["gdn", "attention"],
+                      ffn_types=["moe"] * LAYERS[model], vocab_size=VOCAB)
     kw = dict(weight_format="bf16", kv_dtype="bf16") if model == "bf16" else {}
-    return preset("dense-27b-nvfp4", num_layers=LAYERS, vocab_size=VOCAB, mtp_layers=0, **kw)
+    return preset("dense-27b-nvfp4", num_layers=LAYERS[model], vocab_size=VOCAB, mtp_layers=0, **kw)
 
 
 _E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
@@ -130,7 +132,7 @@ class _Checkpoint:
         self.g = torch.Generator(device=device).manual_seed(seed)
         self.device, c = device, self.cfg
         H = c.hidden_size
-        self.plain("model.embed_tokens", VOCAB, H, std=1.0)
+        self.plain("model.embed_tokens", VOCAB, H, std=STD_STREAM)
         self.plain("lm_head", VOCAB, H)
         self.norm("model.norm", H)
         for i, kind in enumerate(c.layer_types):
@@ -323,7 +325,7 @@ def work(c):
 def tolerance(c):
     # Quantised activations turn a last-bit difference into a step of their grid now and then: sums in another order give
     # a few per cent on an e2m1 grid, a few tenths of one on e4m3.
-    return {"rel": {"nvfp4": 0.1, "bf16": 0.01, "hybrid-fp8": 0.02}[c["model"]]}
+    return {"rel": {"nvfp4": 0.03, "bf16": 0.01, "hybrid-fp8": 0.02}[c["model"]]}
 
 
 # ----------------------------------------------------------------------------- the same pass in 64 bits
