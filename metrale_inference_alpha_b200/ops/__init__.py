@@ -29,8 +29,8 @@ OUT_MODE = {"bf16": 0, "fp8_row": 1, "fp8_g128": 2, "nvfp4": 3}
 launch_count = 0  # kernels launched through this module (bench.py reports it)
 # kernel-selection bits of the GEMM launcher (csrc/gemm_args.h)
 GEMM_ONE_TILE_PER_CTA, GEMM_DECODE_TILE_ORDER, GEMM_PERSISTENT_PREFILL, GEMM_DSMEM_SPLITK = 16, 64, 128, 256
-# prefill GEMMs (several 128-token tiles) also run on the persistent kernel (NVFP4 prefill GEMMs
-# measure 1.5x faster there; METRALE_PERSISTENT_PREFILL=0 keeps one tile per CTA)
+# GEMMs of more than 128 token rows run on the persistent kernel of CTA pairs (csrc/gemm_rows.cu; METRALE_PERSISTENT_PREFILL=0
+# keeps one tile per CTA)
 _PERSIST_PREFILL = GEMM_PERSISTENT_PREFILL if os.environ.get("METRALE_PERSISTENT_PREFILL", "1") != "0" else 0
 GEMM_GROUPED_ONE_CTA = 512
 EPI_SWIGLU, EPI_CLAMP_GLU, EPI_SILU_COLS, EPI_NEG_EXP, EPI_GEGLU, EPI_BIAS, EPI_LOG_SIGMOID, EPI_RELU2, EPI_SIGMOID = 1, 2, 3, 4, 5, 6, 7, 8, 9      # csrc/epilogue.cuh
@@ -505,8 +505,10 @@ def linear(act: Act, w: QuantWeight, *, residual: Optional[torch.Tensor] = None,
         return quantize_act(y, "nvfp4", static_scale=quant_out) if quant_out > 0.0 else y
     if quant_out > 0.0:
         assert swiglu and residual is None and not out_f32 and grouped is None
-        fused = (act.data.is_cuda and M <= 128 and (N + 127) // 128 > runtime(act.data.device).sm_count
-                 and w.fmt in ("nvfp4", "fp8_row", "bf16") and (N // 2) % 256 == 0 and not one_tile_per_cta)
+        decode = M <= 128 and act.data.is_cuda and (N + 127) // 128 > runtime(act.data.device).sm_count
+        rows = M > 128 and _PERSIST_PREFILL and not (force_tn or force_splits or no_cluster or decode_tile_order)      # csrc/gemm_rows.cu
+        fused = (act.data.is_cuda and (decode or rows) and w.fmt in ("nvfp4", "fp8_row", "bf16") and (N // 2) % 256 == 0
+                 and not one_tile_per_cta)
         if not fused:
             y = linear(act, w, swiglu=True, out_f32=not act.data.is_cuda, force_tn=force_tn, force_splits=force_splits,
                        one_tile_per_cta=one_tile_per_cta)

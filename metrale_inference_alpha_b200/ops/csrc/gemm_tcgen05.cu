@@ -35,6 +35,7 @@
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "gemm_args.h"
+#include "gemm_rows.h"
 #include <mutex>
 #include "tensormap.h"
 #include "noalloc.h"
@@ -653,7 +654,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
 // ------------------------------------------------------------------------------------------
 // Persistent variant for layers with more weight-row tiles than SMs (gate_up, lm_head) and one
-// token tile (M <= 128): every CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... with the
+// token tile (M <= 128; more rows take gemm_rows.cu): every CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... with the
 // stage ring running across tile boundaries and two TMEM accumulators, so the epilogue of tile i
 // (TMEM -> registers -> global, no shared-memory staging) overlaps the main loop of tile i + 1
 // and the weight stream never pauses. Same operand kinds except the 128x128-block fp8 kind.
@@ -689,14 +690,12 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   __shared__ __align__(8) uint64_t acc_full[2];
   __shared__ __align__(8) uint64_t acc_empty[2];
   __shared__ uint32_t tmem_base_s;
-  __shared__ __align__(8) float s_ascale[2][TN];
+  __shared__ __align__(8) float s_ascale[TN];
 
   const int warp = threadIdx.x >> 5;
   const int n_tiles = (p.N + kTileN - 1) / kTileN;
-  const int m_tiles = (p.M + TN - 1) / TN;               // 1 for decode; prefill walks token tiles fastest
   const int nkb = p.num_kb;
-  // work item t = blockIdx.x + i * gridDim.x covers weight tile t / m_tiles and token tile t % m_tiles
-  const int my_tiles = (n_tiles * m_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // grid <= tiles
+  const int my_tiles = (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // grid <= tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -728,23 +727,21 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     // ------------------------------------------------------------ producer
     if (mb::elect_one()) {
       const int total = my_tiles * nkb;                   // k blocks this CTA streams, over all its tiles
-      // both streams are issued in increasing g: the (work item, k block) cursors advance
-      // incrementally, with one division per work item instead of several per k block
-      int w_kb = 0, w_item = (int)blockIdx.x, w_tile = w_item / m_tiles;
+      // both streams are issued in increasing g: the (tile, k block) cursors advance incrementally
+      int w_kb = 0, w_tile = (int)blockIdx.x;
       auto load_w = [&](int g) {
         const int s = g % kStages;
         mb::tma_load_2d(sA(s), &tmA, &full_bar[s], w_kb * kCoordStep, w_tile * kTileN);
         if constexpr (KIND == KIND_NVFP4)
           mb::bulk_load(sSFA(s), p.sfa + ((size_t)w_tile * p.sf_k64 + (size_t)w_kb * 4) * 512, 2048, &full_bar[s]);
-        if (++w_kb == nkb) { w_kb = 0; w_item += (int)gridDim.x; w_tile = w_item / m_tiles; }
+        if (++w_kb == nkb) { w_kb = 0; w_tile += (int)gridDim.x; }
       };
-      int x_kb = 0, x_item = (int)blockIdx.x, x_mt = x_item % m_tiles;
+      int x_kb = 0;
       auto load_x = [&](int g) {
         const int s = g % kStages;
-        mb::tma_load_2d(sB(s), &tmB, &full_bar[s], x_kb * kCoordStep, x_mt * TN);
-        if constexpr (KIND == KIND_NVFP4)
-          mb::bulk_load(sSFB(s), p.sfb + ((size_t)((x_mt * TN) / 128) * p.sf_k64 + (size_t)x_kb * 4) * 512, 2048, &full_bar[s]);
-        if (++x_kb == nkb) { x_kb = 0; x_item += (int)gridDim.x; x_mt = x_item % m_tiles; }
+        mb::tma_load_2d(sB(s), &tmB, &full_bar[s], x_kb * kCoordStep, 0);
+        if constexpr (KIND == KIND_NVFP4) mb::bulk_load(sSFB(s), p.sfb + (size_t)x_kb * 4 * 512, 2048, &full_bar[s]);
+        if (++x_kb == nkb) x_kb = 0;
       };
       const int pre = min(total, kStages);
       for (int g = 0; g < pre; ++g) {                     // weights do not depend on the preceding kernel
@@ -830,24 +827,20 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const float outq_inv6gs = p.outq ? 1.f / (6.f * p.outq_gs) : 0.f;
     bool ok = true;
     for (int it = 0; it < my_tiles && ok; ++it) {
-      const int t_lin = (int)blockIdx.x + it * (int)gridDim.x;
-      const int tile = t_lin / m_tiles;
-      const int m_base = (t_lin % m_tiles) * TN;           // first token row of this tile
-      const int m_valid = min(p.M - m_base, TN);
+      const int tile = (int)blockIdx.x + it * (int)gridDim.x;
+      const int m_valid = min(p.M, TN);
       const int buf = it & 1;
-      if (it == 0 || m_tiles > 1) {
-        // per-token activation scales of this token tile. Two buffers and one barrier per tile:
-        // nobody can be two tiles ahead of a thread that has not passed the barrier in between.
+      if (it == 0) {                                       // per-token activation scales
         for (int j = et; j < TN; j += kPersistThreads - 64) {
           float sc = 1.f;
           if constexpr (KIND == KIND_FP8 || KIND == KIND_NVFP4) {
-            if (p.a_scale && j < m_valid) sc = __ldg(&p.a_scale[m_base + j]);
+            if (p.a_scale && j < m_valid) sc = __ldg(&p.a_scale[j]);
           }
-          s_ascale[buf][j] = sc;
+          s_ascale[j] = sc;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kPersistThreads - 64) : "memory");
       }
-      const float* asc = s_ascale[m_tiles > 1 ? buf : 0];
+      const float* asc = s_ascale;
       ok = mb::mbar_wait(&acc_full[buf], (it >> 1) & 1, p.status, MB_ST_TIMEOUT_EPI);
       if (!ok) break;
       mb::tc_fence_after();
@@ -874,8 +867,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             const float other = __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1);
             const float gate = odd ? other : x0, up = odd ? x1 : other;
             const float y = clamp_glu ? mb::clamp_glu_fast(gate, up, p.epi_a, p.epi_b) : geglu ? mb::geglu_fast(gate, up) : mb::silu(gate) * up;
-            const int ml = m0 + (odd ? 1 : 0);                 // row inside the tile
-            const int m = m_base + ml;
+            const int m = m0 + (odd ? 1 : 0);
             if (p.outq) {
               // This warp's 16 even lanes hold one 16-wide quantisation block of token m0, its odd
               // lanes the same block of token m0 + 1 (block index along the consumer's K: tile * 4 + q).
@@ -893,13 +885,13 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
               const float upper = __shfl_down_sync(0xffffffffu, scaled, 2);
               const uint32_t byte = mb::e2m1x2_pack(scaled, upper);
               const int i = lane >> 1;                      // output index inside the block
-              if (ml < m_valid && !(i & 1) && n < p.N)
+              if (m < m_valid && !(i & 1) && n < p.N)
                 p.outq[(size_t)m * p.ldq + ((tile * 64 + q * 16 + i) >> 1)] = (uint8_t)byte;
-              if (ml < m_valid && i == 0 && n < p.N) {
+              if (m < m_valid && i == 0 && n < p.N) {
                 const int kb = tile * 4 + q;
                 p.outq_sf[((size_t)(m >> 7) * p.outq_sf_k64 + (kb >> 2)) * 512 + mb::sf_tile_offset(m & 127, kb & 3)] = sfc;
               }
-            } else if (n_ok && ml < m_valid) {
+            } else if (n_ok && m < m_valid) {
               outp[(size_t)m * p.ldo] = __float2bfloat16(y);
             }
           }
@@ -929,10 +921,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           }
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const int ml = c * 16 + j;
-            if (ml < m_valid && n < p.N) {
-              float y = v[j] * wsc * asc[ml];
-              const size_t o = (size_t)(m_base + ml) * p.ldo + n;
+            const int m = c * 16 + j;
+            if (m < m_valid && n < p.N) {
+              float y = v[j] * wsc * asc[m];
+              const size_t o = (size_t)m * p.ldo + n;
               if (p.residual) y += __bfloat162float(p.residual[o]);
               if (p.out_f32) reinterpret_cast<float*>(p.out)[o] = y;
               else reinterpret_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16(y);
@@ -1070,6 +1062,7 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
   const int tiles_m = grouped ? a->max_tiles : (a->M + tn - 1) / tn;
   if (kind == KIND_FP8_BLOCK && !grouped && a->a_ld < tiles_m * tn) return MB_ERR_BAD_ARG;
   if (kind == KIND_FP8_BLOCK && grouped && a->a_ld < a->M + tn) return MB_ERR_BAD_ARG;
+  if (mb_gemm_rows_serves(a)) return mb_gemm_rows(a, tn, stream);
   // scale-factor tiles are 128 rows: several token tiles only line up at TN = 128
   if (kind == KIND_NVFP4 && !grouped && tiles_m > 1 && tn != 128) return MB_ERR_BAD_ARG;
   const int tiles = tiles_n * tiles_m;
@@ -1139,11 +1132,9 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
   p.m_fastest = (!grouped && tiles_m >= 8 && tiles_m <= 65535 && tiles_n <= 65535 && !(a->flags & MB_GEMM_DECODE_TILE_ORDER)) ? 1 : 0;
   dim3 grid(p.m_fastest ? tiles_m : tiles_n, p.m_fastest ? tiles_n : tiles_m, splits);
   rc = MB_ERR_UNSUPPORTED;
-  // more tiles than SMs: persistent CTAs, balanced tile counts. One token tile (decode) always;
-  // several token tiles (prefill, 128-token tiles) when MB_GEMM_PERSISTENT_PREFILL asks for it.
-  const bool multi_m_ok = tiles_m > 1 && tn == 128 && (a->flags & MB_GEMM_PERSISTENT_PREFILL) && !a->outq;
-  if (!grouped && splits == 1 && (tiles_m == 1 || multi_m_ok) && tn <= 128 && kind != KIND_FP8_BLOCK &&
-      tiles > sms && (tiles_m > 1 || tiles_n > sms) && !(a->flags & MB_GEMM_ONE_TILE_PER_CTA)) {
+  // one token tile and more weight tiles than SMs: persistent CTAs, balanced tile counts
+  if (!grouped && splits == 1 && tiles_m == 1 && tn <= 128 && kind != KIND_FP8_BLOCK && tiles > sms &&
+      !(a->flags & MB_GEMM_ONE_TILE_PER_CTA)) {
     const int waves = (tiles + sms - 1) / sms;
     const int grid_x = (tiles + waves - 1) / waves;
     switch (kind) {
