@@ -14,6 +14,13 @@
 // Measured (B200, 8192 tokens; before = 128 x 128 tiles of one CTA): NVFP4 7168 x 5120 228 -> 139 us, 34816 x 5120 with
 // SwiGLU 990 -> 570 us (5.1 PFLOP/s), 5120 x 17408 499 -> 302 us; bf16, 2532 tokens: 34816 x 5120 708 -> 567 us (1.5 PFLOP/s,
 // under the power cap). The SwiGLU result leaves as NVFP4 from here too: the 134 us quantiser pass over 8192 x 17408 is gone.
+//
+// gemm_block_kernel (fp8 with 128 x 128 weight scales, also over the work list of grouped experts): one CTA per tile of
+// 128 tokens x 128 features. Every 128-deep k block lands in one of four TMEM accumulators and is added to registers
+// with its scale, which is one number per thread here (the token's scale times the weight block's). Small work-list entries
+// load boxes of their own 16 to 64 rows: the rest of the tile's rows are whatever was there, and are not stored.
+// Measured (2724 tokens x 8 of 256 experts and a shared one; before = 64-token tiles as the UMMA "B" operand): 1024 x 2048 per
+// expert 500 -> 167 us, 2048 x 512 417 -> 144 us, plain 8192 x 2048 237 -> 82 us; 16 tokens (rows of 16): 52 -> 51, 48 -> 40 us.
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "gemm_rows.h"
@@ -387,6 +394,167 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// ------------------------------------------------------------------------------------------ fp8, 128 x 128 weight scales
+constexpr int kBlkAccs = 4;
+constexpr int kBlkStageBytes = 2 * 128 * 128;
+constexpr int kBlkStages = 6;
+constexpr int kBlkSmem = kBlkStages * kBlkStageBytes + 1024;
+
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const RowsParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t full_bar[kBlkStages];
+  __shared__ __align__(8) uint64_t empty_bar[kBlkStages];
+  __shared__ __align__(8) uint64_t acc_full[kBlkAccs];
+  __shared__ __align__(8) uint64_t acc_empty[kBlkAccs];
+  __shared__ uint32_t tmem_base_s;
+  const int warp = threadIdx.x >> 5;
+  const int nkb = p.num_kb, items = p.m_tiles * p.n_tiles;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kBlkStages; ++s) {
+      mb::mbar_init(&full_bar[s], 1);
+      mb::mbar_init(&empty_bar[s], 1);
+    }
+    for (int i = 0; i < kBlkAccs; ++i) {
+      mb::mbar_init(&acc_full[i], 1);
+      mb::mbar_init(&acc_empty[i], kEpiWarps);
+    }
+    mb::mbar_fence_init();
+    mb::tma_prefetch_desc(&tmA);
+    mb::tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) mb::tmem_alloc(&tmem_base_s, 128 * kBlkAccs);
+  mb::tc_fence_before();
+  __syncthreads();
+  mb::tc_fence_after();
+  const uint32_t tmem = tmem_base_s;
+  mb::pdl_launch_dependents();
+  mb::pdl_wait();                                            // the work list and the token rows come from preceding kernels
+
+  // item i: token tile i / n_tiles, feature tile i % n_tiles (the CTAs that run together share the token rows in L2 and
+  // stream different weights); entries of the work list without rows are passed over by every role alike
+  struct Item { int row0, rows, w_row0; };
+  auto item = [&](int i, Item& t) {
+    const int mt = i / p.n_tiles, nt = i - mt * p.n_tiles;
+    if (p.tile_expert) {
+      const int e = __ldg(p.tile_expert + mt);
+      if (e < 0) return false;
+      t.row0 = __ldg(p.tile_row0 + mt);
+      t.rows = __ldg(p.tile_nrows + mt);
+      t.w_row0 = e * p.n_per_expert + nt * 128;
+    } else {
+      t.row0 = mt * 128;
+      t.rows = min(128, p.M - t.row0);
+      t.w_row0 = nt * 128;
+    }
+    return true;
+  };
+
+  if (warp == 0) {
+    if (mb::elect_one()) {
+      int g = 0;
+      bool ok = true;
+      for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+        Item t;
+        if (!item(i, t)) continue;
+        for (int kb = 0; kb < nkb; ++kb, ++g) {
+          const int s = g % kBlkStages;
+          ok = mb::mbar_wait(&empty_bar[s], ((g / kBlkStages) & 1) ^ 1, p.status, MB_ST_TIMEOUT_TMA);
+          if (!ok) break;
+          uint8_t* st = smem + s * kBlkStageBytes;
+          mb::mbar_expect_tx(&full_bar[s], p.a_bytes + 128 * 128);
+          mb::tma_load_2d(st + 128 * 128, &tmB, &full_bar[s], kb * 128, t.w_row0);
+          mb::tma_load_2d(st, &tmA, &full_bar[s], kb * 128, t.row0);   // rows past the box keep old bytes: they make rows nobody stores
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (mb::elect_one()) {
+      const uint32_t idesc = mb::umma_idesc(0, 0, 128, 128);
+      int g = 0;
+      bool ok = true;
+      for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+        Item t;
+        if (!item(i, t)) continue;
+        for (int kb = 0; kb < nkb; ++kb, ++g) {
+          const int s = g % kBlkStages, buf = g % kBlkAccs;
+          ok = mb::mbar_wait(&acc_empty[buf], ((g / kBlkAccs) & 1) ^ 1, p.status, MB_ST_TIMEOUT_MMA) &&
+               mb::mbar_wait(&full_bar[s], (g / kBlkStages) & 1, p.status, MB_ST_TIMEOUT_MMA);
+          if (!ok) break;
+          mb::tc_fence_after();
+          const uint32_t a_base = mb::smem_u32(smem + s * kBlkStageBytes), b_base = a_base + 128 * 128;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            mb::umma_f8f6f4(tmem + buf * 128, mb::umma_desc_sw128(a_base + j * 32), mb::umma_desc_sw128(b_base + j * 32), idesc, j != 0);
+          mb::tc_commit(&empty_bar[s]);
+          mb::tc_commit(&acc_full[buf]);
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    constexpr int NC = 64;
+    const int q = warp & 3, half = (warp - 2) >> 2, lane = threadIdx.x & 31;
+    const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + half * NC;
+    int g = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
+      Item t;
+      if (!item(i, t)) continue;
+      const int r = q * 32 + lane;
+      const bool live = r < t.rows;
+      const float* asp = p.a_scale + t.row0 + r;
+      const float* wsp = p.w_scale + (size_t)(t.w_row0 / 128) * nkb;
+      float acc[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = 0.f;
+      // the scales of k block kb + 1 are on their way while block kb is added
+      float a_next = live ? __ldg(asp) : 0.f, w_next = __ldg(wsp);
+      for (int kb = 0; kb < nkb; ++kb, ++g) {
+        const int buf = g % kBlkAccs;
+        const float sc = a_next * w_next;
+        if (kb + 1 < nkb) {
+          a_next = live ? __ldg(asp + (size_t)(kb + 1) * p.a_ld) : 0.f;
+          w_next = __ldg(wsp + kb + 1);
+        }
+        ok = mb::mbar_wait(&acc_full[buf], (g / kBlkAccs) & 1, p.status, MB_ST_TIMEOUT_EPI);
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        mb::tc_fence_after();
+        float v[NC];
+        mb::tmem_ld32_async(src + buf * 128, v);
+        mb::tmem_ld32_async(src + buf * 128 + 32, v + 32);
+        mb::tmem_ld_wait(v);
+        mb::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mb::mbar_arrive(&acc_empty[buf]);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc[c] = fmaf(v[c], sc, acc[c]);
+      }
+      if (ok && live) {
+        const int n0 = (i % p.n_tiles) * 128 + half * NC;
+        const size_t m = (size_t)t.row0 + r;
+#pragma unroll
+        for (int c = 0; c < NC; c += 32) {
+          uint4 res[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) res[k] = residual8(p, m, n0 + c + 8 * k, p.N);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) emit8(p, m, n0 + c + 8 * k, p.N, acc + c + 8 * k, res[k]);
+        }
+      }
+    }
+    mb::tc_fence_before();
+  }
+  __syncthreads();
+  if (warp == 1) {
+    mb::tc_fence_after();
+    mb::tmem_dealloc(tmem, 128 * kBlkAccs);
+  }
+}
+
 template <int KIND, int BN>
 int launch_pair(const CUtensorMap* tm, const RowsParams& p, int pairs, cudaStream_t stream) {
   using C = PairCfg<KIND, BN>;
@@ -404,7 +572,10 @@ int launch_pair(const CUtensorMap* tm, const RowsParams& p, int pairs, cudaStrea
 
 bool mb_gemm_rows_serves(const MbGemmArgs* a) {
   if (a->force_splits > 0 || a->no_cluster || (a->flags & (MB_GEMM_ONE_TILE_PER_CTA | MB_GEMM_DECODE_TILE_ORDER))) return false;
-  if (a->kind == KIND_FP8_BLOCK) return false;
+  if (a->kind == KIND_FP8_BLOCK) {
+    if (a->epilogue != mb::EPI_PLAIN || a->outq) return false;
+    return a->tile_expert ? true : a->force_tn == 0 && a->M > 64;
+  }
   return !a->tile_expert && a->force_tn == 0 && a->M > 128 && (a->flags & MB_GEMM_PERSISTENT_PREFILL);
 }
 
@@ -429,6 +600,27 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
   CUtensorMap tm[4];
   int rc = mbh::encode_2d(&tm[1], dt, a->W, inner, (uint64_t)a->N, row_bytes, box, 128);
   if (rc) return rc;
+
+  if (kind == KIND_FP8_BLOCK) {
+    p.tile_expert = a->tile_expert; p.tile_row0 = a->tile_row0; p.tile_nrows = a->tile_nrows;
+    p.n_per_expert = a->tile_expert ? a->n_per_expert : 0;
+    const int box_rows = !a->tile_expert || a->force_tn == 128 ? 128 : tn;
+    if (box_rows != 16 && box_rows != 32 && box_rows != 64 && box_rows != 128) return MB_ERR_UNSUPPORTED;
+    p.a_bytes = box_rows * 128;
+    p.n_tiles = (p.N + 127) / 128;
+    p.m_tiles = a->tile_expert ? a->max_tiles : (a->M + 127) / 128;
+    if ((rc = mbh::encode_2d(&tm[0], dt, a->X, inner, (uint64_t)a->M, x_pitch, box, (uint32_t)box_rows))) return rc;
+    static bool configured = false;
+    if (!configured) {
+      cudaError_t e = cudaFuncSetAttribute(gemm_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
+      if (e != cudaSuccess) return (int)e;
+      configured = true;
+    }
+    const long long items = (long long)p.m_tiles * p.n_tiles;
+    if (items > 0x7fffffff) return MB_ERR_TOO_LARGE;
+    return (int)mb::launch_kernel_cluster(gemm_block_kernel, dim3(items < sms ? (int)items : sms), dim3(kThreads), kBlkSmem, stream, 1,
+                                          tm[0], tm[1], p);
+  }
 
   if (a->outq) {
     // a warp's 64 or 32 result columns are whole 16-column blocks, and whole 16-byte vectors of the packed row

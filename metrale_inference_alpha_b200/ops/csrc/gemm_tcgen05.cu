@@ -1151,7 +1151,7 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
       case KIND_BF16: return t16 ? launch<KIND_BF16, 16, 2>(tmA, tmB, p, grid, stream) : launch<KIND_BF16, 32, 2>(tmA, tmB, p, grid, stream);
       case KIND_FP8: return t16 ? launch<KIND_FP8, 16, 2>(tmA, tmB, p, grid, stream) : launch<KIND_FP8, 32, 2>(tmA, tmB, p, grid, stream);
       case KIND_NVFP4: return t16 ? launch<KIND_NVFP4, 16, 2>(tmA, tmB, p, grid, stream) : launch<KIND_NVFP4, 32, 2>(tmA, tmB, p, grid, stream);
-      default: return t16 ? launch<KIND_FP8_BLOCK, 16, 2>(tmA, tmB, p, grid, stream) : launch<KIND_FP8_BLOCK, 32, 2>(tmA, tmB, p, grid, stream);
+      default: break;
     }
   }
   switch (kind) {

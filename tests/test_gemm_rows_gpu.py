@@ -1,10 +1,10 @@
-"""GEMMs of many token rows (csrc/gemm_rows.cu): pairs of CTAs for bf16, fp8 per row and NVFP4,
+"""GEMMs of many token rows (csrc/gemm_rows.cu): pairs of CTAs for bf16, fp8 per row and NVFP4, 128 x 128 tiles for fp8 blocks,
 at the edges of their tiles, against the one-tile-per-CTA kernel (the same products in the same order: equal bits) and the oracle."""
 import pytest
 import torch
 
 from metrale_inference_alpha_b200 import ops
-from metrale_inference_alpha_b200.ops import reference as ref
+from metrale_inference_alpha_b200.ops import moe_cuda, reference as ref
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -85,3 +85,39 @@ def test_pair_kernel_quantises_the_swiglu_result(fmt, M, N):
     assert (g != v).float().mean() < 0.02
     exact = ops.linear(ops.encode_act_ref(x.float(), ops.ACT_FOR_WEIGHT[fmt]), w_cpu, swiglu=True, out_f32=True)
     assert (g - exact).norm() <= 1.01 * (v - exact).norm()
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 128, 128), (127, 256, 384), (128, 384, 1024), (129, 136, 1024), (300, 1024, 640), (5000, 256, 256)])
+def test_block_kernel_matches_the_one_tile_kernel_and_the_oracle(M, N, K):
+    x, w_cpu, act, w = _operands("fp8_block", M, N, K, 9)
+    res = torch.randn(M, N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    got = ops.linear(act, w, out_f32=True)
+    assert torch.equal(got, ops.linear(act, w, out_f32=True, one_tile_per_cta=True, force_splits=1))
+    assert torch.equal(ops.linear(act, w, residual=res), ops.linear(act, w, residual=res, one_tile_per_cta=True, force_splits=1))
+    ops.check_status(DEV)
+    want = _oracle(x, w_cpu, "fp8_block")
+    assert (got.cpu().double() - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("tile_rows", [16, 32, 64, 128])
+def test_block_kernel_over_a_work_list_of_experts(tile_rows):
+    """Experts with no row, one row, a whole tile, one more than a tile; pairs of experts that are not here."""
+    E, N, K = 6, 384, 512
+    g = torch.Generator().manual_seed(tile_rows)
+    counts = [0, 1, tile_rows, tile_rows + 1, 3 * tile_rows - 1, 5]
+    ids = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)] + [torch.full((7,), -1)])
+    ids = ids[torch.randperm(len(ids), generator=g)].to(torch.int32)
+    T = len(ids)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    w = ops.make_weight(torch.randn(E * N, K, generator=g) * 0.05, "fp8_block")
+    act = ops.quantize_act(x.to(DEV), "fp8_g128")
+    sp = moe_cuda.SortedPairs(ids.to(DEV).view(T, 1), 0, E, tile_rows)
+    y = ops.linear(moe_cuda.gather_act(act, sp), w.to(DEV), out_f32=True, grouped=(sp.tile_expert, sp.tile_row0, sp.tile_nrows, N, sp.max_tiles, tile_rows))
+    ops.check_status(DEV)
+    a, d, at = ops.encode_act_ref(x.float(), "fp8_g128").data.double(), w.dequant().double(), sp.pair_row.cpu()
+    for i in range(T):
+        e = int(ids[i])
+        assert (int(at[i]) < 0) == (e < 0)
+        if e >= 0:
+            want = d[e * N:(e + 1) * N] @ a[i]
+            assert (y[int(at[i])].cpu().double() - want).norm() <= 1e-5 * want.norm()
