@@ -174,6 +174,124 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const RopeKvParams p) {
   }
 }
 
+// The same for head sizes of 64, 128 and 256 in whole 16-byte vectors: a thread owns 8 neighbouring dims of a head, D / 8
+// threads a head, a CTA one token (its cos / sin row is read once) and 2048 / D heads at a time; a rotation's partner is
+// half / 8 lanes away. Bound by memory: 8192 tokens of 40 + 8 + 8 heads of 128 move 220 MB (34 us at copy bandwidth); a warp per
+// head with 2-byte accesses and its own cos / sin reads took 181 us, this 78 us. Few tokens: blockIdx.y spreads a token's heads
+// over CTAs until the chip has some four each.
+template <int D>
+__global__ void __launch_bounds__(256, 6) rope_kv_vec_kernel(const RopeKvParams p) {
+  constexpr int kLanes = D / 8, kHeads = 256 / kLanes;
+  const int m = blockIdx.x;
+  mb::pdl_wait();
+  mb::pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, sub = threadIdx.x % kLanes, at = threadIdx.x / kLanes;
+  const int Htot = p.Hq + 2 * p.Hkv, half = p.rot / 2;
+  const bool rot = p.cos_tab && sub * 8 < p.rot;
+  float cs[8], sn[8];
+  int partner = lane;
+  if (rot) {
+    int pos = p.positions[m];
+    if (pos < 0 || pos >= p.max_pos) {
+      if (sub == 0 && p.status) atomicCAS(p.status, 0u, MB_ST_BOUNDS);
+      pos = 0;
+    }
+    const bool first = sub * 8 < half;
+    const size_t i0 = (size_t)pos * half + (first ? sub * 8 : sub * 8 - half);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 c4 = __ldg(reinterpret_cast<const float4*>(p.cos_tab + i0) + i), s4 = __ldg(reinterpret_cast<const float4*>(p.sin_tab + i0) + i);
+      cs[4 * i] = c4.x; cs[4 * i + 1] = c4.y; cs[4 * i + 2] = c4.z; cs[4 * i + 3] = c4.w;
+      const float g = first ? -1.f : 1.f;                    // x1 c - x2 s and x2 c + x1 s
+      sn[4 * i] = g * s4.x; sn[4 * i + 1] = g * s4.y; sn[4 * i + 2] = g * s4.z; sn[4 * i + 3] = g * s4.w;
+    }
+    partner = first ? lane + half / 8 : lane - half / 8;
+  }
+  const long long slot = p.slots[m];
+  const bool write = slot >= 0 && slot < p.num_slots;
+  if (slot >= p.num_slots && threadIdx.x == 0 && p.status) atomicCAS(p.status, 0u, MB_ST_BOUNDS);
+  const __nv_bfloat16* row = p.qkv + (size_t)m * p.qkv_ld;
+  for (int hb = blockIdx.y * kHeads; hb < Htot; hb += gridDim.y * kHeads) {
+    const bool live = hb + at < Htot;                        // whole warps go round: the shuffles need every lane
+    const int head = live ? hb + at : 0;
+    const int kind = head < p.Hq ? 0 : head < p.Hq + p.Hkv ? 1 : 2;
+    const int h = kind == 0 ? head : kind == 1 ? head - p.Hq : head - p.Hq - p.Hkv;
+    const __nv_bfloat16* src = row + (kind == 0 ? (size_t)h * p.q_head_stride : (size_t)(kind == 1 ? p.k_off : p.v_off) + (size_t)h * D);
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src + sub * 8));
+    const __nv_bfloat162* rb = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(rb[i]);
+      v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+    if (p.q_norm_w || p.k_norm_w) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+#pragma unroll
+      for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const __nv_bfloat16* nw = kind == 0 ? p.q_norm_w : kind == 1 ? p.k_norm_w : nullptr;
+      if (nw) {
+        const float inv = rsqrtf(ss / (float)D + p.eps);
+        const uint4 w8 = __ldg(reinterpret_cast<const uint4*>(nw + sub * 8));
+        const __nv_bfloat162* wb = reinterpret_cast<const __nv_bfloat162*>(&w8);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float2 w = __bfloat1622float2(wb[i]);
+          if (p.norm_plus_one) { w.x += 1.f; w.y += 1.f; }
+          // the normalised value passes through bf16 like an unfused norm kernel's output
+          v[2 * i] = __bfloat162float(__float2bfloat16(v[2 * i] * inv * w.x));
+          v[2 * i + 1] = __bfloat162float(__float2bfloat16(v[2 * i + 1] * inv * w.y));
+        }
+      }
+    }
+    if (p.cos_tab) {
+      // the values are bf16 numbers at this point (as loaded, or rounded behind the norm): two go in one shuffle
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 mine = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        const uint32_t got = __shfl_sync(0xffffffffu, *reinterpret_cast<const uint32_t*>(&mine), partner);
+        const float2 other = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&got));
+        if (rot && kind != 2) {
+          v[2 * i] = v[2 * i] * cs[2 * i] + other.x * sn[2 * i];
+          v[2 * i + 1] = v[2 * i + 1] * cs[2 * i + 1] + other.y * sn[2 * i + 1];
+        }
+      }
+    }
+    float mx = 0.f;
+    if (p.amax) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
+#pragma unroll
+      for (int o = kLanes / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (!live || (kind != 0 && !write)) continue;
+    const size_t off = ((size_t)slot * p.Hkv + h) * D + sub * 8;
+    if (kind != 0) {
+      // non-negative floats order like their bit patterns
+      if (p.amax && sub == 0) atomicMax(reinterpret_cast<int*>(p.amax + (kind - 1)), __float_as_int(mx));
+      if (p.cache_fp8) {
+        const float inv = 1.f / (kind == 1 ? *p.k_scale : *p.v_scale);
+        uint32_t w[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          w[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(v[4 * i] * inv, v[4 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3) |
+                 ((uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(v[4 * i + 2] * inv, v[4 * i + 3] * inv), __NV_SATFINITE, __NV_E4M3) << 16);
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(kind == 1 ? p.k_cache : p.v_cache) + off) = make_uint2(w[0], w[1]);
+        continue;
+      }
+    }
+    uint4 o;
+    __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ob[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    __nv_bfloat16* dst = kind == 0 ? p.q_out + ((size_t)m * p.Hq + h) * D + sub * 8
+                                   : reinterpret_cast<__nv_bfloat16*>(kind == 1 ? p.k_cache : p.v_cache) + off;
+    *reinterpret_cast<uint4*>(dst) = o;
+  }
+}
+
 // ------------------------------------------------------------------ mma helpers
 template <bool F16>
 __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -1253,6 +1371,19 @@ int mb_qk_norm_rope_kvwrite(const MbRopeKvArgs* a, cudaStream_t stream) {
   p.status = a->status;
   p.amax = a->amax;
   const int Htot = a->Hq + 2 * a->Hkv;
+  // whole 16-byte vectors everywhere: the vector kernel; other head sizes and unaligned rows keep a warp per head
+  const uintptr_t al = reinterpret_cast<uintptr_t>(a->qkv) | reinterpret_cast<uintptr_t>(a->q_out) | reinterpret_cast<uintptr_t>(a->k_cache) |
+                       reinterpret_cast<uintptr_t>(a->v_cache) | reinterpret_cast<uintptr_t>(a->q_norm_w) | reinterpret_cast<uintptr_t>(a->k_norm_w) |
+                       reinterpret_cast<uintptr_t>(a->cos_tab) | reinterpret_cast<uintptr_t>(a->sin_tab);
+  const bool vec = !(al & 15) && a->qkv_ld % 8 == 0 && a->q_head_stride % 8 == 0 && a->k_off % 8 == 0 && a->v_off % 8 == 0;
+  if (vec && (a->D == 64 || a->D == 128 || a->D == 256)) {
+    const int full = (Htot * (a->D / 8) + 255) / 256;
+    const int spread = (592 + a->M - 1) / a->M;              // 148 SMs x 4
+    const dim3 grid(a->M, spread < full ? spread : full);
+    if (a->D == 64) return (int)mb::launch_kernel(rope_kv_vec_kernel<64>, grid, dim3(256), 0, stream, p);
+    if (a->D == 128) return (int)mb::launch_kernel(rope_kv_vec_kernel<128>, grid, dim3(256), 0, stream, p);
+    return (int)mb::launch_kernel(rope_kv_vec_kernel<256>, grid, dim3(256), 0, stream, p);
+  }
   return (int)mb::launch_kernel(rope_kv_kernel, dim3(a->M, (Htot + 3) / 4), dim3(128), 0, stream, p);
 }
 
