@@ -1072,6 +1072,9 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
     splits = 1;
     if (tiles < sms && a->ws) {
       splits = sms / tiles;
+      // a cluster of at most eight finishes a tile together; more than eight leave the whole sum to the last one to arrive
+      // (2048 x 5120 bf16, 128 tokens: nine splits 41 us, eight 23)
+      if (splits > 8 && !a->no_cluster) splits = 8;
       const int max_by_k = num_kb / 4 > 0 ? num_kb / 4 : 1;
       if (splits > max_by_k) splits = max_by_k;
       if (splits < 1) splits = 1;
