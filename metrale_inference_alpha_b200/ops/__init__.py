@@ -886,9 +886,11 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     `quant_out` > 0: return the output as an NVFP4 `Act` [T, Hq * D] quantised with that calibrated
     global scale (inside the split-KV kernel for decode-sized steps, else by a row kernel)."""
     T, Hq, D = q.shape
+    prefill = force_mode == 3 or (force_mode == 0 and _ATTN_TC and D in (128, 256) and window == 0 and max_q_len >= 128)
     if quant_out > 0.0:
         Hkv_ = k_cache.shape[2]
-        fused = q.is_cuda and force_mode == 0 and (Hq // Hkv_) * max_q_len <= 16 and D % 128 == 0 and (Hq * D) % 64 == 0
+        rows = prefill and D == 128 and window == 0 and scale > 0 and _ATTN_TC_VMN != 0                    # csrc/attention_rows.cu
+        fused = q.is_cuda and (rows or (force_mode == 0 and (Hq // Hkv_) * max_q_len <= 16 and D % 128 == 0 and (Hq * D) % 64 == 0))
         if not fused:
             o = paged_attention(q, k_cache, v_cache, block_table, q_start, q_len, ctx_len, max_q_len=max_q_len,
                                 max_ctx=max_ctx, scale=scale, k_scale=k_scale, v_scale=v_scale, window=window,
@@ -903,16 +905,22 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     G = Hq // Hkv
     if part_tokens == 0:
         part_tokens = _ATTN_PART_TOKENS
-    out = torch.empty_like(q)
+    out = torch.empty_like(q) if quant_out <= 0.0 else None
     S = q_len.numel()
+    qact = None
+    if quant_out > 0.0:
+        Kq = Hq * D
+        qact = Act("nvfp4", T, Kq, torch.empty(T, Kq // 2, dtype=torch.uint8, device=q.device))
+        qact.sf, qact.sf_k64 = _sf_buffer(q.device, T, Kq)
+        qact.scale = static_scale_vec(q.device, quant_out, T)
     if force_mode == 0 and G * max_q_len <= 32 and D == 256 and G * max_q_len > 16:
         # two row tiles do not fit the register file at head_dim 256: present every query
         # token as its own single-row sequence (causality then comes from ctx_len alone)
         return _attention_rowwise(q, k_cache, v_cache, block_table, q_start, q_len, ctx_len,
                                   max_ctx=max_ctx, scale=scale, k_scale=k_scale, v_scale=v_scale,
                                   window=window)
-    if force_mode == 3 or (force_mode == 0 and _ATTN_TC and D in (128, 256) and window == 0 and max_q_len >= 128):
-        # prefill chunks: both products on tcgen05 with TMEM accumulators (csrc/attention_tc.cu)
+    if prefill:
+        # prefill chunks: both products on tcgen05 with TMEM accumulators (csrc/attention_tc.cu, csrc/attention_rows.cu)
         t = _native.AttnTcArgs()
         t.q, t.k_cache, t.v_cache, t.block_table = _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_table)
         t.q_start, t.q_len, t.ctx_len = _ptr(q_start), _ptr(q_len), _ptr(ctx_len)
@@ -920,9 +928,11 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
         t.num_blocks, t.max_blocks, t.num_seqs, t.max_q_len = nb, block_table.stride(0), S, max_q_len
         t.Hq, t.Hkv, t.D, t.block_size, t.cache_fp8, t.scale = Hq, Hkv, D, bs, int(k_cache.dtype == torch.uint8), scale
         t.v_mn = 1 if D == 256 else _ATTN_TC_VMN
+        if qact is not None:
+            t.outq, t.ldq, t.outq_sf, t.outq_sf_k64, t.outq_gs = _ptr(qact.data), Kq // 2, _ptr(qact.sf), qact.sf_k64, quant_out
         _native.check(L.mb_attn_prefill_tc(C.byref(t), _stream()), "attn_prefill_tc")
         _count()
-        return out
+        return out if qact is None else qact
     a = _native.AttnArgs()
     a.q, a.k_cache, a.v_cache = _ptr(q), _ptr(k_cache), _ptr(v_cache)
     a.block_table, a.max_blocks = _ptr(block_table), block_table.stride(0)
@@ -930,17 +940,12 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     a.num_seqs, a.max_q_len, a.max_ctx = S, max_q_len, max_ctx
     a.Hq, a.Hkv, a.D, a.block_size, a.num_blocks = Hq, Hkv, D, bs, nb
     a.scale, a.cache_fp8 = scale, int(k_cache.dtype == torch.uint8)
-    a.k_scale, a.v_scale, a.out = _ptr(k_scale), _ptr(v_scale), _ptr(out)
+    a.k_scale, a.v_scale, a.out = _ptr(k_scale), _ptr(v_scale), _ptr(out if qact is None else qact.data)
     need = L.mb_attn_ws_bytes(T, Hq, D, max_ctx, part_tokens)
     rt.ensure_attn_ws(need)
     a.ws, a.ws_bytes, a.total_rows = _ptr(rt.attn_ws), rt.attn_ws.numel(), T
     a.part_tokens, a.window, a.force_mode, a.status = part_tokens, window, force_mode, _ptr(rt.status)
-    qact = None
-    if quant_out > 0.0:
-        Kq = Hq * D
-        qact = Act("nvfp4", T, Kq, torch.empty(T, Kq // 2, dtype=torch.uint8, device=q.device))
-        qact.sf, qact.sf_k64 = _sf_buffer(q.device, T, Kq)
-        qact.scale = static_scale_vec(q.device, quant_out, T)
+    if qact is not None:
         a.outq, a.ldq, a.outq_sf, a.outq_sf_k64, a.outq_gs = _ptr(qact.data), Kq // 2, _ptr(qact.sf), qact.sf_k64, quant_out
     _native.check(L.mb_paged_attention(C.byref(a), _stream()), "paged_attention")
     _count()
