@@ -64,6 +64,7 @@ class _Runtime:
         from ..utils.alloc_ledger import ledger
         self.ws = ledger().alloc(self.ws_bytes, torch.uint8, device, "gemm workspace")
         self.attn_ws = ledger().alloc(32 << 20, torch.uint8, device, "attention workspace")
+        self._outgrown = []
         self.status = ledger().alloc(4, torch.int32, device, "status word")
 
     @classmethod
@@ -77,6 +78,7 @@ class _Runtime:
     def ensure_attn_ws(self, nbytes: int):
         if nbytes > self.attn_ws.numel():
             from ..utils.alloc_ledger import ledger
+            self._outgrown.append(self.attn_ws)               # captured graphs hold its address
             self.attn_ws = ledger().alloc(int(nbytes * 1.25), torch.uint8, self.device, "attention workspace")
 
 
@@ -862,6 +864,7 @@ _native.register_optional("mb_kv_rescale", [C.c_void_p, C.c_void_p, C.c_int, C.c
 # split-KV partition size (tokens); a function of nothing but this lever, so a sequence's
 # partitioning -- and therefore its numerics -- never depends on the rest of the batch
 _ATTN_PART_TOKENS = int(os.environ.get("METRALE_ATTN_PART_TOKENS", "0") or 0)
+_PART_LEVER = _ATTN_PART_TOKENS                  # the plain decode kernel has a size of its own, which only the lever overrules
 
 
 def configure(attn_part_tokens: Optional[int] = None) -> None:
@@ -903,6 +906,7 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     rt = runtime(q.device)
     nb, bs, Hkv, _ = k_cache.shape
     G = Hq // Hkv
+    part_fixed = part_tokens or _PART_LEVER
     if part_tokens == 0:
         part_tokens = _ATTN_PART_TOKENS
     out = torch.empty_like(q) if quant_out <= 0.0 else None
@@ -941,10 +945,10 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     a.Hq, a.Hkv, a.D, a.block_size, a.num_blocks = Hq, Hkv, D, bs, nb
     a.scale, a.cache_fp8 = scale, int(k_cache.dtype == torch.uint8)
     a.k_scale, a.v_scale, a.out = _ptr(k_scale), _ptr(v_scale), _ptr(out if qact is None else qact.data)
-    need = L.mb_attn_ws_bytes(T, Hq, D, max_ctx, part_tokens)
-    rt.ensure_attn_ws(need)
-    a.ws, a.ws_bytes, a.total_rows = _ptr(rt.attn_ws), rt.attn_ws.numel(), T
-    a.part_tokens, a.window, a.force_mode, a.status = part_tokens, window, force_mode, _ptr(rt.status)
+    a.total_rows, a.part_tokens, a.part_fixed, a.sm_count = T, part_tokens, part_fixed, rt.sm_count
+    a.window, a.force_mode, a.status = window, force_mode, _ptr(rt.status)
+    rt.ensure_attn_ws(L.mb_attn_ws_need(C.byref(a)))
+    a.ws, a.ws_bytes = _ptr(rt.attn_ws), rt.attn_ws.numel()
     if qact is not None:
         a.outq, a.ldq, a.outq_sf, a.outq_sf_k64, a.outq_gs = _ptr(qact.data), Kq // 2, _ptr(qact.sf), qact.sf_k64, quant_out
     _native.check(L.mb_paged_attention(C.byref(a), _stream()), "paged_attention")

@@ -99,7 +99,7 @@ class AttnArgs(C.Structure):
         ("outq", c_void_p), ("ldq", c_int), ("outq_sf", c_void_p), ("outq_sf_k64", c_int), ("outq_gs", c_float),
         ("DV", c_int), ("dv", c_int), ("out_ld", c_ll), ("out_scale", c_float), ("sink", c_int), ("split_p", c_int),
         ("sink_w", c_void_p), ("keep", c_int), ("gate", c_void_p), ("gate_ld", c_ll), ("gate_mode", c_int), ("softcap", c_float),
-        ("turn_cos", c_void_p), ("turn_sin", c_void_p), ("turn_max", c_int),
+        ("turn_cos", c_void_p), ("turn_sin", c_void_p), ("turn_max", c_int), ("part_fixed", c_int), ("sm_count", c_int),
     ]
 
 
@@ -161,6 +161,7 @@ def lib():
     L.mb_attn_visible.argtypes, L.mb_attn_visible.restype = [c_int] * 4, c_int
     L.mb_attn_ws_bytes.argtypes = [c_int, c_int, c_int, c_int, c_int]
     L.mb_attn_ws_bytes.restype = c_size_t
+    L.mb_attn_ws_need.argtypes, L.mb_attn_ws_need.restype = [P(AttnArgs)], c_size_t
     L.mb_argmax.argtypes = [c_void_p, c_int, c_ll, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                             c_void_p, c_void_p, c_void_p]
     L.mb_argmax.restype = c_int

@@ -25,6 +25,7 @@
 // reshape_and_cache.cu, rope.cu, paged_decode_attn{,_fp8,_bf16_gqa,_fp8_gqa}.cu
 // (+ split-K reduce), prefill_paged_compute.cuh and attn_prefill_paged{,_fp8,_batched}.cu.
 #include "common.cuh"
+#include "attention_decode.h"
 #include "visible.cuh"
 #include <type_traits>
 
@@ -1431,7 +1432,31 @@ struct MbAttnArgs {
   const float* turn_cos;   // [turn_max, dv / 2] or null: every output row is turned back by its position
   const float* turn_sin;
   int turn_max;
+  int part_fixed;          // partition size that the caller insists on for the plain decode kernel too (0 = its own)
+  int sm_count;
 };
+
+// the plain decode / verify case that attention_decode.cu may serve (force_mode 1 keeps it on the split-KV kernel here)
+static bool decode_args(const MbAttnArgs* a, AttnDecodeArgs* d) {
+  const int DV = a->DV > 0 ? a->DV : a->D, dv = a->dv > 0 ? a->dv : DV;
+  if (a->force_mode != 0 || DV != a->D || dv != DV || a->sink || a->split_p || a->window > 0 || a->gate || a->softcap > 0.f || a->turn_cos ||
+      (a->out_scale != 0.f && a->out_scale != 1.f) || a->Hkv <= 0 || a->Hq % a->Hkv)
+    return false;
+  *d = AttnDecodeArgs{};
+  d->q = reinterpret_cast<const __nv_bfloat16*>(a->q); d->k_cache = a->k_cache; d->v_cache = a->v_cache;
+  d->block_table = a->block_table; d->max_blocks = a->max_blocks;
+  d->q_start = a->q_start; d->q_len = a->q_len; d->ctx_len = a->ctx_len;
+  d->num_seqs = a->num_seqs; d->max_q_len = a->max_q_len; d->max_ctx = a->max_ctx;
+  d->Hq = a->Hq; d->Hkv = a->Hkv; d->D = a->D; d->block_size = a->block_size; d->fp8 = a->cache_fp8; d->num_blocks = a->num_blocks;
+  d->scale = a->scale; d->k_scale = a->k_scale; d->v_scale = a->v_scale;
+  d->out = reinterpret_cast<__nv_bfloat16*>(a->out);
+  d->out_ld = a->out_ld > 0 ? a->out_ld : (long long)a->Hq * a->D;
+  d->outq = reinterpret_cast<uint8_t*>(a->outq); d->ldq = a->ldq;
+  d->outq_sf = reinterpret_cast<uint8_t*>(a->outq_sf); d->outq_sf_k64 = a->outq_sf_k64; d->outq_gs = a->outq_gs;
+  d->ws = a->ws; d->ws_bytes = a->ws_bytes; d->total_rows = a->total_rows; d->part_tokens = a->part_fixed; d->sm_count = a->sm_count;
+  d->status = a->status;
+  return mb_attn_decode_serves(*d);
+}
 
 // most entries of the visible-token list of a sequence: its context, or the kept first tokens and the windows of its
 // queries, each rounded to whole tiles
@@ -1447,6 +1472,13 @@ size_t mb_attn_ws_bytes(int total_rows, int Hq, int D, int max_ctx, int part_tok
   const int parts = (max_ctx + pt - 1) / pt;
   if (parts <= 1) return 0;
   return kAttnCntBytes + (size_t)total_rows * Hq * parts * (D + 2) * sizeof(float);
+}
+
+// workspace bytes of this call (its pointers but the caches' and q's may still be null)
+size_t mb_attn_ws_need(const MbAttnArgs* a) {
+  AttnDecodeArgs d;
+  if (decode_args(a, &d)) return mb_attn_decode_ws(d);
+  return mb_attn_ws_bytes(a->total_rows, a->Hq, a->DV > 0 ? a->DV : a->D, a->max_ctx, a->part_tokens);
 }
 
 int mb_paged_attention(const MbAttnArgs* a, cudaStream_t stream) {
@@ -1490,6 +1522,8 @@ int mb_paged_attention(const MbAttnArgs* a, cudaStream_t stream) {
   }
   if (mode == 1) {
     if (rows > 32) return MB_ERR_UNSUPPORTED;
+    AttnDecodeArgs d;
+    if (decode_args(a, &d) && d.ws_bytes >= mb_attn_decode_ws(d)) return mb_attn_decode(d, stream);
     const int mt = rows <= 16 ? 1 : 2;
     p.part_tokens = a->part_tokens > 0 ? a->part_tokens : 512;
     p.parts = (mb_attn_visible(a->max_ctx, a->max_q_len, p.window, p.keep) + p.part_tokens - 1) / p.part_tokens;

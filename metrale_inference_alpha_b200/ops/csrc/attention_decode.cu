@@ -1,0 +1,660 @@
+// Decode and verify attention for the plain case (softmax without sink, cap, window or gate; head dim 128 or 256; blocks of a
+// multiple of 16 tokens): at most 32 query rows (tokens x heads of a group) against a paged bf16 or e4m3 cache.
+//
+// What bounds it at decode is instructions and their latency: few warps run per scheduler, and the split-KV kernel of
+// attention.cu (which keeps the other cases) spends 2400 instructions per warp around its tiles. Here:
+//   * the four warps of a CTA stream on their own: warp w takes every fourth step of 16 or 32 tokens of its partition, one TMA box
+//     per 16 tokens and 128 bytes of row width for K and for V, issued by one lane into the warp's own ring. No CTA barrier until
+//     the partition ends.
+//   * a fixed number of CTAs walks the list of (sequence, partition, kv head) units. Each CTA finds its units from the lengths
+//     alone (a prefix sum in shared memory), so neither idle partitions of a fixed launch geometry nor long ones cost a wave.
+//     The next unit's first slices are under way while this one's warps are merged.
+//   * partitions depend on the sequence's own length only (never on the batch): part_tokens each, but at most 32 of them;
+//     the last to arrive merges them in order.
+// The tensor-core fragments are as in attention.cu: mma.sync m16n8k16, an e4m3 row widened to f16 in registers.
+// Measured against that kernel (us): e4m3, 40 / 8 heads of 128: one sequence of 700 tokens 22.5 -> 13.7, 128 of 129 to 1151 62 -> 50,
+// nine of 4000 to 16000 73 -> 54, eight verify steps of 4 rows 31 -> 22; bf16, 33 of 100 to 2047 57 -> 32; 16 / 2 heads of 256,
+// bf16, sixteen of 200 to 2000 119 -> 22.
+#include "common.cuh"
+#include "attention_decode.h"
+#include "tensormap.h"
+
+namespace {
+
+constexpr int kMaxParts = 32, kMaxSeqs = 1024, kSlice = 16;
+constexpr size_t kCntBytes = 64 * 1024;      // arrival counters at the head of the workspace, as in attention.cu
+
+struct DecodeParams {
+  const __nv_bfloat16* q;
+  const int* block_table;
+  int max_blocks;
+  const int* q_start;
+  const int* q_len;
+  const int* ctx_len;
+  int num_seqs, Hq, Hkv, G, g_magic;         // r / G = r * g_magic >> 16 for r < 64
+  int block_size, block_shift;               // shift -1: no power of two
+  long long num_blocks;
+  float scale;
+  const float* k_scale;
+  const float* v_scale;
+  __nv_bfloat16* out;
+  long long out_ld;
+  uint8_t* outq;
+  int ldq;
+  uint8_t* outq_sf;
+  int outq_sf_k64;
+  float outq_gs;
+  float* part_o;                             // [rows * Hq, parts, D]
+  float2* part_ml;                           // [rows * Hq, parts]: log2-domain maximum, sum
+  uint32_t* part_cnt;                        // [seqs * Hkv]
+  int parts, part_tokens;
+  int ahead;                                 // slots of the ring that the next unit may fill while warps are merged
+  uint32_t merge_off, tail_off, len_off;     // byte offsets of the merge buffer and of what lies behind both
+  int over;                                  // the merge buffer lies over slots of the ring
+  uint32_t* status;
+};
+
+__device__ __forceinline__ void mma16816_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma16816_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool F16>
+__device__ __forceinline__ void mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  if constexpr (F16) mma16816_f16(c, a, b0, b1);
+  else mma16816_bf16(c, a, b0, b1);
+}
+__device__ __forceinline__ void ldsm4(uint32_t* r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t* r, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <bool F16>
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  if constexpr (F16) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+__device__ __forceinline__ uint32_t e4m3x2(uint32_t two) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"((uint16_t)two));
+  return r;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int D, bool FP8, int MT>
+struct DecodeCfg {
+  static constexpr int kRowB = FP8 ? D : 2 * D;              // bytes of a cached row
+  static constexpr int kSpans = kRowB / 128;                 // TMA boxes (and swizzled spans) across it
+  // slices that a warp takes together: two chains of products in flight, and one maximum and one wait for 32 tokens
+  static constexpr int kSub = FP8 && D == 128 ? 2 : 1;
+  static constexpr int kTok = kSub * kSlice;
+  static constexpr int kHalf = kTok * kRowB;                 // K or V of one step
+  static constexpr int kSlot = 2 * kHalf;
+  static constexpr int kSlots = 2;
+  static constexpr int kRing = 4 * kSlots * kSlot;           // slot s of warp w at (s * 4 + w) * kSlot
+  static constexpr int kCtas = MT > 1 ? (D == 256 ? 1 : 2) : D == 256 ? 1 : 3;
+  static constexpr int kQPitch = 2 * D + 16;                 // bytes between query rows in shared memory
+};
+
+template <int D, bool FP8, int MT>
+__global__ void __launch_bounds__(128, DecodeCfg<D, FP8, MT>::kCtas)
+attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeParams p) {
+  using C = DecodeCfg<D, FP8, MT>;
+  constexpr int kSlots = C::kSlots, kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t bars[4 * kSlots];
+  __shared__ int s_last, s_wsum[4];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  float* s_o = reinterpret_cast<float*>(smem + p.merge_off);                  // [4 warps][rows][D]
+  int* s_off = reinterpret_cast<int*>(smem + p.tail_off);                     // [seqs + 1]
+  float2* s_ml = reinterpret_cast<float2*>(s_off + ((p.num_seqs + 2) & ~1));  // [4][MT * 16]
+  int4* s_len = reinterpret_cast<int4*>(smem + p.len_off);                    // [seqs]: q_len, ctx_len, q_start
+  uint8_t* s_q = smem + p.len_off + p.num_seqs * 16;                          // the unit's query rows, as loaded
+  if (tid == 0) {
+    for (int i = 0; i < 4 * kSlots; ++i) mb::mbar_init(&bars[i], 1);
+    mb::mbar_fence_init();
+    mb::tma_prefetch_desc(&tmK);
+    mb::tma_prefetch_desc(&tmV);
+  }
+  mb::pdl_wait();
+  mb::pdl_launch_dependents();
+
+  // ---- the list of units: partitions of every sequence in front of it
+  auto part_size = [&](int len) { return max(p.part_tokens, ((len + kMaxParts - 1) / kMaxParts + 63) & ~63); };
+  auto count = [&](int len, int P) { return len <= P ? 1 : (len + P - 1) / P; };
+  {
+    int base = 0;
+    for (int s0 = 0; s0 < p.num_seqs; s0 += 128) {
+      const int s = s0 + tid;
+      int n = 0;
+      if (s < p.num_seqs) {
+        const int4 x = make_int4(p.q_len[s], p.ctx_len[s], p.q_start[s], 0);
+        const int len = max(1, x.y);
+        s_len[s] = x;
+        if (x.x > 0) n = min(count(len, part_size(len)), p.parts);
+      }
+      int x = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+      }
+      if (lane == 31) s_wsum[warp] = x;
+      __syncthreads();
+      int before = base;
+      for (int w = 0; w < warp; ++w) before += s_wsum[w];
+      if (s < p.num_seqs) s_off[s + 1] = before + x;
+      base += s_wsum[0] + s_wsum[1] + s_wsum[2] + s_wsum[3];
+      __syncthreads();
+    }
+    if (tid == 0) s_off[0] = 0;
+    __syncthreads();
+  }
+  const int units = s_off[p.num_seqs] * p.Hkv;
+
+  // ---- one unit: its place and this warp's slices of it
+  struct Unit {
+    int seq, part, nparts, kvh, begin, slices;               // slices: of this warp
+    int qlen, ctx, qs;
+    int blk, within;                                         // lane l: block and first token in it of this warp's slice l
+  };
+  auto find = [&](int u, Unit& x) {
+    const int at = u / p.Hkv;
+    x.kvh = u - at * p.Hkv;
+    int lo = 0, hi = p.num_seqs;                             // s_off[lo] <= at < s_off[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_off[mid] <= at) lo = mid;
+      else hi = mid;
+    }
+    x.seq = lo;
+    x.part = at - s_off[lo];
+    x.nparts = s_off[lo + 1] - s_off[lo];
+    const int4 ln = s_len[lo];
+    x.qlen = ln.x;
+    x.ctx = ln.y;
+    x.qs = ln.z;
+    const int len = (((x.ctx + x.nparts - 1) / x.nparts) + 63) & ~63;
+    x.begin = x.part * len;
+    const int end = min(x.ctx, x.begin + len), n = (max(0, end - x.begin) + kTok - 1) / kTok;
+    x.slices = (n - warp + 3) >> 2;
+  };
+  // places of the slices of this warp's steps i0 .. i0 + 32 / kSub - 1, one per lane
+  auto blocks = [&](Unit& x, int i0) {
+    const int i = i0 + lane / kSub, tok = x.begin + (warp + 4 * i) * kTok + lane % kSub * kSlice;
+    x.blk = x.within = 0;                                    // a slice behind the context reads the null block
+    if (i < x.slices && tok < x.ctx) {
+      const int bi = p.block_shift >= 0 ? tok >> p.block_shift : tok / p.block_size;
+      int b = __ldg(p.block_table + (size_t)x.seq * p.max_blocks + bi);
+      if (b < 0 || b >= p.num_blocks) {
+        if (p.status) atomicCAS(p.status, 0u, MB_ST_BOUNDS);
+        b = 0;
+      }
+      x.blk = b;
+      x.within = tok - bi * p.block_size;
+    }
+  };
+  const uint32_t my = mb::smem_u32(smem) + warp * C::kSlot;
+  auto issue = [&](const Unit& x, int i, int slot) {         // whole warp; one lane issues
+    const int place = x.blk * p.block_size + x.within;
+    uint64_t* bar = &bars[slot * 4 + warp];
+    uint8_t* dst = smem + (slot * 4 + warp) * C::kSlot;
+    if (lane == 0) mb::mbar_expect_tx(bar, C::kSlot);
+#pragma unroll
+    for (int b = 0; b < kSub; ++b) {
+      const int tok = __shfl_sync(0xffffffffu, place, (i * kSub + b) & 31);
+      if (lane == 0) {
+#pragma unroll
+        for (int h = 0; h < kSpans; ++h) {
+          mb::tma_load_3d(dst + (b * kSpans + h) * (kSlice * 128), &tmK, bar, h * 128, x.kvh, tok);
+          mb::tma_load_3d(dst + C::kHalf + (b * kSpans + h) * (kSlice * 128), &tmV, bar, h * 128, x.kvh, tok);
+        }
+      }
+    }
+  };
+  // the unit's query rows into shared memory: the whole CTA, 16 bytes a copy
+  auto fetch_q = [&](const Unit& x) {
+    const int n = p.G * x.qlen * (D / 8);
+    for (int i = tid; i < n; i += 128) {
+      const int r = i / (D / 8), c = i % (D / 8), tq = (r * p.g_magic) >> 16;
+      const __nv_bfloat16* src = p.q + ((size_t)(x.qs + tq) * p.Hq + x.kvh * p.G + (r - tq * p.G)) * D + c * 8;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mb::smem_u32(s_q + r * C::kQPitch + c * 16)), "l"(src) : "memory");
+    }
+  };
+
+  const float kmul = FP8 ? *p.k_scale : 1.f, vmul = FP8 ? *p.v_scale : 1.f;
+  const float sc_log2 = p.scale * kmul * 1.44269504088896f;
+  uint32_t phase = 0;                                        // bit s: parity of slot s's next completion
+  Unit cur;
+  int u = blockIdx.x;
+  if (u < units) {
+    find(u, cur);
+    blocks(cur, 0);
+    for (int i = 0; i < min(cur.slices, kSlots); ++i) issue(cur, i, i);
+    fetch_q(cur);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncthreads();
+  bool ok = true;
+  int started = kSlots;                                      // slices of `cur` that are under way already, at most
+  while (u < units) {
+    const int R = p.G * cur.qlen;
+    // ---- queries as A fragments: rows g and g + 8 of each 16-row tile
+    uint32_t qf[MT][D / 16][4];
+    int lim[MT][2], min_limit = 0x7fffffff;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int r = mt * 16 + g + hr * 8, tq = (r * p.g_magic) >> 16;
+        const bool live = r < R;
+        lim[mt][hr] = live ? cur.ctx - cur.qlen + tq + 1 : 0x7fffffff;        // rows past R are never stored
+        min_limit = min(min_limit, lim[mt][hr]);
+        const uint8_t* qrow = s_q + r * C::kQPitch;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          uint32_t a = 0, b = 0;
+          if (live) {
+            if constexpr (FP8) {                             // four neighbouring dims: the order e4m3 fragments come in
+              const uint2 v = *reinterpret_cast<const uint2*>(qrow + ks * 32 + 8 * t);
+              const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+              const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+              a = pack2<true>(f0.x, f0.y);
+              b = pack2<true>(f1.x, f1.y);
+            } else {
+              a = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t);
+              b = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t + 16);
+            }
+          }
+          qf[mt][ks][hr] = a;
+          qf[mt][ks][2 + hr] = b;
+        }
+      }
+    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 4));
+    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 8));
+    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 16));
+
+    float o[MT][D / 8][4], m_run[MT][2], l_run[MT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      m_run[mt][0] = m_run[mt][1] = -INFINITY;
+      l_run[mt][0] = l_run[mt][1] = 0.f;
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[mt][n][i] = 0.f;
+    }
+
+    for (int i = started; i < min(cur.slices, kSlots); ++i) issue(cur, i, i);
+    int slot = 0;
+    for (int i = 0; i < cur.slices; ++i) {
+      ok = ok && mb::mbar_wait(&bars[slot * 4 + warp], (phase >> slot) & 1, p.status, MB_ST_TIMEOUT_TMA);
+      phase ^= 1u << slot;
+      const uint32_t kT = my + slot * 4 * C::kSlot, vT = kT + C::kHalf;
+      const int pos0 = cur.begin + (warp + 4 * i) * kTok;
+      if (pos0 + kTok > cur.ctx) {
+        // rows behind the context hold whatever the block holds: a weight of zero must not meet a NaN there
+        const int from = cur.ctx - pos0;
+        for (int c = lane; c < (kTok - from) * 8 * kSpans; c += 32) {
+          const int r = from + c / (8 * kSpans), cc = c % (8 * kSpans);
+          asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(vT + ((r >> 4) * kSpans + (cc >> 3)) * (kSlice * 128) + (r & 15) * 128 + (cc & 7) * 16),
+                       "r"(0)
+                       : "memory");
+        }
+        __syncwarp();
+      }
+      float s[MT][2 * kSub][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int n = 0; n < 2 * kSub; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[mt][n][e] = 0.f;
+      const int krow = (lane & 7) + ((lane >> 4) << 3), kc = (lane >> 3) & 1, ksw = lane & 7;
+      if constexpr (FP8) {
+#pragma unroll
+        for (int kg = 0; kg < D / 32; ++kg) {
+#pragma unroll
+          for (int b = 0; b < kSub; ++b) {
+            uint32_t r[4];
+            ldsm4(r, kT + (b * kSpans + (kg >> 2)) * (kSlice * 128) + krow * 128 + (((((kg & 3) * 2) + kc) ^ ksw) << 4));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t b00 = e4m3x2(r[h]), b01 = e4m3x2(r[h] >> 16), b10 = e4m3x2(r[2 + h]), b11 = e4m3x2(r[2 + h] >> 16);
+#pragma unroll
+              for (int mt = 0; mt < MT; ++mt) {
+                mma<true>(s[mt][2 * b], qf[mt][kg * 2 + h], b00, b01);
+                mma<true>(s[mt][2 * b + 1], qf[mt][kg * 2 + h], b10, b11);
+              }
+            }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          uint32_t b[4];
+          ldsm4(b, kT + (ks >> 2) * (kSlice * 128) + krow * 128 + (((((ks & 3) * 2) + kc) ^ ksw) << 4));
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            mma<false>(s[mt][0], qf[mt][ks], b[0], b[1]);
+            mma<false>(s[mt][1], qf[mt][ks], b[2], b[3]);
+          }
+        }
+      }
+      // ---- online softmax; the running maximum moves when the new one is more than 2^8 above it
+      const bool mask = pos0 + kTok > min_limit;
+      uint32_t pa[MT][kSub][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+          float v[4 * kSub], mx = -INFINITY;
+#pragma unroll
+          for (int e = 0; e < 4 * kSub; ++e) {
+            v[e] = s[mt][e >> 1][hr * 2 + (e & 1)] * sc_log2;
+            if (mask && pos0 + (e >> 1) * 8 + t * 2 + (e & 1) >= lim[mt][hr]) v[e] = -INFINITY;
+            mx = fmaxf(mx, v[e]);
+          }
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+          if (mx > m_run[mt][hr] + 8.f) {                    // also true on a row's first visible token
+            const float alpha = ex2(m_run[mt][hr] - mx);
+            m_run[mt][hr] = mx;
+            l_run[mt][hr] *= alpha;
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n) {
+              o[mt][n][hr * 2] *= alpha;
+              o[mt][n][hr * 2 + 1] *= alpha;
+            }
+          }
+          const float m_use = m_run[mt][hr] == -INFINITY ? 0.f : m_run[mt][hr];
+#pragma unroll
+          for (int e = 0; e < 4 * kSub; ++e) v[e] = ex2(v[e] - m_use);
+#pragma unroll
+          for (int b = 0; b < kSub; ++b) {
+            l_run[mt][hr] += (v[4 * b] + v[4 * b + 1]) + (v[4 * b + 2] + v[4 * b + 3]);
+            pa[mt][b][hr] = pack2<FP8>(v[4 * b], v[4 * b + 1]);
+            pa[mt][b][2 + hr] = pack2<FP8>(v[4 * b + 2], v[4 * b + 3]);
+          }
+        }
+      }
+      const int vrow = (lane & 7) + (((lane >> 3) & 1) << 3), vc = lane >> 4;
+      if constexpr (FP8) {
+#pragma unroll
+        for (int d2 = 0; d2 < D / 32; ++d2) {
+#pragma unroll
+          for (int b = 0; b < kSub; ++b) {
+          uint32_t r[4];
+          ldsm4t(r, vT + (b * kSpans + (d2 >> 2)) * (kSlice * 128) + vrow * 128 + (((((d2 & 3) * 2) + vc) ^ ksw) << 4));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t e0 = e4m3x2(__byte_perm(r[2 * h], 0, 0x4420)), e1 = e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4420));
+            const uint32_t o0 = e4m3x2(__byte_perm(r[2 * h], 0, 0x4431)), o1 = e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4431));
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+              mma<true>(o[mt][(d2 * 2 + h) * 2], pa[mt][b], e0, e1);        // even dims of the group of 16
+              mma<true>(o[mt][(d2 * 2 + h) * 2 + 1], pa[mt][b], o0, o1);    // odd dims
+            }
+          }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int n2 = 0; n2 < D / 16; ++n2) {
+          uint32_t b[4];
+          ldsm4t(b, vT + (n2 >> 2) * (kSlice * 128) + vrow * 128 + (((((n2 & 3) * 2) + vc) ^ ksw) << 4));
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            mma<false>(o[mt][n2 * 2], pa[mt][0], b[0], b[1]);
+            mma<false>(o[mt][n2 * 2 + 1], pa[mt][0], b[2], b[3]);
+          }
+        }
+      }
+      __syncwarp();                                          // every lane has read the slot
+      const int nx = i + kSlots;
+      if (nx < cur.slices) {
+        if (nx * kSub % 32 == 0) blocks(cur, nx);
+        issue(cur, nx, slot);
+      }
+      slot = slot + 1 == kSlots ? 0 : slot + 1;
+    }
+
+    // ---- the next unit's first slices travel while this one is merged (slots behind `ahead` hold the merge buffer)
+    const int un = u + gridDim.x;
+    Unit next;
+    started = 0;
+    // zeros written behind a context must not be overtaken by the copies that come into the slot next
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (p.over) __syncthreads();                             // no warp writes the merge buffer before all slots are free
+    else __syncwarp();
+    if (un < units) {
+      find(un, next);
+      blocks(next, 0);
+      for (; started < min(next.slices, p.ahead); ++started) issue(next, started, started);
+    }
+    if (!p.over) __syncthreads();                            // every warp has its query fragments: the rows may be replaced
+    if (un < units) fetch_q(next);
+    const int RP = MT * 16;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        const int r = mt * 16 + g + hr * 8;
+        float l = l_run[mt][hr];
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        if (r < R) {
+          if (t == 0) s_ml[warp * RP + r] = make_float2(m_run[mt][hr], l);
+          float* orow = s_o + (warp * R + r) * D;
+          if constexpr (FP8) {
+#pragma unroll
+            for (int dg = 0; dg < D / 16; ++dg)              // even tile (2t, 2t+1) -> dims 4t, 4t+2; odd tile -> 4t+1, 4t+3
+              *reinterpret_cast<float4*>(orow + dg * 16 + 4 * t) =
+                  make_float4(o[mt][dg * 2][hr * 2], o[mt][dg * 2 + 1][hr * 2], o[mt][dg * 2][hr * 2 + 1], o[mt][dg * 2 + 1][hr * 2 + 1]);
+          } else {
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n)
+              *reinterpret_cast<float2*>(orow + n * 8 + t * 2) = make_float2(o[mt][n][hr * 2], o[mt][n][hr * 2 + 1]);
+          }
+        }
+      }
+    __syncthreads();
+    // final values of four dims of row r: the group's head, the token's row, bf16 or a quantised block (four lanes a block of 16)
+    auto store = [&](int r, int c4, float4 a) {
+      const int tq = (r * p.g_magic) >> 16, head = cur.kvh * p.G + r - tq * p.G;
+      const uint32_t m = cur.qs + tq;
+      if (p.outq) {
+        float bmax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
+        bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
+        bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
+        const uint8_t sfc = mb::float_to_e4m3(bmax / (6.f * p.outq_gs));
+        const float sff = mb::e4m3_to_float(sfc);
+        const float qi = sff > 0.f ? __fdividef(1.f, sff * p.outq_gs) : 0.f;
+        const uint32_t w = mb::e2m1x2_pack(a.x * qi, a.y * qi) | (mb::e2m1x2_pack(a.z * qi, a.w * qi) << 8);
+        const int col = head * D + c4 * 4, kb = col >> 4;
+        *reinterpret_cast<uint16_t*>(p.outq + (size_t)m * p.ldq + (col >> 1)) = (uint16_t)w;
+        if ((c4 & 3) == 0) p.outq_sf[((size_t)(m >> 7) * p.outq_sf_k64 + (kb >> 2)) * 512 + mb::sf_tile_offset(m & 127, kb & 3)] = sfc;
+        return;
+      }
+      __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+      *reinterpret_cast<uint2*>(p.out + (size_t)m * p.out_ld + (size_t)head * D + c4 * 4) =
+          make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    };
+    constexpr int kC4 = D / 4;                               // a multiple of 32: whole warps go round together
+    for (int idx = tid; idx < R * kC4; idx += 128) {
+      const int r = idx / kC4, c4 = idx % kC4;
+      float2 ml[4];
+      float mx = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        ml[w] = s_ml[w * RP + r];
+        mx = fmaxf(mx, ml[w].x);
+      }
+      float l = 0.f;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float f = ml[w].x == -INFINITY ? 0.f : ex2(ml[w].x - mx);
+        const float4 ov = *reinterpret_cast<const float4*>(s_o + (w * R + r) * D + c4 * 4);
+        l += ml[w].y * f;
+        acc.x += ov.x * f; acc.y += ov.y * f; acc.z += ov.z * f; acc.w += ov.w * f;
+      }
+      if (cur.nparts == 1) {
+        const float inv = l > 0.f ? vmul / l : 0.f;
+        store(r, c4, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+      } else {                                               // sums as they are, relative to 2^mx
+        const int tq = (r * p.g_magic) >> 16;
+        const size_t row = ((size_t)(cur.qs + tq) * p.Hq + cur.kvh * p.G + r - tq * p.G) * p.parts + cur.part;
+        *reinterpret_cast<float4*>(p.part_o + row * D + c4 * 4) = acc;
+        if (c4 == 0) p.part_ml[row] = make_float2(mx, l);
+      }
+    }
+    if (cur.nparts > 1) {
+      // the last partition of this (sequence, kv head) to arrive sums all of them in order and re-arms the counter
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) {
+        const uint32_t prev = atomicAdd(&p.part_cnt[cur.seq * p.Hkv + cur.kvh], 1u);
+        s_last = prev == (uint32_t)cur.nparts - 1;
+        if (s_last) p.part_cnt[cur.seq * p.Hkv + cur.kvh] = 0;
+      }
+      __syncthreads();
+      if (s_last) {
+        __threadfence();
+        for (int idx = tid; idx < R * kC4; idx += 128) {
+          const int r = idx / kC4, c4 = idx % kC4, tq = (r * p.g_magic) >> 16;
+          const size_t row = ((size_t)(cur.qs + tq) * p.Hq + cur.kvh * p.G + r - tq * p.G) * p.parts;
+          const float* po = p.part_o + row * D + c4 * 4;
+          float mx = -INFINITY, l = 0.f;
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int s0 = 0; s0 < cur.nparts; s0 += 4) {       // four partitions' loads in flight
+            float2 ml[4];
+            float4 ov[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int sx = min(s0 + k, cur.nparts - 1);
+              ml[k] = __ldcg(p.part_ml + row + sx);
+              ov[k] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)sx * D));
+              if (s0 + k >= cur.nparts) ml[k] = make_float2(-INFINITY, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float mn = fmaxf(mx, ml[k].x);
+              const float fa = mx == -INFINITY ? 0.f : ex2(mx - mn), fb = ml[k].x == -INFINITY ? 0.f : ex2(ml[k].x - mn);
+              mx = mn;
+              l = l * fa + ml[k].y * fb;
+              acc.x = acc.x * fa + ov[k].x * fb; acc.y = acc.y * fa + ov[k].y * fb;
+              acc.z = acc.z * fa + ov[k].z * fb; acc.w = acc.w * fa + ov[k].w * fb;
+            }
+          }
+          const float inv = l > 0.f ? vmul / l : 0.f;
+          store(r, c4, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+        }
+      }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the merge buffer's slots are filled by copies again
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    cur = next;
+    u = un;
+  }
+}
+
+int parts_of(int max_ctx, int part) {
+  const int n = (max_ctx + part - 1) / part;
+  return n < 1 ? 1 : n > kMaxParts ? kMaxParts : n;
+}
+// Long partitions pay a unit's fixed instructions less often, short ones fill the chip with fewer sequences; the size is a constant
+// of the model, so that a sequence's sums never depend on its batch. Measured with 256 / 512 / 1024 tokens, us: 8 kv heads, 128
+// sequences of 129 to 1151 tokens 74 / 60 / 50, nine of 4000 to 16000 89 / 73 / 54, one of 700 11.6 / 12.6 / 13.7; 2 kv heads of 256,
+// sixteen sequences of 200 to 2000 28 / 22 / 32.
+int part_tokens_of(const AttnDecodeArgs& a) { return ((a.part_tokens > 0 ? a.part_tokens : a.Hkv >= 8 ? 1024 : 512) + 63) & ~63; }
+
+template <int D, bool FP8, int MT>
+int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
+  using C = DecodeCfg<D, FP8, MT>;
+  auto kern = attn_decode_kernel<D, FP8, MT>;
+  CUtensorMap tm[2];
+  for (int i = 0; i < 2; ++i) {
+    const int rc = mbh::encode_3d(&tm[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, i ? a.v_cache : a.k_cache, C::kRowB, a.Hkv, (uint64_t)a.num_blocks * a.block_size,
+                                  C::kRowB, (uint64_t)a.Hkv * C::kRowB, 128, 1, kSlice);
+    if (rc) return rc;
+  }
+  // the merge buffer lies over the ring's last slots where it fits in front of the next unit's first ones
+  const int rows = a.max_q_len * (a.Hq / a.Hkv), merge = 4 * rows * D * 4;
+  const int behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
+  const bool over = behind < C::kSlots;
+  p.ahead = over ? C::kSlots - behind : C::kSlots;
+  p.over = over;
+  p.merge_off = over ? (uint32_t)(p.ahead * 4 * C::kSlot) : (uint32_t)C::kRing;
+  p.tail_off = over ? (uint32_t)C::kRing : (uint32_t)(C::kRing + merge);
+  p.len_off = (p.tail_off + (uint32_t)(a.num_seqs + 2) * 4 + 4 * MT * 16 * 8 + 8 + 15) & ~15u;
+  const size_t smem = 1024 + (size_t)p.len_off + (size_t)a.num_seqs * 16 + (size_t)rows * C::kQPitch;
+  static size_t configured = 0;
+  if (smem > 220 * 1024) return MB_ERR_TOO_LARGE;
+  if (smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    configured = 220 * 1024;
+  }
+  const int sms = a.sm_count > 0 ? a.sm_count : 148;
+  const long long most = (long long)a.num_seqs * a.Hkv * p.parts;
+  const int grid = most < (long long)sms * C::kCtas ? (int)most : sms * C::kCtas;
+  return (int)mb::launch_kernel(kern, dim3(grid), dim3(128), smem, stream, tm[0], tm[1], p);
+}
+
+}  // namespace
+
+bool mb_attn_decode_serves(const AttnDecodeArgs& a) {
+  const int G = a.Hq / a.Hkv, rows = G * a.max_q_len;
+  const uintptr_t al = reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache);
+  return (a.D == 128 || a.D == 256) && rows <= (a.D == 256 ? 16 : 32) && a.num_seqs <= kMaxSeqs && a.block_size % kSlice == 0 && !(al & 15) &&
+         !(reinterpret_cast<uintptr_t>(a.q) & 15) && a.num_blocks * a.block_size < (1ll << 31) &&
+         (a.outq || (a.out_ld % 4 == 0 && !(reinterpret_cast<uintptr_t>(a.out) & 7)));
+}
+
+size_t mb_attn_decode_ws(const AttnDecodeArgs& a) {
+  const int parts = parts_of(a.max_ctx, part_tokens_of(a));
+  return parts <= 1 ? 0 : kCntBytes + (size_t)a.total_rows * a.Hq * parts * (a.D + 2) * sizeof(float);
+}
+
+int mb_attn_decode(const AttnDecodeArgs& a, cudaStream_t stream) {
+  DecodeParams p{};
+  p.q = a.q; p.block_table = a.block_table; p.max_blocks = a.max_blocks;
+  p.q_start = a.q_start; p.q_len = a.q_len; p.ctx_len = a.ctx_len;
+  p.num_seqs = a.num_seqs; p.Hq = a.Hq; p.Hkv = a.Hkv; p.G = a.Hq / a.Hkv; p.g_magic = (65536 + p.G - 1) / p.G;
+  p.block_size = a.block_size;
+  p.block_shift = (a.block_size & (a.block_size - 1)) == 0 ? 31 - __builtin_clz(a.block_size) : -1;
+  p.num_blocks = a.num_blocks; p.scale = a.scale; p.k_scale = a.k_scale; p.v_scale = a.v_scale;
+  p.out = a.out; p.out_ld = a.out_ld;
+  p.outq = a.outq; p.ldq = a.ldq; p.outq_sf = a.outq_sf; p.outq_sf_k64 = a.outq_sf_k64; p.outq_gs = a.outq_gs;
+  p.status = a.status;
+  p.part_tokens = part_tokens_of(a);
+  p.parts = parts_of(a.max_ctx, p.part_tokens);
+  if (p.parts > 1) {
+    if (!a.ws || a.ws_bytes < mb_attn_decode_ws(a) || (size_t)a.num_seqs * a.Hkv * 4 > kCntBytes) return MB_ERR_TOO_LARGE;
+    p.part_cnt = reinterpret_cast<uint32_t*>(a.ws);
+    p.part_o = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a.ws) + kCntBytes);
+    p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)a.total_rows * a.Hq * p.parts * a.D);
+  }
+  const int mt = a.max_q_len * p.G <= 16 ? 1 : 2;
+  if (a.D == 256) return a.fp8 ? launch<256, true, 1>(a, p, stream) : launch<256, false, 1>(a, p, stream);
+  if (a.fp8) return mt == 1 ? launch<128, true, 1>(a, p, stream) : launch<128, true, 2>(a, p, stream);
+  return mt == 1 ? launch<128, false, 1>(a, p, stream) : launch<128, false, 2>(a, p, stream);
+}
