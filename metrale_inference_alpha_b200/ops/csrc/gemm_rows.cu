@@ -16,11 +16,12 @@
 // under the power cap). The SwiGLU result leaves as NVFP4 from here too: the 134 us quantiser pass over 8192 x 17408 is gone.
 //
 // gemm_block_kernel (fp8 with 128 x 128 weight scales, also over the work list of grouped experts): one CTA per tile of
-// 128 tokens x 128 features. Every 128-deep k block lands in one of four TMEM accumulators and is added to registers
+// 128 tokens x 128 or 256 features. Every 128-deep k block lands in one of four or two TMEM accumulators and is added to registers
 // with its scale, which is one number per thread here (the token's scale times the weight block's). Small work-list entries
 // load boxes of their own 16 to 64 rows: the rest of the tile's rows are whatever was there, and are not stored.
 // Measured (2724 tokens x 8 of 256 experts and a shared one; before = 64-token tiles as the UMMA "B" operand): 1024 x 2048 per
-// expert 500 -> 167 us, 2048 x 512 417 -> 144 us, plain 8192 x 2048 237 -> 82 us; 16 tokens (rows of 16): 52 -> 51, 48 -> 40 us.
+// expert 500 -> 134 us (167 at 128 features a tile), 2048 x 512 417 -> 122 us (144), plain 8192 x 2048 237 -> 64 us (82); 16
+// tokens (rows of 16): 52 -> 49, 48 -> 37 us.
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "gemm_rows.h"
@@ -395,13 +396,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------ fp8, 128 x 128 weight scales
-constexpr int kBlkAccs = 4;
-constexpr int kBlkStageBytes = 2 * 128 * 128;
-constexpr int kBlkStages = 6;
-constexpr int kBlkSmem = kBlkStages * kBlkStageBytes + 1024;
+constexpr int kBlkThreads = 384;   // producer warp, MMA warp, two that wait; eight epilogue warps
 
-__global__ void __launch_bounds__(kThreads, 1)
+template <int BN>
+struct BlkCfg {
+  static constexpr int kAccs = 512 / BN;
+  static constexpr int kStageBytes = 128 * 128 + BN * 128;
+  static constexpr int kStages = BN == 256 ? 4 : 6;
+  static constexpr int kSmem = kStages * kStageBytes + 1024;
+};
+
+template <int BN>
+__global__ void __launch_bounds__(kBlkThreads, 1)
 gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const RowsParams p) {
+  constexpr int kBlkStages = BlkCfg<BN>::kStages, kBlkStageBytes = BlkCfg<BN>::kStageBytes, kBlkAccs = BlkCfg<BN>::kAccs;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full_bar[kBlkStages];
@@ -425,7 +433,7 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     mb::tma_prefetch_desc(&tmA);
     mb::tma_prefetch_desc(&tmB);
   }
-  if (warp == 1) mb::tmem_alloc(&tmem_base_s, 128 * kBlkAccs);
+  if (warp == 1) mb::tmem_alloc(&tmem_base_s, 512);
   mb::tc_fence_before();
   __syncthreads();
   mb::tc_fence_after();
@@ -443,15 +451,18 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (e < 0) return false;
       t.row0 = __ldg(p.tile_row0 + mt);
       t.rows = __ldg(p.tile_nrows + mt);
-      t.w_row0 = e * p.n_per_expert + nt * 128;
+      t.w_row0 = e * p.n_per_expert + nt * BN;
     } else {
       t.row0 = mt * 128;
       t.rows = min(128, p.M - t.row0);
-      t.w_row0 = nt * 128;
+      t.w_row0 = nt * BN;
     }
     return true;
   };
 
+  // BN = 256: 128 sums and 64 fresh columns a thread; the registers come from the four warps that copy and issue
+  if (warp < 4) {
+  if constexpr (BN == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
   if (warp == 0) {
     if (mb::elect_one()) {
       int g = 0;
@@ -464,7 +475,7 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           ok = mb::mbar_wait(&empty_bar[s], ((g / kBlkStages) & 1) ^ 1, p.status, MB_ST_TIMEOUT_TMA);
           if (!ok) break;
           uint8_t* st = smem + s * kBlkStageBytes;
-          mb::mbar_expect_tx(&full_bar[s], p.a_bytes + 128 * 128);
+          mb::mbar_expect_tx(&full_bar[s], p.a_bytes + BN * 128);
           mb::tma_load_2d(st + 128 * 128, &tmB, &full_bar[s], kb * 128, t.w_row0);
           mb::tma_load_2d(st, &tmA, &full_bar[s], kb * 128, t.row0);   // rows past the box keep old bytes: they make rows nobody stores
         }
@@ -473,7 +484,7 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     __syncwarp();
   } else if (warp == 1) {
     if (mb::elect_one()) {
-      const uint32_t idesc = mb::umma_idesc(0, 0, 128, 128);
+      const uint32_t idesc = mb::umma_idesc(0, 0, 128, BN);
       int g = 0;
       bool ok = true;
       for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
@@ -488,16 +499,18 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           const uint32_t a_base = mb::smem_u32(smem + s * kBlkStageBytes), b_base = a_base + 128 * 128;
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            mb::umma_f8f6f4(tmem + buf * 128, mb::umma_desc_sw128(a_base + j * 32), mb::umma_desc_sw128(b_base + j * 32), idesc, j != 0);
+            mb::umma_f8f6f4(tmem + buf * BN, mb::umma_desc_sw128(a_base + j * 32), mb::umma_desc_sw128(b_base + j * 32), idesc, j != 0);
           mb::tc_commit(&empty_bar[s]);
           mb::tc_commit(&acc_full[buf]);
         }
       }
     }
     __syncwarp();
+  }
   } else {
-    constexpr int NC = 64;
-    const int q = warp & 3, half = (warp - 2) >> 2, lane = threadIdx.x & 31;
+    if constexpr (BN == 256) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    constexpr int NC = BN / 2;
+    const int q = warp & 3, half = (warp - 4) >> 2, lane = threadIdx.x & 31;
     const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + half * NC;
     int g = 0;
     bool ok = true;
@@ -507,7 +520,8 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int r = q * 32 + lane;
       const bool live = r < t.rows;
       const float* asp = p.a_scale + t.row0 + r;
-      const float* wsp = p.w_scale + (size_t)(t.w_row0 / 128) * nkb;
+      const int n0 = (i % p.n_tiles) * BN + half * NC;
+      const float* wsp = p.w_scale + (size_t)((t.w_row0 + (n0 < p.N ? half * NC : 0)) / 128) * nkb;   // a half behind the last feature reads the first's
       float acc[NC];
 #pragma unroll
       for (int c = 0; c < NC; ++c) acc[c] = 0.f;
@@ -523,18 +537,22 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         ok = mb::mbar_wait(&acc_full[buf], (g / kBlkAccs) & 1, p.status, MB_ST_TIMEOUT_EPI);
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
         mb::tc_fence_after();
-        float v[NC];
-        mb::tmem_ld32_async(src + buf * 128, v);
-        mb::tmem_ld32_async(src + buf * 128 + 32, v + 32);
-        mb::tmem_ld_wait(v);
-        mb::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mb::mbar_arrive(&acc_empty[buf]);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) acc[c] = fmaf(v[c], sc, acc[c]);
+        for (int c0 = 0; c0 < NC; c0 += 64) {
+          float v[64];
+          mb::tmem_ld32_async(src + buf * BN + c0, v);
+          mb::tmem_ld32_async(src + buf * BN + c0 + 32, v + 32);
+          mb::tmem_ld_wait(v);
+          if (c0 + 64 == NC) {                               // the accumulator is free for the next k block
+            mb::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mb::mbar_arrive(&acc_empty[buf]);
+          }
+#pragma unroll
+          for (int c = 0; c < 64; ++c) acc[c0 + c] = fmaf(v[c], sc, acc[c0 + c]);
+        }
       }
       if (ok && live) {
-        const int n0 = (i % p.n_tiles) * 128 + half * NC;
         const size_t m = (size_t)t.row0 + r;
 #pragma unroll
         for (int c = 0; c < NC; c += 32) {
@@ -551,7 +569,7 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   if (warp == 1) {
     mb::tc_fence_after();
-    mb::tmem_dealloc(tmem, 128 * kBlkAccs);
+    mb::tmem_dealloc(tmem, 512);
   }
 }
 
@@ -566,6 +584,18 @@ int launch_pair(const CUtensorMap* tm, const RowsParams& p, int pairs, cudaStrea
     configured = true;
   }
   return (int)mb::launch_kernel_cluster(kern, dim3(2 * pairs), dim3(kThreads), C::kSmemBytes, stream, 1, tm[0], tm[1], tm[2], tm[3], p);
+}
+
+template <int BN>
+int launch_block(const CUtensorMap* tm, const RowsParams& p, int grid, cudaStream_t stream) {
+  auto kern = gemm_block_kernel<BN>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BlkCfg<BN>::kSmem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  return (int)mb::launch_kernel_cluster(kern, dim3(grid), dim3(kBlkThreads), BlkCfg<BN>::kSmem, stream, 1, tm[0], tm[1], p);
 }
 
 }  // namespace
@@ -598,8 +628,7 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
   p.epi_a = a->epi_a; p.epi_b = a->epi_b; p.epi_n = a->epi_n; p.epi_bias = a->epi_bias;
   p.status = a->status;
   CUtensorMap tm[4];
-  int rc = mbh::encode_2d(&tm[1], dt, a->W, inner, (uint64_t)a->N, row_bytes, box, 128);
-  if (rc) return rc;
+  int rc = 0;
 
   if (kind == KIND_FP8_BLOCK) {
     p.tile_expert = a->tile_expert; p.tile_row0 = a->tile_row0; p.tile_nrows = a->tile_nrows;
@@ -607,19 +636,19 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
     const int box_rows = !a->tile_expert || a->force_tn == 128 ? 128 : tn;
     if (box_rows != 16 && box_rows != 32 && box_rows != 64 && box_rows != 128) return MB_ERR_UNSUPPORTED;
     p.a_bytes = box_rows * 128;
-    p.n_tiles = (p.N + 127) / 128;
     p.m_tiles = a->tile_expert ? a->max_tiles : (a->M + 127) / 128;
+    // 256 features a tile read the token rows half as often (at 128 x 128 the operands of 2700 tokens' experts come from L2 at its
+    // rate); short entries of a work list are bound by the weights' stream and keep the finer tiles
+    auto waves = [&](int bn) { return ((long long)p.m_tiles * ((p.N + bn - 1) / bn) + sms - 1) / sms; };
+    const bool wide = a->tile_expert ? box_rows == 128 : waves(256) * 2.0 <= waves(128) * 1.3;
+    const int bn = wide ? 256 : 128;
+    p.n_tiles = (p.N + bn - 1) / bn;
     if ((rc = mbh::encode_2d(&tm[0], dt, a->X, inner, (uint64_t)a->M, x_pitch, box, (uint32_t)box_rows))) return rc;
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(gemm_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlkSmem);
-      if (e != cudaSuccess) return (int)e;
-      configured = true;
-    }
+    if ((rc = mbh::encode_2d(&tm[1], dt, a->W, inner, (uint64_t)a->N, row_bytes, box, (uint32_t)bn))) return rc;
     const long long items = (long long)p.m_tiles * p.n_tiles;
     if (items > 0x7fffffff) return MB_ERR_TOO_LARGE;
-    return (int)mb::launch_kernel_cluster(gemm_block_kernel, dim3(items < sms ? (int)items : sms), dim3(kThreads), kBlkSmem, stream, 1,
-                                          tm[0], tm[1], p);
+    const int grid = items < sms ? (int)items : sms;
+    return wide ? launch_block<256>(tm, p, grid, stream) : launch_block<128>(tm, p, grid, stream);
   }
 
   if (a->outq) {

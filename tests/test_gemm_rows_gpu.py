@@ -87,7 +87,8 @@ def test_pair_kernel_quantises_the_swiglu_result(fmt, M, N):
     assert (g - exact).norm() <= 1.01 * (v - exact).norm()
 
 
-@pytest.mark.parametrize("M,N,K", [(65, 128, 128), (127, 256, 384), (128, 384, 1024), (129, 136, 1024), (300, 1024, 640), (5000, 256, 256)])
+@pytest.mark.parametrize("M,N,K", [(65, 128, 128), (127, 256, 384), (128, 384, 1024), (129, 136, 1024), (300, 1024, 640), (5000, 256, 256),
+                                   (5000, 2176, 384), (5000, 2100, 256)])       # the last two: 256 features a tile, a last half and a last row block missing
 def test_block_kernel_matches_the_one_tile_kernel_and_the_oracle(M, N, K):
     x, w_cpu, act, w = _operands("fp8_block", M, N, K, 9)
     res = torch.randn(M, N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
