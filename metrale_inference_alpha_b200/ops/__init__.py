@@ -47,8 +47,15 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr()
 
 
+# The current stream's handle without a Stream object around it: a prompt of 333 tokens, 13 launches, took 225 us with one for each
+# launch and 183 without, all of it host time.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch._C._cuda_getDevice())
 
 
 class _Runtime:
@@ -69,6 +76,8 @@ class _Runtime:
 
     @classmethod
     def get(cls, device) -> "_Runtime":
+        if isinstance(device, torch.device) and device.index in cls._inst:
+            return cls._inst[device.index]
         device = torch.device(device)
         idx = device.index if device.index is not None else torch.cuda.current_device()
         if idx not in cls._inst:
