@@ -879,13 +879,14 @@ _PART_LEVER = _ATTN_PART_TOKENS                  # the plain decode kernel has a
 def configure(attn_part_tokens: Optional[int] = None) -> None:
     """Deployment constants of the kernel library. ``attn_part_tokens``: split-KV partition size;
     larger partitions amortise the per-CTA prologue and merge when the batch alone fills the GPU,
-    smaller ones give short batches more CTAs. The environment lever wins over this call."""
+    smaller ones give short batches more CTAs. The environment lever wins over this call. The plain decode
+    kernel (csrc/attention_decode.cu) shares its units out evenly and keeps its own size."""
     global _ATTN_PART_TOKENS
     if attn_part_tokens is not None and "METRALE_ATTN_PART_TOKENS" not in os.environ:
         _ATTN_PART_TOKENS = int(attn_part_tokens)
 
 
-# prefill chunks of >= 128 query rows at head_dim 128 take the tcgen05 / TMEM kernel
+# prefill chunks of >= 128 query rows at head_dim 128 or 256 take the tcgen05 / TMEM kernels
 _ATTN_TC = os.environ.get("METRALE_ATTN_TC", "1") != "0"
 # 1: the V tile is staged as stored and read as an MN-major operand; 0: transposed on the way into shared memory
 _ATTN_TC_VMN = int(os.environ.get("METRALE_ATTN_TC_VMN", "1"))
@@ -896,7 +897,7 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
                     window: int = 0, force_mode: int = 0, part_tokens: int = 0, quant_out: float = 0.0):
     """q [T, Hq, D] bf16 -> [T, Hq, D] bf16. Caches [num_blocks, block, Hkv, D] bf16 or e4m3 bytes.
     `quant_out` > 0: return the output as an NVFP4 `Act` [T, Hq * D] quantised with that calibrated
-    global scale (inside the split-KV kernel for decode-sized steps, else by a row kernel)."""
+    global scale (inside the decode kernels and the plain head_dim 128 prefill kernel, else by a row kernel)."""
     T, Hq, D = q.shape
     prefill = force_mode == 3 or (force_mode == 0 and _ATTN_TC and D in (128, 256) and window == 0 and max_q_len >= 128)
     if quant_out > 0.0:

@@ -12,9 +12,12 @@
 //                                shared memory, partitions merge in a second kernel.
 //                                The partition size is fixed, so the result for one
 //                                sequence never depends on what else is in the batch.
+//                                Plain heads of 128 or 256 without a window, gate, sink or
+//                                soft cap take attention_decode.cu instead.
 //                              * "split-Q" kernel (prefill): a CTA owns 64 query rows of
 //                                one (q head, sequence), 16 per warp, and walks the
-//                                causal range of cached tokens FlashAttention-2 style.
+//                                causal range of cached tokens FlashAttention-2 style;
+//                                q_len >= 128 takes attention_tc.cu or attention_rows.cu.
 // Cache layout (both K and V): [num_blocks, block_size, kv_heads, head_dim].
 // e4m3 cache rows are widened to f16 while being staged into shared memory with an
 // integer bit trick (exact, 2^-8 scale folded into the softmax/output scales); bf16

@@ -25,8 +25,9 @@
 // product with V as two bf16 terms (hi + rest: 16 mantissa bits), for models whose attention weights are
 // 32-bit quantities; the output may be a column range of a wider matrix and takes a constant factor.
 //
-// Serves q_len >= 128 chunks with head_dim 128 or 256, bf16 or e4m3 caches; other
-// shapes stay on the mma.sync kernels in attention.cu, which are also the oracle in the tests.
+// Serves q_len >= 128 chunks with head_dim 128 or 256, bf16 or e4m3 caches, except the plain head_dim 128
+// case, which attention_rows.cu takes; other shapes stay on the mma.sync kernels in attention.cu, which are
+// also the oracle in the tests.
 // Reference behaviour covered: the prefill paged-attention family
 // (kernels/gb10/common/prefill_paged_compute.cuh:3-7,37-41), re-designed for TMEM accumulators.
 #include "common.cuh"

@@ -4,7 +4,8 @@
 // the activation tile is the "B" operand (UMMA N = TN tokens, 16..256), so decode
 // batches of 1..128 tokens waste no tensor work and each CTA streams a
 // [128 x K] slab of weights exactly once through a TMA -> shared -> tcgen05.mma
-// pipeline with the fp32 accumulator in TMEM.
+// pipeline with the fp32 accumulator in TMEM. More than 128 tokens, and fp8 blocks
+// of more than 64, take the kernels of gemm_rows.cu.
 //
 // Operand kinds
 //   KIND_BF16   W, X bf16                    tcgen05.mma kind::f16
