@@ -29,7 +29,7 @@ OUT_MODE = {"bf16": 0, "fp8_row": 1, "fp8_g128": 2, "nvfp4": 3}
 launch_count = 0  # kernels launched through this module (bench.py reports it)
 # kernel-selection bits of the GEMM launcher (csrc/gemm_args.h)
 GEMM_ONE_TILE_PER_CTA, GEMM_DECODE_TILE_ORDER, GEMM_PERSISTENT_PREFILL, GEMM_DSMEM_SPLITK = 16, 64, 128, 256
-# GEMMs of more than 128 token rows run on the persistent kernel of CTA pairs (csrc/gemm_rows.cu; METRALE_PERSISTENT_PREFILL=0
+# GEMMs of more than 128 token rows (bf16: 256) run on the persistent kernel of CTA pairs (csrc/gemm_rows.cu; METRALE_PERSISTENT_PREFILL=0
 # keeps one tile per CTA)
 _PERSIST_PREFILL = GEMM_PERSISTENT_PREFILL if os.environ.get("METRALE_PERSISTENT_PREFILL", "1") != "0" else 0
 GEMM_GROUPED_ONE_CTA = 512

@@ -606,6 +606,10 @@ bool mb_gemm_rows_serves(const MbGemmArgs* a) {
     if (a->epilogue != mb::EPI_PLAIN || a->outq) return false;
     return a->tile_expert ? true : a->force_tn == 0 && a->M > 64;
   }
+  // bf16 of one token tile is bound by the weights' stream, which 74 pairs pull slower than 148 CTAs (or splits of K) do: two dense
+  // layers of 5120 at 144 / 200 / 256 tokens 537 / 546 / 552 us here, 505 / 515 / 529 a tile per CTA; at 300 tokens 713 against 869.
+  // NVFP4 weights are a quarter of the bytes: 159 / 161 / 165 here against 178 / 187 / 187.
+  if (a->kind == KIND_BF16 && a->M <= 256 && !a->outq) return false;
   return !a->tile_expert && a->force_tn == 0 && a->M > 128 && (a->flags & MB_GEMM_PERSISTENT_PREFILL);
 }
 

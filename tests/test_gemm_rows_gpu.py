@@ -29,9 +29,10 @@ def _oracle(x, w, fmt):
 def test_pair_kernel_matches_the_one_tile_kernel_and_the_oracle(fmt, M, N, K):
     x, w_cpu, act, w = _operands(fmt, M, N, K)
     res = torch.randn(M, N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
-    assert torch.equal(ops.linear(act, w, residual=res), ops.linear(act, w, residual=res, one_tile_per_cta=True, force_splits=1))
     got = ops.linear(act, w, out_f32=True)
-    assert torch.equal(got, ops.linear(act, w, out_f32=True, one_tile_per_cta=True, force_splits=1))
+    if fmt != "bf16" or M > 256:                           # bf16 of one token tile stays with a tile per CTA, in splits of K
+        assert torch.equal(ops.linear(act, w, residual=res), ops.linear(act, w, residual=res, one_tile_per_cta=True, force_splits=1))
+        assert torch.equal(got, ops.linear(act, w, out_f32=True, one_tile_per_cta=True, force_splits=1))
     ops.check_status(DEV)
     # fp32 sums of K products of the encoded operands: K ulps of the largest partial sum, far below this
     want = _oracle(x, w_cpu, fmt)
