@@ -342,10 +342,6 @@ class ModelRunner:
         todo = [f for f in ffns if f.down_in_scale <= 0.0]
         todo_a = [m for m in attns if m.o_in_scale <= 0.0]
         if not todo and not todo_a:
-            for f in ffns:
-                ops.static_scale_vec(self.device, f.down_in_scale, 256)
-            for m in attns:
-                ops.static_scale_vec(self.device, m.o_in_scale, 256)
             return 0
         tokens = min(tokens, self.sched.max_prefill_tokens, self.sched.max_model_len - 1)
         g = torch.Generator().manual_seed(seed)
@@ -376,12 +372,6 @@ class ModelRunner:
                 amax = float(calib[id(m)])
                 if amax > 0.0:
                     m.o_in_scale = margin * amax / (6.0 * 448.0)
-        for f in ffns:
-            if f.down_in_scale > 0.0:
-                ops.static_scale_vec(self.device, f.down_in_scale, 256)
-        for m in attns:
-            if m.o_in_scale > 0.0:
-                ops.static_scale_vec(self.device, m.o_in_scale, 256)
         return n
 
     def _adapter_rows(self, plan: StepPlan) -> Optional[torch.Tensor]:

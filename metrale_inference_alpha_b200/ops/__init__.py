@@ -209,10 +209,25 @@ class Act:
     M: int
     K: int
     data: torch.Tensor                      # bf16 [M,K] | u8 [M,K] | u8 [M,K/2]; CPU: fp32 dequantised
-    scale: Optional[torch.Tensor] = None    # fp8_row / nvfp4: [M]; fp8_g128: [K/128, ld]
+    scale: Optional[torch.Tensor] = None    # fp8_row / nvfp4: [M]; fp8_g128: [K/128, ld]. Made on request where `static_scale` is set
     sf: Optional[torch.Tensor] = None       # nvfp4 tiled scale factors (CUDA)
     sf_k64: int = 0
     bf16: Optional[torch.Tensor] = None     # extra bf16 copy when requested
+    static_scale: float = 0.0               # nvfp4, > 0: one calibrated scale for all rows. GEMMs take it as a number: a captured graph
+                                            # then holds no address of it
+
+
+def _act_scale(self: Act) -> Optional[torch.Tensor]:
+    if self._scale is None and self.static_scale > 0.0:
+        return torch.full((self.M,), self.static_scale, dtype=torch.float32, device=self.data.device)
+    return self._scale
+
+
+def _set_act_scale(self: Act, scale: Optional[torch.Tensor]) -> None:
+    self._scale = scale
+
+
+Act.scale = property(_act_scale, _set_act_scale)
 
 
 _SF_ZERO: dict = {}
@@ -556,7 +571,10 @@ def linear(act: Act, w: QuantWeight, *, residual: Optional[torch.Tensor] = None,
             w.prepare_cuda()
         a.sfa, a.sfb, a.sf_k64 = _ptr(w.sf_tiled), _ptr(act.sf), w.sf_k64
         assert act.sf_k64 == w.sf_k64
-        a.a_scale = _ptr(act.scale)
+        if act.static_scale > 0.0:
+            a.a_static = act.static_scale
+        else:
+            a.a_scale = _ptr(act.scale)
         a.w_scale = _ptr(w.row_gscale)
         a.alpha = w.gscale
     a.epilogue, a.out_f32 = int(swiglu), int(out_f32)
@@ -584,10 +602,9 @@ def linear(act: Act, w: QuantWeight, *, residual: Optional[torch.Tensor] = None,
     qact = None
     if quant_out > 0.0:
         Kq, dev = N // 2, act.data.device
-        qact = Act("nvfp4", M, Kq, torch.empty(M, Kq // 2, dtype=torch.uint8, device=dev))
+        qact = Act("nvfp4", M, Kq, torch.empty(M, Kq // 2, dtype=torch.uint8, device=dev), static_scale=quant_out)
         qact.sf_k64 = Kq // 64
         qact.sf = torch.empty(((M + 127) // 128) * qact.sf_k64 * 512, dtype=torch.uint8, device=dev)
-        qact.scale = static_scale_vec(dev, quant_out, M)
         a.out = _ptr(qact.data)                              # the bf16 output does not exist in this mode
         a.outq, a.ldq, a.outq_sf, a.outq_sf_k64, a.outq_gs = _ptr(qact.data), Kq // 2, _ptr(qact.sf), qact.sf_k64, quant_out
     if grouped is not None:
@@ -597,24 +614,6 @@ def linear(act: Act, w: QuantWeight, *, residual: Optional[torch.Tensor] = None,
     _native.check(L.mb_gemm(C.byref(a), _stream()), f"gemm[{w.fmt} M={M} N={N} K={w.K}]")
     _count()
     return qact if qact is not None else out
-
-
-_SCALE_VECS: dict = {}
-
-
-def static_scale_vec(device, gs: float, M: int) -> torch.Tensor:
-    """[M] fp32 filled with a static activation scale (the per-token scale array the W4A4 GEMM
-    epilogue reads). Vectors are created once per (device, scale), outside any stream capture:
-    the engine calls this at calibration time; a miss during capture allocates without caching."""
-    key = (str(device), float(gs))
-    t = _SCALE_VECS.get(key)
-    if t is None or t.numel() < M:
-        n = max(256, M)
-        t = torch.full((n,), float(gs), dtype=torch.float32, device=device)
-        if torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing():
-            return t[:M]
-        _SCALE_VECS[key] = t
-    return t[:M]
 
 
 def concat_weights(ws) -> QuantWeight:
@@ -924,9 +923,8 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     qact = None
     if quant_out > 0.0:
         Kq = Hq * D
-        qact = Act("nvfp4", T, Kq, torch.empty(T, Kq // 2, dtype=torch.uint8, device=q.device))
+        qact = Act("nvfp4", T, Kq, torch.empty(T, Kq // 2, dtype=torch.uint8, device=q.device), static_scale=quant_out)
         qact.sf, qact.sf_k64 = _sf_buffer(q.device, T, Kq)
-        qact.scale = static_scale_vec(q.device, quant_out, T)
     if force_mode == 0 and G * max_q_len <= 32 and D == 256 and G * max_q_len > 16:
         # two row tiles do not fit the register file at head_dim 256: present every query
         # token as its own single-row sequence (causality then comes from ctx_len alone)

@@ -52,6 +52,7 @@ struct MbGemmArgs {
   int epi_n;
   const float* epi_bias;
   long long ldx;            // elements between the rows of X (0 = K); bf16 operands
+  float a_static;           // fp8 per row, NVFP4: the activation scale of every token where a_scale is null (0 = 1)
 };
 
 extern "C" int mb_gemm(const MbGemmArgs* args, cudaStream_t stream);

@@ -38,6 +38,7 @@ struct RowsParams {
   const __nv_bfloat16* residual;
   const float* w_scale;      // per feature or null; fp8 block: [features / 128, k blocks]
   const float* a_scale;      // per token or null; fp8 block: [k blocks, a_ld]
+  float a_static;            // every token's scale where a_scale is null (not fp8 block)
   int a_ld;
   float alpha;
   int epilogue, out_f32, vec;   // vec: rows of `out` (and `residual`) are whole 16-byte vectors
@@ -371,7 +372,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     for (int it = 0; it < my_tiles && ok; ++it) {
       const int t = pair + it * pairs, mt = t % p.m_tiles, nt = t / p.m_tiles, buf = it % C::kAccs;
       const int m = (mt * 2 + (int)rank) * 128 + q * 32 + lane;
-      float as = 1.f;
+      float as = KIND == KIND_BF16 ? 1.f : p.a_static;
       if (KIND != KIND_BF16 && p.a_scale && m < p.M) as = __ldg(p.a_scale + m);
       ok = mb::mbar_wait(&acc_full[buf], (it / C::kAccs) & 1, p.status, MB_ST_TIMEOUT_EPI);
       if (!__all_sync(0xffffffffu, ok)) break;
@@ -627,6 +628,7 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
   p.M = a->M; p.N = a->tile_expert ? a->n_per_expert : a->N; p.num_kb = (a->K + kelems - 1) / kelems;
   p.ldo = a->ldo; p.out = a->out; p.residual = reinterpret_cast<const __nv_bfloat16*>(a->residual);
   p.w_scale = a->w_scale; p.a_scale = a->a_scale; p.a_ld = a->a_ld; p.alpha = a->alpha;
+  p.a_static = a->a_static != 0.f ? a->a_static : 1.f;
   p.epilogue = a->epilogue; p.out_f32 = a->out_f32;
   p.vec = a->ldo % 8 == 0 && ((reinterpret_cast<uintptr_t>(a->out) | reinterpret_cast<uintptr_t>(a->residual)) & 15) == 0;
   p.epi_a = a->epi_a; p.epi_b = a->epi_b; p.epi_n = a->epi_n; p.epi_bias = a->epi_bias;

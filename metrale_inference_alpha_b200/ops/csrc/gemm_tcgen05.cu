@@ -61,6 +61,7 @@ struct GemmParams {
   const __nv_bfloat16* residual;
   const float* w_scale;   // KIND_FP8: [N]; KIND_NVFP4: optional per-row global scale [N]; KIND_FP8_BLOCK: [ceil(N/128), ceil(K/128)]
   const float* a_scale;   // KIND_FP8 / NVFP4: [M] or null; KIND_FP8_BLOCK: [ceil(K/128), a_ld]
+  float a_static;         // KIND_FP8 / NVFP4: every token's scale where a_scale is null
   int a_ld;
   float alpha;
   const uint8_t* sfa;     // NVFP4 tiled scale factors of W: [ceil(N/128)][k64 groups][512]
@@ -332,7 +333,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     for (int j = et; j < TN; j += 128) {
       float sc = 1.f;
       if constexpr (KIND == KIND_FP8 || KIND == KIND_NVFP4) {
-        if (p.a_scale && m0 + j < m_end) sc = __ldg(&p.a_scale[m0 + j]);
+        if (!p.a_scale) sc = p.a_static;
+        else if (m0 + j < m_end) sc = __ldg(&p.a_scale[m0 + j]);
       }
       s_ascale[j] = sc;
     }
@@ -835,7 +837,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         for (int j = et; j < TN; j += kPersistThreads - 64) {
           float sc = 1.f;
           if constexpr (KIND == KIND_FP8 || KIND == KIND_NVFP4) {
-            if (p.a_scale && j < m_valid) sc = __ldg(&p.a_scale[j]);
+            if (!p.a_scale) sc = p.a_static;
+            else if (j < m_valid) sc = __ldg(&p.a_scale[j]);
           }
           s_ascale[j] = sc;
         }
@@ -1089,7 +1092,7 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
   p.M = a->M; p.N = a->N; p.K = a->K; p.ldo = a->ldo;
   p.out = a->out;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a->residual);
-  p.w_scale = a->w_scale; p.a_scale = a->a_scale; p.a_ld = a->a_ld;
+  p.w_scale = a->w_scale; p.a_scale = a->a_scale; p.a_ld = a->a_ld; p.a_static = a->a_static != 0.f ? a->a_static : 1.f;
   p.alpha = a->alpha;
   p.sfa = reinterpret_cast<const uint8_t*>(a->sfa);
   p.sfb = reinterpret_cast<const uint8_t*>(a->sfb);

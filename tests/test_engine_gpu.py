@@ -93,6 +93,27 @@ def _tiny_family(name):
     raise KeyError(name)
 
 
+def test_decode_graphs_outlive_longer_prompts():
+    """A decode graph captured behind a short prompt reads the calibrated activation scales of the o and down projections.
+    Prompts longer than any before it, which quantise with the same scales, and later allocations must not move them."""
+    cfg = preset("dense-27b-nvfp4", num_layers=2, hidden_size=1024, num_heads=8, num_kv_heads=2,
+                 intermediate_size=64 * 160, vocab_size=8192, mtp_layers=0, max_position=2048)
+    p = lambda n: [(7 * j + n) % 8000 + 1 for j in range(n)]
+    outs = {}
+    for graphs in (False, True):
+        eng = LLMEngine(EngineArgs(model=cfg, device="cuda", max_num_seqs=8, max_model_len=2048, num_kv_blocks=512,
+                                   use_cuda_graphs=graphs, enable_prefix_caching=False))
+        assert all(lw.ffn.down_in_scale > 0 and lw.mixer.o_in_scale > 0 for lw in eng.weights.layers)
+        first = _drive(eng, {0: [(p(20), 16)]})
+        longer = _drive(eng, {0: [(p(300), 8)]}) + _drive(eng, {0: [(p(1500), 8)]})
+        held = [torch.full((n,), 1e3, device="cuda") for n in (64, 256, 300, 512, 1500, 2048, 4096) for _ in range(64)]
+        again = _drive(eng, {0: [(p(20), 16)]})
+        assert again == first
+        outs[graphs] = first + longer
+        del held
+    assert outs[True] == outs[False]
+
+
 @pytest.mark.parametrize("family", ["hybrid-moe", "nemotron-h", "deepseek-mla"])
 def test_other_architecture_families_run_on_the_gpu_and_graphs_equal_eager(family):
     """Tiny instances of the hybrid GDN + MoE, Mamba2 hybrid and MLA + MoE families: prefill, ragged

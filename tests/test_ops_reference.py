@@ -177,3 +177,15 @@ def test_rope_scaling_tables_match_transformers():
     cos, sin = ref.rope_tables(64, 128, 1e6, scaling={"rope_type": "linear", "factor": 2.0})
     c0, s0 = ref.rope_tables(64, 128, 1e6)
     assert torch.allclose(cos[2 * 7], c0[7], atol=1e-6) and torch.allclose(sin[2 * 7], s0[7], atol=1e-6)
+
+
+def test_a_calibrated_activation_scale_is_a_number_that_reads_as_a_vector():
+    """The GEMM takes it by value, so that a captured graph holds no address of it; whoever asks for the scales gets them."""
+    from metrale_inference_alpha_b200 import ops
+    from metrale_inference_alpha_b200.ops import _native
+    act = ops.Act("nvfp4", 300, 64, torch.zeros(300, 32, dtype=torch.uint8), static_scale=0.375)
+    assert act.scale.dtype == torch.float32 and act.scale.tolist() == [0.375] * 300 and act.scale.is_contiguous()
+    assert ops.Act("nvfp4", 3, 64, act.data).scale is None
+    own = torch.ones(3)
+    assert ops.Act("nvfp4", 3, 64, act.data, own).scale is own
+    assert _native.GemmArgs().a_static == 0.0          # C callers that leave it out keep a scale of one
