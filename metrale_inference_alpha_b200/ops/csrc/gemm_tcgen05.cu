@@ -1067,6 +1067,8 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
   if (kind == KIND_FP8_BLOCK && !grouped && a->a_ld < tiles_m * tn) return MB_ERR_BAD_ARG;
   if (kind == KIND_FP8_BLOCK && grouped && a->a_ld < a->M + tn) return MB_ERR_BAD_ARG;
   if (mb_gemm_rows_serves(a)) return mb_gemm_rows(a, tn, stream);
+  // a work list whose entries may hold more rows than the tile takes: rows behind the tile would be left unwritten
+  if (grouped && a->force_tn > tn) return MB_ERR_UNSUPPORTED;
   // scale-factor tiles are 128 rows: several token tiles only line up at TN = 128
   if (kind == KIND_NVFP4 && !grouped && tiles_m > 1 && tn != 128) return MB_ERR_BAD_ARG;
   const int tiles = tiles_n * tiles_m;

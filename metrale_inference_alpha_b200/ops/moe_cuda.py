@@ -158,8 +158,8 @@ def grouped_pairs(cfg, a: Act, idx: torch.Tensor, w):
         return gemm_simt(h, ge.down.data, y, grouped=g(ge.n_down)), sp
     nvfp4 = ge.gate_up.fmt == "nvfp4"
     # NVFP4: every token tile starts on a 128-row block of scale factors and takes its first tile_rows rows; fp8 blocks: rows
-    # of the 128 x 128 tiles of csrc/gemm_rows.cu
-    tall = nvfp4 or ge.gate_up.fmt == ge.down.fmt == "fp8_block"
+    # of the 128 x 128 tiles of csrc/gemm_rows.cu. The other formats take at most 64 rows an entry (and refuse more).
+    tall = ge.down.fmt in ("nvfp4", "fp8_block") and (nvfp4 or ge.gate_up.fmt == ge.down.fmt)
     tile_rows = 16 if per_expert <= 16 else (32 if per_expert <= 32 else (64 if per_expert <= 64 or not tall else 128))
     sp = SortedPairs(idx, w.expert_lo, ge.num, tile_rows, align=128 if nvfp4 else 1)
     xa = gather_act(a, sp)

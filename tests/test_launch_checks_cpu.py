@@ -1,0 +1,33 @@
+"""What the launchers refuse before they touch a device, called through the library's C entry points."""
+import ctypes as C
+
+import pytest
+import torch
+
+from metrale_inference_alpha_b200 import ops
+from metrale_inference_alpha_b200.ops import _native
+
+BAD_ARG, UNSUPPORTED = -1, -2
+
+
+@pytest.fixture(scope="module")
+def lib():
+    if not _native.LIB_PATH.exists():
+        pytest.skip("kernel library not built")
+    L = C.CDLL(str(_native.LIB_PATH))
+    L.mb_gemm.argtypes, L.mb_gemm.restype = [C.POINTER(_native.GemmArgs), C.c_void_p], C.c_int
+    return L
+
+
+@pytest.mark.parametrize("fmt,rows", [("bf16", 128), ("fp8_row", 128), ("fp8_block", 128)])
+@pytest.mark.parametrize("flags,no_cluster,epilogue", [(ops.GEMM_ONE_TILE_PER_CTA, 0, 0), (ops.GEMM_DECODE_TILE_ORDER, 0, 0), (0, 1, 0),
+                                                       (0, 0, ops.EPI_SWIGLU)])
+def test_a_work_list_entry_has_no_more_rows_than_the_tile(lib, fmt, rows, flags, no_cluster, epilogue):
+    buf = torch.zeros(1 << 20, dtype=torch.uint8)
+    p = buf.data_ptr()
+    a = _native.GemmArgs()
+    a.kind, a.M, a.N, a.K, a.ldo, a.a_ld = ops.KIND[fmt], 512, 1024, 128, 256, 512 + rows
+    a.W = a.X = a.out = a.w_scale = a.a_scale = a.tile_expert = a.tile_row0 = a.tile_nrows = p
+    a.alpha, a.n_per_expert, a.max_tiles, a.force_tn, a.sm_count = 1.0, 256, 8, rows, 148
+    a.flags, a.no_cluster, a.epilogue = flags | ops.GEMM_PERSISTENT_PREFILL, no_cluster, epilogue
+    assert lib.mb_gemm(C.byref(a), None) == UNSUPPORTED
