@@ -2,7 +2,9 @@
 #pragma once
 #include "gemm_args.h"
 
-// Whether gemm_rows.cu serves this call. `splits_forced`: the caller asked for a split-K count.
+// Ranges of K that a GEMM of one tile per CTA (gemm_tcgen05.cu) is cut into when the caller names no number.
+extern "C" int mb_gemm_auto_splits(int tiles, int num_kb, int sms, bool clusters);
+// Whether gemm_rows.cu serves this call.
 bool mb_gemm_rows_serves(const MbGemmArgs* a);
 // `tn`: mb_gemm's token tile, for grouped calls the most rows of an entry of the work list
 int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream);

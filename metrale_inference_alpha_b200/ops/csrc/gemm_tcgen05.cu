@@ -1016,6 +1016,24 @@ extern "C" {
 size_t mb_gemm_counter_bytes() { return 64 * 1024; }
 
 
+int mb_gemm_auto_splits(int tiles, int num_kb, int sms, bool clusters) {
+  if (tiles >= sms) return 1;
+  int splits = sms / tiles;
+  if (clusters) {
+    // A cluster of at most eight finishes a tile together; more leave the whole sum to the last CTA to arrive. bf16 of 128 / 640 /
+    // 896 / 1280 x 5120: 128 tokens, 8 splits 16 / 16 / 16 / 18 us, uncapped (20 / 20 / 20 / 14) 51 / 53 / 55 / 47; one token 12 to 14
+    // against 14 to 17; fp8 and NVFP4 (17408 deep) alike.
+    // And no more clusters than the chip holds at once, or the last ones run as a second wave. A cluster lives in one GPC, so
+    // fewer CTAs fit than SMs: clusters of 2 to 8 CTAs that a B200 holds at one CTA per SM. 16 tiles of bf16, K = 5120, 1 / 16 /
+    // 128 tokens: 8 splits 19 / 20 / 28 us, 6 splits 15 / 16 / 20; 24 tiles: 6 splits 22 / 23 / 33, 5 splits 18 / 19 / 23.
+    constexpr int kResident[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    if (splits > 8) splits = 8;
+    while (splits > 1 && tiles > kResident[splits]) --splits;
+  }
+  const int max_by_k = num_kb / 4 > 0 ? num_kb / 4 : 1;
+  return splits > max_by_k ? max_by_k : splits;
+}
+
 int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
   if (!a || !a->W || !a->X || !a->out || a->M <= 0 || a->N <= 0 || a->K <= 0) return MB_ERR_BAD_ARG;
   const int kind = a->kind;
@@ -1074,18 +1092,7 @@ int mb_gemm(const MbGemmArgs* a, cudaStream_t stream) {
   const int tiles = tiles_n * tiles_m;
   const int sms = a->sm_count > 0 ? a->sm_count : 148;
   int splits = a->force_splits;
-  if (splits <= 0) {
-    splits = 1;
-    if (tiles < sms && a->ws) {
-      splits = sms / tiles;
-      // a cluster of at most eight finishes a tile together; more than eight leave the whole sum to the last one to arrive
-      // (2048 x 5120 bf16, 128 tokens: nine splits 41 us, eight 23)
-      if (splits > 8 && !a->no_cluster) splits = 8;
-      const int max_by_k = num_kb / 4 > 0 ? num_kb / 4 : 1;
-      if (splits > max_by_k) splits = max_by_k;
-      if (splits < 1) splits = 1;
-    }
-  }
+  if (splits <= 0) splits = a->ws ? mb_gemm_auto_splits(tiles, num_kb, sms, !a->no_cluster) : 1;
   if (splits > num_kb) splits = num_kb;
   int kb_per = (num_kb + splits - 1) / splits;
   splits = (num_kb + kb_per - 1) / kb_per;              // no empty split

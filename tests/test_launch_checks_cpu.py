@@ -31,3 +31,15 @@ def test_a_work_list_entry_has_no_more_rows_than_the_tile(lib, fmt, rows, flags,
     a.alpha, a.n_per_expert, a.max_tiles, a.force_tn, a.sm_count = 1.0, 256, 8, rows, 148
     a.flags, a.no_cluster, a.epilogue = flags | ops.GEMM_PERSISTENT_PREFILL, no_cluster, epilogue
     assert lib.mb_gemm(C.byref(a), None) == UNSUPPORTED
+
+
+def test_splits_of_k_keep_their_clusters_resident(lib):
+    """No cluster beyond what the chip holds at once (measured: 74, 45, 33, 26, 22, 15, 15 of 2 to 8 CTAs), no split without four k blocks."""
+    lib.mb_gemm_auto_splits.argtypes, lib.mb_gemm_auto_splits.restype = [C.c_int, C.c_int, C.c_int, C.c_bool], C.c_int
+    held = {1: 148, 2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 7: 15, 8: 15}
+    for tiles in range(1, 200):
+        for num_kb in (1, 4, 11, 20, 80):
+            s = lib.mb_gemm_auto_splits(tiles, num_kb, 148, True)
+            want = max((n for n in held if tiles <= held[n] and n * tiles <= 148 and (n == 1 or 4 * n <= num_kb)), default=1)
+            assert s == want, (tiles, num_kb)
+            assert lib.mb_gemm_auto_splits(tiles, num_kb, 148, False) == max(1, min(148 // tiles, num_kb // 4))
