@@ -26,6 +26,7 @@
 #include "epilogue.cuh"
 #include "gemm_rows.h"
 #include "tensormap.h"
+#include <type_traits>
 
 namespace {
 
@@ -72,7 +73,7 @@ __device__ __forceinline__ void store_bf16x8(__nv_bfloat16* dst, const float* y)
 // 8 results of one token at feature n (of n_limit): residual and store
 __device__ __forceinline__ void emit8(const RowsParams& p, size_t m, int n, int n_limit, float* y, const uint4& res) {
   const size_t o = m * (size_t)p.ldo + n;
-  if (p.vec && n + 8 <= n_limit) {
+  if (n + 8 <= n_limit) {
     if (p.residual) {
       const __nv_bfloat162* rb = reinterpret_cast<const __nv_bfloat162*>(&res);
 #pragma unroll
@@ -101,13 +102,82 @@ __device__ __forceinline__ void emit8(const RowsParams& p, size_t m, int n, int 
   }
 }
 
+// Rows that are not whole vectors start anywhere in one: a thread moves its features up by what its row lacks to the next 16-byte
+// boundary, one step per bit of that, and stores whole vectors between single elements at both ends. With single stores throughout
+// (32 lines a store, 64 or 128 of them a tile) NVFP4 rows of 4099 features, 5120 deep, took 78 us at 1300 tokens and 377 at 8192,
+// fp8 blocks of 257 by 7168 54 us at 300 tokens; now 31, 103 and 39.
+template <int NC, bool F32>
+__device__ __forceinline__ void emit_shifted(const RowsParams& p, size_t m, int n0, int left, float* v) {
+  using T = std::conditional_t<F32, float, __nv_bfloat16>;
+  constexpr int kPer = F32 ? 1 : 2, kWords = NC / kPer, kVec = 4 * kPer;      // elements of a word, words, elements of a vector
+  left = min(left, NC);
+  const size_t o = m * (size_t)p.ldo + n0;
+  if (p.residual) {
+#pragma unroll
+    for (int i = 0; i < NC; ++i) v[i] += i < left ? __bfloat162float(p.residual[o + i]) : 0.f;
+  }
+  uint32_t w[kWords];
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) {
+    if constexpr (F32) {
+      w[i] = __float_as_uint(v[i]);
+    } else {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+  }
+  T* dst = reinterpret_cast<T*>(p.out) + o;
+  auto single = [&](int i) {                                 // element i of the words as they stand
+    if constexpr (F32) dst[i] = __uint_as_float(w[i]);
+    else reinterpret_cast<uint16_t*>(dst)[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+  };
+  const int lead = (int)((0u - (uint32_t)(reinterpret_cast<uintptr_t>(dst) / sizeof(T))) & (kVec - 1));
+#pragma unroll
+  for (int i = 0; i < kVec - 1; ++i)
+    if (i < lead && i < left) single(i);
+  if constexpr (!F32) {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = lead & 1 ? __byte_perm(w[i], i + 1 < kWords ? w[i + 1] : 0, 0x5432) : w[i];
+  }
+  const int up = lead / kPer;
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) w[i] = up & 1 ? (i + 1 < kWords ? w[i + 1] : 0) : w[i];
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) w[i] = up & 2 ? (i + 2 < kWords ? w[i + 2] : 0) : w[i];
+  dst += lead;
+  if (left == NC) {
+#pragma unroll
+    for (int k = 0; k < NC / kVec - 1; ++k, dst += kVec) *reinterpret_cast<uint4*>(dst) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = w[kWords - 4 + i];
+    left = kVec;
+  }
+#pragma unroll 1
+  for (left -= lead; left > 0; left -= kVec, dst += kVec) {
+    if (left >= kVec) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+    for (int i = 0; i < kVec - 1; ++i)
+      if (left < kVec && i < left) single(i);
+#pragma unroll
+    for (int i = 0; i < kWords - 4; ++i) w[i] = w[i + 4];
+  }
+}
+
+template <int NC>
+__device__ __forceinline__ void emit_ragged(const RowsParams& p, size_t m, int n0, int n_limit, float* v) {
+  if (n0 >= n_limit) return;
+  if (p.out_f32) emit_shifted<NC, true>(p, m, n0, n_limit - n0, v);
+  else emit_shifted<NC, false>(p, m, n0, n_limit - n0, v);
+}
+
 __device__ __forceinline__ uint4 residual8(const RowsParams& p, size_t m, int n, int n_limit) {
-  if (p.residual && p.vec && n + 8 <= n_limit) return __ldg(reinterpret_cast<const uint4*>(p.residual + m * (size_t)p.ldo + n));
+  if (p.residual && n + 8 <= n_limit) return __ldg(reinterpret_cast<const uint4*>(p.residual + m * (size_t)p.ldo + n));
   return make_uint4(0, 0, 0, 0);
 }
 
-// One token's NC features from n0 on, accumulator values in v.
-template <int KIND, int NC>
+// One token's NC features from n0 on, accumulator values in v. VEC: rows are whole vectors (a kernel of its own for other rows: their
+// code in the same one cost NVFP4 prompts 3 %).
+template <int KIND, int NC, bool VEC>
 __device__ __forceinline__ void finish_row(const RowsParams& p, float (&v)[NC], int m, int n0, float as) {
   const bool glu = p.epilogue == mb::EPI_SWIGLU || (KIND == KIND_BF16 && (p.epilogue == mb::EPI_CLAMP_GLU || p.epilogue == mb::EPI_GEGLU));
   constexpr bool kWScale = KIND == KIND_FP8 || KIND == KIND_NVFP4;
@@ -170,6 +240,7 @@ __device__ __forceinline__ void finish_row(const RowsParams& p, float (&v)[NC], 
       return;
     }
     if (m >= p.M) return;
+    if constexpr (!VEC) return emit_ragged<NC / 2>(p, (size_t)m, n0 / 2, p.N / 2, v);
 #pragma unroll
     for (int c = 0; c < NC / 2; c += 8) emit8(p, (size_t)m, n0 / 2 + c, p.N / 2, v + c, make_uint4(0, 0, 0, 0));
     return;
@@ -197,6 +268,7 @@ __device__ __forceinline__ void finish_row(const RowsParams& p, float (&v)[NC], 
     }
   }
   if (m >= p.M) return;
+  if constexpr (!VEC) return emit_ragged<NC>(p, (size_t)m, n0, p.N, v);
 #pragma unroll
   for (int c = 0; c < NC; c += 32) {                         // four residual vectors in flight at a time
     uint4 r[4];
@@ -226,7 +298,7 @@ struct PairCfg {
   static_assert(kStageBytes % 1024 == 0 && kNeedCols <= 512, "");
 };
 
-template <int KIND, int BN>
+template <int KIND, int BN, bool VEC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSB, const RowsParams p) {
@@ -384,7 +456,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mb::tc_fence_before();
       __syncwarp();
       if (lane == 0) mb::mbar_arrive_cluster(empty0 + buf * 8);
-      finish_row<KIND, NC>(p, v, m, nt * BN + half * NC, as);
+      finish_row<KIND, NC, VEC>(p, v, m, nt * BN + half * NC, as);
     }
     mb::tc_fence_before();
   }
@@ -407,7 +479,7 @@ struct BlkCfg {
   static constexpr int kSmem = kStages * kStageBytes + 1024;
 };
 
-template <int BN>
+template <int BN, bool VEC>
 __global__ void __launch_bounds__(kBlkThreads, 1)
 gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const RowsParams p) {
   constexpr int kBlkStages = BlkCfg<BN>::kStages, kBlkStageBytes = BlkCfg<BN>::kStageBytes, kBlkAccs = BlkCfg<BN>::kAccs;
@@ -555,13 +627,17 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
       if (ok && live) {
         const size_t m = (size_t)t.row0 + r;
+        if constexpr (VEC) {
 #pragma unroll
-        for (int c = 0; c < NC; c += 32) {
-          uint4 res[4];
+          for (int c = 0; c < NC; c += 32) {
+            uint4 res[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) res[k] = residual8(p, m, n0 + c + 8 * k, p.N);
+            for (int k = 0; k < 4; ++k) res[k] = residual8(p, m, n0 + c + 8 * k, p.N);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) emit8(p, m, n0 + c + 8 * k, p.N, acc + c + 8 * k, res[k]);
+            for (int k = 0; k < 4; ++k) emit8(p, m, n0 + c + 8 * k, p.N, acc + c + 8 * k, res[k]);
+          }
+        } else {
+          emit_ragged<NC>(p, m, n0, p.N, acc);
         }
       }
     }
@@ -574,10 +650,10 @@ gemm_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
 }
 
-template <int KIND, int BN>
+template <int KIND, int BN, bool VEC>
 int launch_pair(const CUtensorMap* tm, const RowsParams& p, int pairs, cudaStream_t stream) {
   using C = PairCfg<KIND, BN>;
-  auto kern = gemm_pair_kernel<KIND, BN>;
+  auto kern = gemm_pair_kernel<KIND, BN, VEC>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
@@ -587,9 +663,15 @@ int launch_pair(const CUtensorMap* tm, const RowsParams& p, int pairs, cudaStrea
   return (int)mb::launch_kernel_cluster(kern, dim3(2 * pairs), dim3(kThreads), C::kSmemBytes, stream, 1, tm[0], tm[1], tm[2], tm[3], p);
 }
 
-template <int BN>
+template <int KIND>
+int launch_pair(const CUtensorMap* tm, const RowsParams& p, bool wide, int pairs, cudaStream_t stream) {
+  if (p.vec || p.outq) return wide ? launch_pair<KIND, 256, true>(tm, p, pairs, stream) : launch_pair<KIND, 128, true>(tm, p, pairs, stream);
+  return wide ? launch_pair<KIND, 256, false>(tm, p, pairs, stream) : launch_pair<KIND, 128, false>(tm, p, pairs, stream);
+}
+
+template <int BN, bool VEC>
 int launch_block(const CUtensorMap* tm, const RowsParams& p, int grid, cudaStream_t stream) {
-  auto kern = gemm_block_kernel<BN>;
+  auto kern = gemm_block_kernel<BN, VEC>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BlkCfg<BN>::kSmem);
@@ -654,7 +736,8 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
     const long long items = (long long)p.m_tiles * p.n_tiles;
     if (items > 0x7fffffff) return MB_ERR_TOO_LARGE;
     const int grid = items < sms ? (int)items : sms;
-    return wide ? launch_block<256>(tm, p, grid, stream) : launch_block<128>(tm, p, grid, stream);
+    if (p.vec) return wide ? launch_block<256, true>(tm, p, grid, stream) : launch_block<128, true>(tm, p, grid, stream);
+    return wide ? launch_block<256, false>(tm, p, grid, stream) : launch_block<128, false>(tm, p, grid, stream);
   }
 
   if (a->outq) {
@@ -688,8 +771,8 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
     if ((rc = mbh::encode_2d(&tm[3], dt, a->sfa, 256, (uint64_t)((a->N + 127) / 128) * p.sfb_rows, 256, 256, 8, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
   }
   switch (kind) {
-    case KIND_BF16: return wide ? launch_pair<KIND_BF16, 256>(tm, p, pairs, stream) : launch_pair<KIND_BF16, 128>(tm, p, pairs, stream);
-    case KIND_FP8: return wide ? launch_pair<KIND_FP8, 256>(tm, p, pairs, stream) : launch_pair<KIND_FP8, 128>(tm, p, pairs, stream);
-    default: return wide ? launch_pair<KIND_NVFP4, 256>(tm, p, pairs, stream) : launch_pair<KIND_NVFP4, 128>(tm, p, pairs, stream);
+    case KIND_BF16: return launch_pair<KIND_BF16>(tm, p, wide, pairs, stream);
+    case KIND_FP8: return launch_pair<KIND_FP8>(tm, p, wide, pairs, stream);
+    default: return launch_pair<KIND_NVFP4>(tm, p, wide, pairs, stream);
   }
 }

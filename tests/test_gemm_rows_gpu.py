@@ -52,6 +52,29 @@ def test_pair_kernel_ragged_features_and_depth(N, K):
     assert torch.equal(wide[:, :N], got.to(torch.bfloat16)) and bool((wide[:, N:] == 7).all())
 
 
+@pytest.mark.parametrize("fmt", ["bf16", "fp8_row", "nvfp4", "fp8_block"])
+@pytest.mark.parametrize("M,N", [(257, 257), (300, 1030), (389, 4099)])
+def test_rows_that_are_not_whole_vectors(fmt, M, N):
+    """Odd and even row lengths; a last row block of one row, of part of a warp, of whole warps: the same sums as a tile per CTA."""
+    x, w_cpu, act, w = _operands(fmt, M, N, 512, 11)
+    res = torch.randn(M, N, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    one = dict(one_tile_per_cta=True, force_splits=1)
+    got = ops.linear(act, w, out_f32=True)
+    assert torch.equal(got, ops.linear(act, w, out_f32=True, **one))
+    want = ops.linear(act, w, residual=res, **one)
+    assert torch.equal(ops.linear(act, w, residual=res), want)
+    wide = torch.full((M, N + 3), 7.0, dtype=torch.bfloat16, device=DEV)
+    wide[:, :N] = res
+    ops.linear(act, w, residual=wide[:, :N], out=wide[:, :N])                   # in place, rows of a wider matrix
+    assert torch.equal(wide[:, :N], want) and bool((wide[:, N:] == 7).all())
+    if N % 2 == 0 and fmt != "fp8_block":
+        glu, other = ops.linear(act, w, swiglu=True), ops.linear(act, w, swiglu=True, **one)
+        assert glu.shape[1] == N // 2 and (glu.float() - other.float()).abs().max() <= 2.0 ** -7 * other.float().abs().max()
+    ops.check_status(DEV)
+    exact = _oracle(x, w_cpu, fmt)
+    assert (got.cpu().double() - exact).norm() <= 1e-5 * exact.norm()
+
+
 @pytest.mark.parametrize("M", [129, 300])
 def test_pair_kernel_epilogues(M):
     N, K = 9600, 256
