@@ -683,17 +683,38 @@ int launch_block(const CUtensorMap* tm, const RowsParams& p, int grid, cudaStrea
 
 }  // namespace
 
+// Few tiles of long rows: the kernels here walk the k blocks of a tile in series, a quarter of a microsecond each (fp8 blocks 0.58)
+// however few tiles there are; one tile per CTA (gemm_tcgen05.cu) can split them, at a fixed price (the exchange of a tile of 128
+// features by 256 tokens, NVFP4 128, fp8 blocks 64) that weighs more the fewer splits there are. Here / split, us (tiles x splits;
+// depth in k blocks):
+//   bf16       32: 12 x 8 18.1 / 18.5; 40: 12 x 8 20.3 / 18.7, 22 x 6 20.5 / 22.1; 64: 24 x 5 26.5 / 24.1, 36 x 3 26.9 / 26.9;
+//              80: 12 x 8 28.9 / 20.8, 32 x 4 31.2 / 28.8, 48 x 2 30.9 / 34.9; 112: 44 x 3 40.7 / 37.4
+//   fp8        32: 12 x 8 18.5 / 18.5, 16 x 6 18.6 / 20.5; 56: 12 x 8 24.7 / 18.7, 24 x 5 25.0 / 22.7, 48 x 2 26.2 / 28.9
+//   NVFP4      12: 24 x 3 14.5 / 14.9; 16: 24 x 4 16.5 / 14.6; 20: 40 x 3 16.7 / 16.6; 28: 60 x 2 20.2 / 18.6; 68: 12 x 8 28.7 / 16.5
+//   fp8 blocks 16: 32 x 4 16.4 / 14.8, 40 x 3 16.4 / 16.4, 48 x 2 16.4 / 18.5; 32: 8 x 8 26 / 16; 56: 10 x 8 39 / 17, 48 x 2 35 / 33
+static bool splits_pay(const MbGemmArgs* a) {
+  if (!a->ws) return false;
+  const int kelems = a->kind == KIND_BF16 ? 64 : a->kind == KIND_NVFP4 ? 256 : 128;
+  const int tn = a->kind == KIND_NVFP4 ? 128 : a->kind == KIND_FP8_BLOCK ? 64 : 256;
+  const int num_kb = (a->K + kelems - 1) / kelems, sms = a->sm_count > 0 ? a->sm_count : 148;
+  const long long tiles = (long long)((a->N + 127) / 128) * ((a->M + tn - 1) / tn);
+  if (tiles >= sms) return false;
+  const int splits = mb_gemm_auto_splits((int)tiles, num_kb, sms, true), saved = num_kb - (num_kb + splits - 1) / splits;
+  return a->kind == KIND_NVFP4 ? saved > 11 : a->kind == KIND_FP8_BLOCK ? splits >= 3 && saved > 10 : saved > 64 - 4 * splits;
+}
+
 bool mb_gemm_rows_serves(const MbGemmArgs* a) {
   if (a->force_splits > 0 || a->no_cluster || (a->flags & (MB_GEMM_ONE_TILE_PER_CTA | MB_GEMM_DECODE_TILE_ORDER))) return false;
   if (a->kind == KIND_FP8_BLOCK) {
     if (a->epilogue != mb::EPI_PLAIN || a->outq) return false;
-    return a->tile_expert ? true : a->force_tn == 0 && a->M > 64;
+    return a->tile_expert ? true : a->force_tn == 0 && a->M > 64 && !splits_pay(a);
   }
   // bf16 of one token tile is bound by the weights' stream, which 74 pairs pull slower than 148 CTAs (or splits of K) do: two dense
   // layers of 5120 at 144 / 200 / 256 tokens 537 / 546 / 552 us here, 505 / 515 / 529 a tile per CTA; at 300 tokens 713 against 869.
   // NVFP4 weights are a quarter of the bytes: 159 / 161 / 165 here against 178 / 187 / 187.
   if (a->kind == KIND_BF16 && a->M <= 256 && !a->outq) return false;
-  return !a->tile_expert && a->force_tn == 0 && a->M > 128 && (a->flags & MB_GEMM_PERSISTENT_PREFILL);
+  if (a->tile_expert || a->force_tn != 0 || a->M <= 128 || !(a->flags & MB_GEMM_PERSISTENT_PREFILL)) return false;
+  return a->outq || !splits_pay(a);
 }
 
 int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
