@@ -70,6 +70,13 @@ __device__ __forceinline__ void store_bf16x8(__nv_bfloat16* dst, const float* y)
   *reinterpret_cast<uint4*>(dst) = pk;
 }
 
+// a whole 32-byte sector
+__device__ __forceinline__ void store_f32x8(float* dst, const float* y) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "f"(y[0]), "f"(y[1]), "f"(y[2]), "f"(y[3]), "f"(y[4]), "f"(y[5]),
+               "f"(y[6]), "f"(y[7])
+               : "memory");
+}
+
 // 8 results of one token at feature n (of n_limit): residual and store
 __device__ __forceinline__ void emit8(const RowsParams& p, size_t m, int n, int n_limit, float* y, const uint4& res) {
   const size_t o = m * (size_t)p.ldo + n;
@@ -83,9 +90,7 @@ __device__ __forceinline__ void emit8(const RowsParams& p, size_t m, int n, int 
       }
     }
     if (p.out_f32) {
-      float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + o);
-      dst[0] = make_float4(y[0], y[1], y[2], y[3]);
-      dst[1] = make_float4(y[4], y[5], y[6], y[7]);
+      store_f32x8(reinterpret_cast<float*>(p.out) + o, y);
     } else {
       store_bf16x8(reinterpret_cast<__nv_bfloat16*>(p.out) + o, y);
     }
@@ -109,7 +114,7 @@ __device__ __forceinline__ void emit8(const RowsParams& p, size_t m, int n, int 
 template <int NC, bool F32>
 __device__ __forceinline__ void emit_shifted(const RowsParams& p, size_t m, int n0, int left, float* v) {
   using T = std::conditional_t<F32, float, __nv_bfloat16>;
-  constexpr int kPer = F32 ? 1 : 2, kWords = NC / kPer, kVec = 4 * kPer;      // elements of a word, words, elements of a vector
+  constexpr int kPer = F32 ? 1 : 2, kWords = NC / kPer, kVec = 8, kVecWords = kVec / kPer;     // elements of a word, of a vector (16 or 32 bytes)
   left = min(left, NC);
   const size_t o = m * (size_t)p.ldo + n0;
   if (p.residual) {
@@ -144,22 +149,30 @@ __device__ __forceinline__ void emit_shifted(const RowsParams& p, size_t m, int 
   for (int i = 0; i < kWords; ++i) w[i] = up & 1 ? (i + 1 < kWords ? w[i + 1] : 0) : w[i];
 #pragma unroll
   for (int i = 0; i < kWords; ++i) w[i] = up & 2 ? (i + 2 < kWords ? w[i + 2] : 0) : w[i];
+  if constexpr (F32) {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = up & 4 ? (i + 4 < kWords ? w[i + 4] : 0) : w[i];
+  }
   dst += lead;
+  auto vector = [&](int i) {                                 // the words from i on
+    if constexpr (F32) store_f32x8(dst, reinterpret_cast<const float*>(w + i));
+    else *reinterpret_cast<uint4*>(dst) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
+  };
   if (left == NC) {
 #pragma unroll
-    for (int k = 0; k < NC / kVec - 1; ++k, dst += kVec) *reinterpret_cast<uint4*>(dst) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+    for (int k = 0; k < NC / kVec - 1; ++k, dst += kVec) vector(k * kVecWords);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = w[kWords - 4 + i];
+    for (int i = 0; i < kVecWords; ++i) w[i] = w[kWords - kVecWords + i];
     left = kVec;
   }
 #pragma unroll 1
   for (left -= lead; left > 0; left -= kVec, dst += kVec) {
-    if (left >= kVec) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (left >= kVec) vector(0);
 #pragma unroll
     for (int i = 0; i < kVec - 1; ++i)
       if (left < kVec && i < left) single(i);
 #pragma unroll
-    for (int i = 0; i < kWords - 4; ++i) w[i] = w[i + 4];
+    for (int i = 0; i < kWords - kVecWords; ++i) w[i] = w[i + kVecWords];
   }
 }
 
@@ -733,7 +746,7 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
   p.w_scale = a->w_scale; p.a_scale = a->a_scale; p.a_ld = a->a_ld; p.alpha = a->alpha;
   p.a_static = a->a_static != 0.f ? a->a_static : 1.f;
   p.epilogue = a->epilogue; p.out_f32 = a->out_f32;
-  p.vec = a->ldo % 8 == 0 && ((reinterpret_cast<uintptr_t>(a->out) | reinterpret_cast<uintptr_t>(a->residual)) & 15) == 0;
+  p.vec = a->ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(a->out) & (a->out_f32 ? 31 : 15)) == 0 && (reinterpret_cast<uintptr_t>(a->residual) & 15) == 0;
   p.epi_a = a->epi_a; p.epi_b = a->epi_b; p.epi_n = a->epi_n; p.epi_bias = a->epi_bias;
   p.status = a->status;
   CUtensorMap tm[4];
