@@ -586,6 +586,33 @@ int parts_of(int max_ctx, int part) {
 // sixteen sequences of 200 to 2000 28 / 22 / 32.
 int part_tokens_of(const AttnDecodeArgs& a) { return ((a.part_tokens > 0 ? a.part_tokens : a.Hkv >= 8 ? 1024 : 512) + 63) & ~63; }
 
+struct Layout {
+  int ahead, over;
+  uint32_t merge_off, tail_off, len_off;
+  size_t smem;
+  int per_sm;                                                // CTAs that an SM holds
+};
+// Shared memory of a launch. What lies beside the ring grows with the rows (the merge buffer, the queries) and with the batch (the
+// list of units), so it may leave room for fewer CTAs than the registers do: the grid has as many as are resident, since the
+// units are shared out over it evenly and CTAs beyond would start on theirs when the others are done (e4m3, 40 / 8 heads, 512 sequences
+// of 100 to 1000 tokens 229 -> 172 us, the split-KV kernel 207; bf16, 16 / 2 heads, 1024 of 60 to 700 136 -> 112; 32 rows 225 -> 219).
+template <int D, bool FP8, int MT>
+Layout layout(int rows, int num_seqs) {
+  using C = DecodeCfg<D, FP8, MT>;
+  Layout l;
+  // the merge buffer lies over the ring's last slots where it fits in front of the next unit's first ones
+  const int merge = 4 * rows * D * 4, behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
+  l.over = behind < C::kSlots;
+  l.ahead = l.over ? C::kSlots - behind : C::kSlots;
+  l.merge_off = l.over ? (uint32_t)(l.ahead * 4 * C::kSlot) : (uint32_t)C::kRing;
+  l.tail_off = l.over ? (uint32_t)C::kRing : (uint32_t)(C::kRing + merge);
+  l.len_off = (l.tail_off + (uint32_t)(num_seqs + 2) * 4 + 4 * MT * 16 * 8 + 8 + 15) & ~15u;
+  l.smem = 1024 + (size_t)l.len_off + (size_t)num_seqs * 16 + (size_t)rows * C::kQPitch;
+  const int fit = (int)(228 * 1024 / (l.smem + 1024 + 256));   // a block's own kilobyte, its static arrays
+  l.per_sm = fit < 1 ? 1 : fit < C::kCtas ? fit : C::kCtas;
+  return l;
+}
+
 template <int D, bool FP8, int MT>
 int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
   using C = DecodeCfg<D, FP8, MT>;
@@ -596,30 +623,35 @@ int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
                                   C::kRowB, (uint64_t)a.Hkv * C::kRowB, 128, 1, kSlice);
     if (rc) return rc;
   }
-  // the merge buffer lies over the ring's last slots where it fits in front of the next unit's first ones
-  const int rows = a.max_q_len * (a.Hq / a.Hkv), merge = 4 * rows * D * 4;
-  const int behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
-  const bool over = behind < C::kSlots;
-  p.ahead = over ? C::kSlots - behind : C::kSlots;
-  p.over = over;
-  p.merge_off = over ? (uint32_t)(p.ahead * 4 * C::kSlot) : (uint32_t)C::kRing;
-  p.tail_off = over ? (uint32_t)C::kRing : (uint32_t)(C::kRing + merge);
-  p.len_off = (p.tail_off + (uint32_t)(a.num_seqs + 2) * 4 + 4 * MT * 16 * 8 + 8 + 15) & ~15u;
-  const size_t smem = 1024 + (size_t)p.len_off + (size_t)a.num_seqs * 16 + (size_t)rows * C::kQPitch;
+  const Layout l = layout<D, FP8, MT>(a.max_q_len * (a.Hq / a.Hkv), a.num_seqs);
+  p.ahead = l.ahead;
+  p.over = l.over;
+  p.merge_off = l.merge_off;
+  p.tail_off = l.tail_off;
+  p.len_off = l.len_off;
   static size_t configured = 0;
-  if (smem > 220 * 1024) return MB_ERR_TOO_LARGE;
-  if (smem > configured) {
+  if (l.smem > 220 * 1024) return MB_ERR_TOO_LARGE;
+  if (l.smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     if (e != cudaSuccess) return (int)e;
     configured = 220 * 1024;
   }
   const int sms = a.sm_count > 0 ? a.sm_count : 148;
   const long long most = (long long)a.num_seqs * a.Hkv * p.parts;
-  const int grid = most < (long long)sms * C::kCtas ? (int)most : sms * C::kCtas;
-  return (int)mb::launch_kernel(kern, dim3(grid), dim3(128), smem, stream, tm[0], tm[1], p);
+  const int grid = most < (long long)sms * l.per_sm ? (int)most : sms * l.per_sm;
+  return (int)mb::launch_kernel(kern, dim3(grid), dim3(128), l.smem, stream, tm[0], tm[1], p);
 }
 
 }  // namespace
+
+extern "C" int mb_attn_decode_per_sm(int D, int fp8, int rows, int num_seqs, size_t* smem) {
+  const bool two = rows > 16;
+  const Layout l = D == 256 ? (fp8 ? layout<256, true, 1>(rows, num_seqs) : layout<256, false, 1>(rows, num_seqs))
+                   : fp8    ? (two ? layout<128, true, 2>(rows, num_seqs) : layout<128, true, 1>(rows, num_seqs))
+                            : (two ? layout<128, false, 2>(rows, num_seqs) : layout<128, false, 1>(rows, num_seqs));
+  if (smem) *smem = l.smem;
+  return l.per_sm;
+}
 
 bool mb_attn_decode_serves(const AttnDecodeArgs& a) {
   const int G = a.Hq / a.Hkv, rows = G * a.max_q_len;

@@ -33,6 +33,8 @@ struct AttnDecodeArgs {
   uint32_t* status;
 };
 
+// CTAs of a launch that an SM holds, and the shared memory of each (D 128 or 256; rows = tokens x heads of a group)
+extern "C" int mb_attn_decode_per_sm(int D, int fp8, int rows, int num_seqs, size_t* smem);
 bool mb_attn_decode_serves(const AttnDecodeArgs& a);
 size_t mb_attn_decode_ws(const AttnDecodeArgs& a);
 int mb_attn_decode(const AttnDecodeArgs& a, cudaStream_t stream);

@@ -35,7 +35,7 @@ def _case(fp8, D, Hq, Hkv, q_lens, ctx_lens, bs, seed=0):
     (128, 40, 8, [1], [1], 16), (128, 5, 1, [1, 1, 1, 1, 1], [15, 16, 17, 64, 65], 16), (128, 40, 8, [1, 1, 1], [255, 256, 257], 16),
     (128, 1, 1, [1, 1], [8191, 9000], 16), (128, 16, 1, [1], [700], 64), (128, 5, 1, [4, 1, 3], [4, 333, 600], 16),
     (128, 4, 1, [8, 2], [100, 513], 48), (128, 40, 8, [1] * 130, [7 * i % 900 + 1 for i in range(130)], 16),
-    (256, 16, 2, [1, 1], [90, 1025], 16), (256, 8, 1, [1, 2], [33, 300], 32)])
+    (256, 16, 2, [1, 1], [90, 1025], 16), (256, 8, 1, [1, 2], [33, 300], 32), (128, 32, 8, [8] * 41, [9 + 29 * i % 700 for i in range(41)], 16)])
 def test_matches_attention_in_64_bits(fp8, D, Hq, Hkv, q_lens, ctx_lens, bs):
     args, kw, want = _case(fp8, D, Hq, Hkv, q_lens, ctx_lens, bs)
     for part in (0, 64, 1024):

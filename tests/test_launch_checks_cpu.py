@@ -43,3 +43,19 @@ def test_splits_of_k_keep_their_clusters_resident(lib):
             want = max((n for n in held if tiles <= held[n] and n * tiles <= 148 and (n == 1 or 4 * n <= num_kb)), default=1)
             assert s == want, (tiles, num_kb)
             assert lib.mb_gemm_auto_splits(tiles, num_kb, 148, False) == max(1, min(148 // tiles, num_kb // 4))
+
+
+@pytest.mark.parametrize("D,most", [(128, 3), (256, 1)])
+def test_decode_attention_launches_only_resident_ctas(lib, D, most):
+    """Shared memory beside the ring grows with rows and batch: 228 KB an SM, a kilobyte of it a block's own."""
+    lib.mb_attn_decode_per_sm.argtypes, lib.mb_attn_decode_per_sm.restype = [C.c_int] * 4 + [C.POINTER(C.c_size_t)], C.c_int
+    seen = set()
+    for fp8 in (0, 1):
+        for rows in range(1, 33 if D == 128 else 17):
+            for seqs in (1, 64, 128, 512, 1024):
+                smem = C.c_size_t()
+                n = lib.mb_attn_decode_per_sm(D, fp8, rows, seqs, C.byref(smem))
+                assert n * (smem.value + 1024 + 256) <= 228 * 1024 and smem.value <= 220 * 1024, (fp8, rows, seqs)
+                assert n == (2 if rows > 16 else most) or (n + 1) * (smem.value + 1024) > 227 * 1024, (fp8, rows, seqs)
+                seen.add(n)
+    assert seen == ({1, 2, 3} if D == 128 else {1})
