@@ -7,11 +7,16 @@
 //   warps 0-3, 4-7   softmax of row tile 0 / 1, thread = row: S from TMEM, P back to TMEM (over S), the output row at the end
 //   warps 8-11       K and V tiles of 128 cached tokens into two stages of shared memory, 128-byte swizzle, a row's 16-byte
 //                    pieces on neighbouring threads; an e4m3 cache becomes f16 on the way (exact, one conversion per two
-//                    values; Q and P are f16 then, as in the split-KV kernel), a bf16 cache is copied asynchronously
+//                    values; Q and P are f16 then), a bf16 cache is copied asynchronously
 //   warp 12          issues the products: S0 S1 | PV0 S0' | PV1 S1' | ... so that one tile's softmax runs under the other
 //                    tile's products. P is the A operand in TMEM, V is read as stored (MN-major).
 // A commit covers everything issued before it, so S(j) seen means P V(j - 1) done: the output may be rescaled (only when a
 // row's maximum has moved by more than 2^8) without a wait of its own.
+//
+// f16 has less range than the bf16 that queries come in and the exponentials have, so with an e4m3 cache a row's queries are scaled
+// by the power of two that takes their largest to [2^14, 2^15) (elements down to 2^-31 of it keep their 8 bits; the scores' factor
+// takes the power back), and the weights are held 2^7 larger than the running maximum says: up to 2^15, and the smallest that is not
+// zero is 2^-32 of it.
 //
 // Bounds: per row tile and 128 tokens, 16384 exponentials are 1024 cycles of the special function units and the two products 1024
 // of the tensor cores. Measured against attention_tc.cu (40 / 8 heads): 8192 tokens, e4m3 1720 -> 695 us (0.99 PFLOP/s); 64
@@ -26,6 +31,7 @@ constexpr int kRows = 256, kT = 128, kD = 128;
 constexpr int kThreads = 512;
 constexpr int kTileB = kT * kD * 2;                       // a staged K or V tile
 constexpr int kSmem = 2 * 128 * kD * 2 + 4 * kTileB + 1024;
+constexpr float kLift = 7.f;                              // log2 of what f16 weights are held larger by
 
 __device__ __forceinline__ uint32_t sw_off(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 __device__ __forceinline__ float ex2(float x) {
@@ -93,6 +99,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
   uint8_t* sV = sK + 2 * kTileB;
   __shared__ __align__(8) uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full[2];
   __shared__ uint32_t s_tmem;
+  __shared__ float s_qscale[kRows];                       // what a row's scores are too large by (e4m3 cache)
   const int kvh = blockIdx.x, seq = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   mb::pdl_wait();
   const int qlen = p.q_len[seq], ctx = p.ctx_len[seq], qs = p.q_start[seq];
@@ -145,14 +152,25 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
         const int qr = (tid >> 4) + 16 * i, c = tid & 15;
         if (row0 + qr >= nrows) v[i] = make_uint4(0, 0, 0, 0);
         if constexpr (FP8) {
-          const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
+          // bf16 bits without the sign order like the values: the row's largest over its sixteen threads
+          const uint32_t x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+          uint32_t top = 0;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) top = __vmaxu2(top, x[j] & 0x7fff7fffu);
+#pragma unroll
+          for (int d = 1; d < 16; d <<= 1) top = __vmaxu2(top, __shfl_xor_sync(0xffffffffu, top, d));
+          const int e = (int)(max(top & 0xffff, top >> 16) >> 7);              // its exponent, biased by 127
+          // 2^(141 - e), and its inverse; zeros and subnormal rows as if their exponent were 15, infinities and NaN as they are
+          const int up = e == 255 ? 0 : 141 - max(e, 15);
+          const float f = __int_as_float((127 + up) << 23);
           uint32_t h[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(b[j]);
-            h[j] = pack2<true>(f.x, f.y);
+            const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[j]));
+            h[j] = pack2<true>(y.x * f, y.y * f);
           }
           v[i] = make_uint4(h[0], h[1], h[2], h[3]);
+          if (c == 0) s_qscale[qr] = __int_as_float((127 - up) << 23);
         }
         *reinterpret_cast<uint4*>(sQ + (qr >> 7) * (128 * kD * 2) + (c >> 3) * (128 * 128) + sw_off(qr & 127, c & 7)) = v[i];
       }
@@ -160,9 +178,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
     fence_async_smem();
     __syncwarp();
     if (lane == 0) mb::mbar_arrive(&q_full);
+    if constexpr (FP8) asm volatile("bar.sync 1, 256;" ::: "memory");         // the rows' scales come from other softmax warps
     const bool live = row < nrows;
     const int tok = live ? row / G : 0, limit = live ? past + tok + 1 : 0;   // tokens [0, limit) are visible
-    const float sc = p.scale * (FP8 ? *p.k_scale : 1.f) * 1.44269504088896f;
+    const float sc = p.scale * (FP8 ? *p.k_scale : 1.f) * 1.44269504088896f * (FP8 ? s_qscale[w * 128 + r] : 1.f);
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     for (int j = 0; j < tiles; ++j) {
@@ -199,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
           mb::tmem_st16(tO + c, ov);
         }
       }
-      const float nm = m_run == -INFINITY ? 0.f : -m_run;
+      const float nm = m_run == -INFINITY ? 0.f : (FP8 ? kLift : 0.f) - m_run;
       const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(nm, nm);
       float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll

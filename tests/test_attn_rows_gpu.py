@@ -80,6 +80,53 @@ def test_scores_that_grow_along_the_context_rescale_the_output():
     assert (got[:, 0] - want).norm() <= 2.0 ** -8 * want.norm()
 
 
+@pytest.mark.parametrize("power", [20, 120, -30, -100])
+def test_queries_keep_the_range_of_bf16(power):
+    """An e4m3 cache is read as f16; queries far outside its range give the same bits with a softmax scale that takes the power back."""
+    args, kw, _ = _case(True, 10, 2, [129, 200], [129, 900], 16)
+    want = ops.paged_attention(*args, **kw)
+    got = ops.paged_attention(args[0] * 2.0 ** power, *args[1:], **dict(kw, scale=kw["scale"] * 2.0 ** -power))
+    ops.check_status(DEV)
+    assert got.isfinite().all() and torch.equal(got, want)
+
+
+def test_a_large_query_leaves_its_row_finite():
+    """One element of a row beyond f16, on a dim where the keys are zero: the row's other dims decide, as for its neighbours."""
+    args, kw, _ = _case(True, 2, 1, [140], [140], 16)
+    q, kc = args[0], args[1]
+    kc[..., 7] = 0
+    want = ops.paged_attention(*args, **kw).double()
+    q[3:90, :, 7] = 1e6
+    got = ops.paged_attention(*args, **kw).double()
+    ops.check_status(DEV)
+    # elements above 2^-31 of 1e6 keep their bits, smaller ones are off by 2^-20 at most: far less than the weights' and the result's rounding
+    assert (got - want).norm() <= 2.0 ** -8 * want.norm()
+
+
+def test_small_weights_beside_a_large_one_reach_the_output():
+    """The first token takes the row's maximum and has no value; some four thousand others of 2^-26 of its weight make the output."""
+    args, kw, _ = _case(True, 1, 1, [128], [4096], 16)
+    q, kc, vc, bt, qs, ql, ctx = args
+    g = torch.Generator(device=DEV).manual_seed(3)
+    k = torch.randn(4096, 128, generator=g, device=DEV) * 0.25
+    k[:, 0] = 0
+    k[0] = 0
+    k[0, 0] = 16.0
+    v = torch.rand(4096, 128, generator=g, device=DEV) + 0.5
+    v[0] = 0
+    for cache, x in ((kc, k), (vc, v)):
+        cache[bt[0, :256].long()] = x.to(torch.float8_e4m3fn).view(torch.uint8).view(256, 16, 1, 128)
+    q.copy_(torch.randn(128, 1, 128, generator=g, device=DEV) * 0.25)
+    q[:, :, 0] = 25.75 * math.log(2) * 128 ** 0.5 / (16 * 0.8)      # k_scale is 0.8
+    got = ops.paged_attention(*args, **kw)[:, 0].double()
+    ops.check_status(DEV)
+    kk, vv = (t[bt[0, :256].long()].view(torch.float8_e4m3fn).reshape(-1, 128).double() * s.double() for t, s in ((kc, kw["k_scale"]), (vc, kw["v_scale"])))
+    mask = torch.arange(4096, device=DEV)[None] <= torch.arange(3968, 4096, device=DEV)[:, None]
+    want = torch.softmax((q[:, 0].double() @ kk.t() * 128 ** -0.5).masked_fill(~mask, -math.inf), -1) @ vv
+    # the result's bf16 rounding; the weights' steps of 2^-31 of the maximum average out over the tokens
+    assert (got - want).norm() <= 2.0 ** -8 * want.norm()
+
+
 @pytest.mark.parametrize("Hq,Hkv,q_lens,ctx_lens", [(40, 8, [129], [129]), (4, 2, [140, 300], [500, 300])])
 def test_quantised_output(Hq, Hkv, q_lens, ctx_lens):
     args, kw, want = _case(True, Hq, Hkv, q_lens, ctx_lens, 16)
