@@ -54,7 +54,7 @@ def main():
                                 k_scale=sc, v_scale=sc)
     elif a.op == "prefill_attn":
         # one sequence of --ctx query tokens over its own keys (fresh prefill), 40 / 8 heads of 128, e4m3 cache:
-        # the tcgen05 / TMEM kernel (csrc/attention_tc.cu); --fmt bf16 for a bf16 cache
+        # the kernel of two row tiles (csrc/attention_rows.cu); --fmt bf16 for a bf16 cache
         Hq, Hkv, D, bs, q = 40, 8, 128, 16, a.ctx
         nblk = (q + bs - 1) // bs
         if a.fmt == "bf16":

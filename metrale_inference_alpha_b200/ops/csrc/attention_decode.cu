@@ -11,7 +11,9 @@
 //     The next unit's first slices are under way while this one's warps are merged.
 //   * partitions depend on the sequence's own length only (never on the batch): part_tokens each, but at most 32 of them;
 //     the last to arrive merges them in order.
-// The tensor-core fragments are as in attention.cu: mma.sync m16n8k16, an e4m3 row widened to f16 in registers.
+// The tensor-core fragments are as in attention.cu: mma.sync m16n8k16, an e4m3 row widened to f16 in registers. So with an e4m3 cache
+// queries and weights are f16 here, as there: a query element beyond 65504 makes its row NaN, weights below 2^-24 of the running
+// maximum vanish.
 // Measured against that kernel (us): e4m3, 40 / 8 heads of 128: one sequence of 700 tokens 22.5 -> 13.7, 128 of 129 to 1151 62 -> 50,
 // nine of 4000 to 16000 73 -> 54, eight verify steps of 4 rows 31 -> 22; bf16, 33 of 100 to 2047 57 -> 32; 16 / 2 heads of 256,
 // bf16, sixteen of 200 to 2000 119 -> 22.
@@ -580,10 +582,16 @@ int parts_of(int max_ctx, int part) {
   const int n = (max_ctx + part - 1) / part;
   return n < 1 ? 1 : n > kMaxParts ? kMaxParts : n;
 }
-// Long partitions pay a unit's fixed instructions less often, short ones fill the chip with fewer sequences; the size is a constant
-// of the model, so that a sequence's sums never depend on its batch. Measured with 256 / 512 / 1024 tokens, us: 8 kv heads, 128
-// sequences of 129 to 1151 tokens 74 / 60 / 50, nine of 4000 to 16000 89 / 73 / 54, one of 700 11.6 / 12.6 / 13.7; 2 kv heads of 256,
-// sixteen sequences of 200 to 2000 28 / 22 / 32.
+// Long partitions pay a unit's fixed instructions less often, short ones fill the chip with fewer sequences. The size depends on the
+// cache's heads alone, so that a sequence's sums never depend on its batch; a tensor-parallel shard, which has fewer heads, cuts the
+// same sequence finer. Where the line lies, 512 / 1024 tokens, us (e4m3, five heads of 128 a group):
+//                                    8 kv heads     4              2              1
+//   1 sequence of 4000               13.3 / 17.3    12.9 / 17.0    12.7 / 16.8    12.4 / 16.4
+//   16 of 200 to 2000                17.7 / 20.7    14.6 / 18.0    12.8 / 17.4    12.4 / 17.2
+//   33 of 100 to 2047                29.6 / 25.8    17.8 / 20.6    14.6 / 17.8    12.7 / 17.2
+//   128 of 129 to 1151               61.3 / 49.1    36.9 / 32.3    25.2 / 19.2    15.1 / 16.0
+//   9 of 4000 to 16000               72.1 / 50.5    38.0 / 28.8    23.1 / 22.7    19.2 / 19.3
+// Twelve such batches together, time at 1024 over time at 512: e4m3 0.91, 1.01, 1.12, 1.19; bf16 0.95, 1.04, -, 1.26; two heads of 256 1.04.
 int part_tokens_of(const AttnDecodeArgs& a) { return ((a.part_tokens > 0 ? a.part_tokens : a.Hkv >= 8 ? 1024 : 512) + 63) & ~63; }
 
 struct Layout {

@@ -8,7 +8,7 @@
 //   * every spin on an mbarrier or on a flag is bounded by a clock budget;
 //     on expiry the kernel writes a non-zero code into the caller-provided
 //     status word, drains, frees TMEM and returns (no trap, no endless loop);
-//   * all TMA loads are plain (no cluster multicast anywhere in the library).
+//   * no load is multicast to a cluster anywhere in the library (tc_commit2 multicasts an arrival, not data).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
