@@ -20,8 +20,10 @@
 //
 // Bounds: per row tile and 128 tokens, 16384 exponentials are 1024 cycles of the special function units and the two products 1024
 // of the tensor cores. Measured against attention_tc.cu (40 / 8 heads): 8192 tokens, e4m3 1720 -> 695 us (0.99 PFLOP/s); 64
-// prompts of 128 tokens, e4m3 167 -> 120; two bf16 portions of 1001 and 1531 tokens behind 2500 to 2900, 644 -> 226. With the
-// NVFP4 output written here the 36 us quantiser pass over 8192 x 5120 is gone.
+// prompts of 128 tokens, e4m3 167 -> 134; two bf16 portions of 1001 and 1531 tokens behind 2500 to 2900, 644 -> 226. With the
+// NVFP4 output written here the 36 us quantiser pass over 8192 x 5120 is gone. A CTA whose second row tile has no rows leaves it out:
+// 128 tokens of one head a group behind 1000 / 16000, 8 kv heads, bf16 29.3 -> 25.5 / 317 -> 299 us. One form stays slower than in
+// attention_tc.cu, whose CTAs share an SM: many prompts of 128 tokens with one head a group (16 prompts, 32 heads: 35 us there, 39 here).
 #include "common.cuh"
 #include "attention_rows.h"
 
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
   const int G = p.Hq / p.Hkv, nrows = qlen * G;
   const int row0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRows;   // the longest rows first
   if (row0 >= nrows) return;
+  const bool two = nrows - row0 > 128;                    // the second row tile has rows
   const int past = ctx - qlen;
   const int last_limit = past + (min(nrows, row0 + kRows) - 1) / G + 1;
   const int tiles = (last_limit + kT - 1) / kT;
@@ -184,7 +187,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
     const float sc = p.scale * (FP8 ? *p.k_scale : 1.f) * 1.44269504088896f * (FP8 ? s_qscale[w * 128 + r] : 1.f);
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < tiles; ++j) {
+    const int mine = w == 0 || two ? tiles : 0;
+    for (int j = 0; j < mine; ++j) {
       ok = mb::mbar_wait(&s_full[w], j & 1, p.status, MB_ST_TIMEOUT_MMA);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       mb::tc_fence_after();
@@ -240,6 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
       if (lane == 0) mb::mbar_arrive(&p_full[w]);
       l_run = l_run * alpha + ((sum[0].x + sum[0].y) + (sum[1].x + sum[1].y));
     }
+    ok = ok && mine > 0;
     if (ok) {
       ok = mb::mbar_wait(&o_full[w], 0, p.status, MB_ST_TIMEOUT_MMA);
       mb::tc_fence_after();
@@ -439,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
       ok = mb::mbar_wait(&q_full, 0, p.status, MB_ST_TIMEOUT_MMA) && mb::mbar_wait(&k_full[0], 0, p.status, MB_ST_TIMEOUT_MMA);
       if (ok) {
         scores(0, 0);
-        scores(1, 0);
+        if (two) scores(1, 0);
         mb::tc_commit(&k_empty[0]);
       }
       for (int j = 0; j < tiles && ok; ++j) {
@@ -455,14 +460,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_rows_kernel(const AttnRowsPa
         } else {
           mb::tc_commit(&o_full[0]);
         }
-        ok = mb::mbar_wait(&p_full[1], j & 1, p.status, MB_ST_TIMEOUT_MMA);
-        if (!ok) break;
-        values(1, j);
+        if (two) {
+          ok = mb::mbar_wait(&p_full[1], j & 1, p.status, MB_ST_TIMEOUT_MMA);
+          if (!ok) break;
+          values(1, j);
+        }
         mb::tc_commit(&v_empty[b]);
         if (more) {
-          scores(1, j + 1);
+          if (two) scores(1, j + 1);
           mb::tc_commit(&k_empty[b ^ 1]);
-        } else {
+        } else if (two) {
           mb::tc_commit(&o_full[1]);
         }
       }
