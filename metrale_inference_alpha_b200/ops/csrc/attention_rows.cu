@@ -20,7 +20,7 @@
 //
 // Bounds: per row tile and 128 tokens, 16384 exponentials are 1024 cycles of the special function units and the two products 1024
 // of the tensor cores. Measured against attention_tc.cu (40 / 8 heads): 8192 tokens, e4m3 1720 -> 695 us (0.99 PFLOP/s); 64
-// prompts of 128 tokens, e4m3 167 -> 134; two bf16 portions of 1001 and 1531 tokens behind 2500 to 2900, 644 -> 226. With the
+// prompts of 128 tokens, e4m3 167 -> 123; two bf16 portions of 1001 and 1531 tokens behind 2500 to 2900, 644 -> 226. With the
 // NVFP4 output written here the 36 us quantiser pass over 8192 x 5120 is gone. A CTA whose second row tile has no rows leaves it out:
 // 128 tokens of one head a group behind 1000 / 16000, 8 kv heads, bf16 29.3 -> 25.5 / 317 -> 299 us. One form stays slower than in
 // attention_tc.cu, whose CTAs share an SM: many prompts of 128 tokens with one head a group (16 prompts, 32 heads: 35 us there, 39 here).
