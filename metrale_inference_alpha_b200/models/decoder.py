@@ -23,7 +23,7 @@ from ..ops import ACT_FOR_WEIGHT, Act
 from ..ops import reference as ref
 from ..ops import mixers
 from ..weights.loader import AttnW, FfnW, LayerW, ModelW
-from .stream import CanonStream, HyperStream, ResidualStream
+from .stream import CanonStream, HyperStream, ResidualStream, TableRows
 
 
 class LayerCaches:
@@ -356,9 +356,19 @@ class Decoder:
             x = x * torch.tensor(self.cfg.embed_scale, dtype=torch.bfloat16).to(x.dtype)
         return x
 
+    def _embeds_in_norm(self, batch: ForwardBatch) -> bool:
+        """The first layer reads the embeddings through a plain RMSNorm, and nothing comes between them."""
+        c, lw = self.cfg, self.w.layers[0]
+        return (c.streams == 0 and c.canon_taps == 0 and not c.stream32 and c.hc_mult <= 1 and c.embed_scale == 1.0
+                and self.side_head is None and getattr(batch, "embed_override", None) is None
+                and lw.kind in ("attention", "gdn") and lw.out is None and torch.is_tensor(lw.ln1) and self.w.embed.dtype == torch.bfloat16)
+
     def backbone(self, batch: ForwardBatch, caches: LayerCaches) -> torch.Tensor:
         """Token ids -> final residual stream [T, hidden] (before the final norm)."""
-        x = self.embed(batch.token_ids, batch.positions)
+        if self._embeds_in_norm(batch):
+            x = TableRows(self.w.embed, batch.token_ids)
+        else:
+            x = self.embed(batch.token_ids, batch.positions)
         if getattr(batch, "embed_override", None) is not None:
             rows, emb = batch.embed_override
             x = x.index_copy(0, rows, emb.to(x.dtype))
@@ -423,7 +433,12 @@ class Decoder:
         [R, vocab / size] (greedy selection then merges per-rank maxima instead)."""
         x = self.backbone(batch, caches)
         if batch.logit_rows.numel() != x.shape[0]:
-            rows = x.take(batch.logit_rows) if hasattr(x, "take") and not torch.is_tensor(x) else self.full(x).index_select(0, batch.logit_rows)
+            if not torch.is_tensor(x) and hasattr(x, "take"):
+                rows = x.take(batch.logit_rows)
+            elif torch.is_tensor(self.w.final_norm) and self.full(x).dtype == torch.bfloat16:
+                rows = TableRows(self.full(x), batch.logit_rows)       # the final norm takes its rows itself
+            else:
+                rows = self.full(x).index_select(0, batch.logit_rows)
         else:
             rows = self.full(x) if isinstance(x, (CanonStream, HyperStream)) else x
         lg = self.logits(rows, out_f32=out_f32, gather=gather_logits)

@@ -163,3 +163,25 @@ class CanonStream:
     @property
     def value(self) -> torch.Tensor:
         return self.resolve()
+
+
+class TableRows:
+    """Rows of a table, by index, in front of the norm that reads them first: the embeddings of a step's tokens, the rows of
+    the final stream that logits are wanted of. The norm's kernel takes the rows from the table itself; ``value`` holds
+    them afterwards. Has the surface of ``parallel.fused.PendingSum``."""
+
+    def __init__(self, table: torch.Tensor, rows: torch.Tensor):
+        self.owner, self.table, self.rows = self, table, rows
+        self.value = None
+        self.shape, self.dtype, self.device, self.is_cuda = torch.Size((rows.numel(), table.shape[1])), table.dtype, table.device, table.is_cuda
+
+    def resolve(self) -> torch.Tensor:
+        if self.value is None:
+            self.value = ops.embed(self.rows, self.table) if self.rows.dtype == torch.int32 else self.table.index_select(0, self.rows)
+        return self.value
+
+    def reduce_norm(self, _, w: torch.Tensor, fmt: str, *, plus_one: bool = False, eps: float = 1e-6, also_bf16: bool = False, **unused):
+        if self.value is not None:
+            return ops.row_op(self.value, fmt, ops.IN_RMSNORM, w=w, plus_one=plus_one, eps=eps, also_bf16=also_bf16)[0]
+        act, self.value = ops.row_op(self.table, fmt, ops.IN_RMSNORM, w=w, plus_one=plus_one, eps=eps, also_bf16=also_bf16, gather=self.rows)
+        return act

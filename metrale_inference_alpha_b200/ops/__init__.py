@@ -263,18 +263,23 @@ def row_op(x: torch.Tensor, out_fmt: str = "bf16", mode: int = IN_COPY, *, K: Op
            residual=None, write_residual: bool = False, w=None, plus_one: bool = False,
            eps: float = 1e-6, gate=None, head_dim: int = 0, gate_head_stride: int = 0,
            gate_head_off: int = 0, group: int = 0, also_bf16: bool = False, static_scale: float = 0.0,
-           scale_pad: int = 0, row_index: Optional[torch.Tensor] = None):
+           scale_pad: int = 0, row_index: Optional[torch.Tensor] = None, gather: Optional[torch.Tensor] = None):
     """Fused producer: builds y = recipe(x) per row and encodes it as `out_fmt`. `static_scale`
     (nvfp4 only): calibrated global scale used instead of the row's amax / (6 * 448).
     `scale_pad` (fp8_g128): extra token columns in the per-group scale matrix (grouped expert GEMMs
     read whole row tiles past the last row). `row_index` (CUDA): int32 list of the rows to work on
     (negative entries are skipped); the other rows' outputs stay unwritten (an expert-sorted layout with
-    aligned tiles is mostly padding). Returns (Act,
+    aligned tiles is mostly padding). `gather` (IN_RMSNORM; int32 or int64 [M]): row m of the input is row
+    gather[m] of x, and the rows as gathered are the second result (an index that x has no row for gives zeros and
+    sets the status word). Returns (Act,
     residual_out or None). x is bf16 (or fp32 for IN_GATED_RMSNORM inputs)."""
-    M = x.shape[0]
+    M = x.shape[0] if gather is None else gather.numel()
     if K is None:
         K = x.shape[1] // 2 if mode == IN_SILU_MUL else x.shape[1]
     if not x.is_cuda:
+        if gather is not None:
+            rows = x[gather.long()]
+            return _row_op_ref(rows, out_fmt, mode, K, None, False, w, plus_one, eps, None, 0, 0, 0, 0, also_bf16, static_scale)[0], rows
         return _row_op_ref(x, out_fmt, mode, K, residual, write_residual, w, plus_one, eps, gate,
                            head_dim, gate_head_stride, gate_head_off, group, also_bf16, static_scale)
     L = _native.lib()
@@ -295,6 +300,11 @@ def row_op(x: torch.Tensor, out_fmt: str = "bf16", mode: int = IN_COPY, *, K: Op
     if write_residual:
         res_out = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
         a.residual_out = _ptr(res_out)
+    if gather is not None:
+        assert gather.dtype in (torch.int32, torch.int64) and gather.is_contiguous() and x.dtype == torch.bfloat16 and x.stride(1) == 1
+        res_out = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
+        a.gather, a.gather_wide, a.gather_rows = _ptr(gather), int(gather.dtype == torch.int64), x.shape[0]
+        a.gather_out, a.status = _ptr(res_out), _ptr(runtime(dev).status)
     a.w = _ptr(w)
     a.w_plus_one = int(plus_one)
     a.eps = eps

@@ -44,6 +44,7 @@ class RowArgs(C.Structure):
         ("out_bf16", c_void_p), ("out_bf16_ld", c_ll),
         ("scale", c_void_p), ("scale_ld", c_int), ("sf", c_void_p), ("sf_k64", c_int), ("static_gs", c_float),
         ("row_index", c_void_p),
+        ("gather", c_void_p), ("gather_wide", c_int), ("gather_rows", c_ll), ("gather_out", c_void_p), ("status", c_void_p),
     ]
 
 
