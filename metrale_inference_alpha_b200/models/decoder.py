@@ -206,11 +206,11 @@ class Decoder:
             # the attention kernel's final store quantises for o_proj with the calibrated scale
             oa = ops.paged_attention(q, kc, vc, batch.block_table, batch.q_start, batch.q_len, batch.ctx_len,
                                      max_q_len=batch.max_q_len, max_ctx=batch.max_ctx, scale=self.scale,
-                                     k_scale=ks, v_scale=vs, window=window, quant_out=static)
+                                     k_scale=ks, v_scale=vs, window=window, quant_out=static, early=kv_layer >= 0)
             return self.tp.linear_reduce(oa, w.o, residual=res, defer=defer)
         o = ops.paged_attention(q, kc, vc, batch.block_table, batch.q_start, batch.q_len, batch.ctx_len,
                                 max_q_len=batch.max_q_len, max_ctx=batch.max_ctx, scale=self.scale,
-                                k_scale=ks, v_scale=vs, window=window)
+                                k_scale=ks, v_scale=vs, window=window, early=kv_layer >= 0)
         o = o.view(o.shape[0], w.heads * D)
         if self.calib is not None:
             m = o.float().abs().max()

@@ -903,8 +903,10 @@ _ATTN_TC_VMN = int(os.environ.get("METRALE_ATTN_TC_VMN", "1"))
 
 def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_len, ctx_len, *,
                     max_q_len: int, max_ctx: int, scale: float, k_scale=None, v_scale=None,
-                    window: int = 0, force_mode: int = 0, part_tokens: int = 0, quant_out: float = 0.0):
-    """q [T, Hq, D] bf16 -> [T, Hq, D] bf16. Caches [num_blocks, block, Hkv, D] bf16 or e4m3 bytes.
+                    window: int = 0, force_mode: int = 0, part_tokens: int = 0, quant_out: float = 0.0, early: bool = False):
+    """q [T, Hq, D] bf16 -> [T, Hq, D] bf16. `early`: the launch in front is `qk_norm_rope_kvwrite` of the same rows, which wrote q and
+    these tokens' cache rows, and nothing before it in this call chain is still to be waited for: the decode kernel then starts on
+    the older tokens under it. Caches [num_blocks, block, Hkv, D] bf16 or e4m3 bytes.
     `quant_out` > 0: return the output as an NVFP4 `Act` [T, Hq * D] quantised with that calibrated
     global scale (inside the decode kernels and the plain head_dim 128 prefill kernel, else by a row kernel)."""
     T, Hq, D = q.shape
@@ -912,7 +914,8 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     if quant_out > 0.0:
         Hkv_ = k_cache.shape[2]
         rows = prefill and D == 128 and window == 0 and scale > 0 and _ATTN_TC_VMN != 0                    # csrc/attention_rows.cu
-        fused = q.is_cuda and (rows or (force_mode == 0 and (Hq // Hkv_) * max_q_len <= 16 and D % 128 == 0 and (Hq * D) % 64 == 0))
+        plain = D == 128 and window == 0 and k_cache.shape[1] % 16 == 0 and q_len.numel() <= 1024                  # csrc/attention_decode.cu
+        fused = q.is_cuda and (rows or (force_mode == 0 and (Hq // Hkv_) * max_q_len <= (32 if plain else 16) and D % 128 == 0 and (Hq * D) % 64 == 0))
         if not fused:
             o = paged_attention(q, k_cache, v_cache, block_table, q_start, q_len, ctx_len, max_q_len=max_q_len,
                                 max_ctx=max_ctx, scale=scale, k_scale=k_scale, v_scale=v_scale, window=window,
@@ -964,7 +967,7 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     a.scale, a.cache_fp8 = scale, int(k_cache.dtype == torch.uint8)
     a.k_scale, a.v_scale, a.out = _ptr(k_scale), _ptr(v_scale), _ptr(out if qact is None else qact.data)
     a.total_rows, a.part_tokens, a.part_fixed, a.sm_count = T, part_tokens, part_fixed, rt.sm_count
-    a.window, a.force_mode, a.status = window, force_mode, _ptr(rt.status)
+    a.window, a.force_mode, a.status, a.early = window, force_mode, _ptr(rt.status), int(early)
     rt.ensure_attn_ws(L.mb_attn_ws_need(C.byref(a)))
     a.ws, a.ws_bytes = _ptr(rt.attn_ws), rt.attn_ws.numel()
     if qact is not None:

@@ -1437,6 +1437,7 @@ struct MbAttnArgs {
   int turn_max;
   int part_fixed;          // partition size that the caller insists on for the plain decode kernel too (0 = its own)
   int sm_count;
+  int early;               // see AttnDecodeArgs
 };
 
 // the plain decode / verify case that attention_decode.cu may serve (force_mode 1 keeps it on the split-KV kernel here)
@@ -1456,7 +1457,7 @@ static bool decode_args(const MbAttnArgs* a, AttnDecodeArgs* d) {
   d->out_ld = a->out_ld > 0 ? a->out_ld : (long long)a->Hq * a->D;
   d->outq = reinterpret_cast<uint8_t*>(a->outq); d->ldq = a->ldq;
   d->outq_sf = reinterpret_cast<uint8_t*>(a->outq_sf); d->outq_sf_k64 = a->outq_sf_k64; d->outq_gs = a->outq_gs;
-  d->ws = a->ws; d->ws_bytes = a->ws_bytes; d->total_rows = a->total_rows; d->part_tokens = a->part_fixed; d->sm_count = a->sm_count;
+  d->ws = a->ws; d->ws_bytes = a->ws_bytes; d->total_rows = a->total_rows; d->part_tokens = a->part_fixed; d->sm_count = a->sm_count; d->early = a->early;
   d->status = a->status;
   return mb_attn_decode_serves(*d);
 }

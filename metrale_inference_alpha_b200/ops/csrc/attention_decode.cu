@@ -23,7 +23,7 @@
 
 namespace {
 
-constexpr int kMaxParts = 32, kMaxSeqs = 1024, kSlice = 16;
+constexpr int kMaxParts = 32, kMaxSeqs = 1024, kSlice = 16, kMaxSlots = 6;
 constexpr size_t kCntBytes = 64 * 1024;      // arrival counters at the head of the workspace, as in attention.cu
 
 struct DecodeParams {
@@ -50,7 +50,9 @@ struct DecodeParams {
   float2* part_ml;                           // [rows * Hq, parts]: log2-domain maximum, sum
   uint32_t* part_cnt;                        // [seqs * Hkv]
   int parts, part_tokens;
+  int slots;                                 // of every warp's ring
   int ahead;                                 // slots of the ring that the next unit may fill while warps are merged
+  int early;                                 // all but q and the cache's rows of this step's tokens stood before the kernel in front began
   uint32_t merge_off, tail_off, len_off;     // byte offsets of the merge buffer and of what lies behind both
   int over;                                  // the merge buffer lies over slots of the ring
   uint32_t* status;
@@ -107,8 +109,7 @@ struct DecodeCfg {
   static constexpr int kTok = kSub * kSlice;
   static constexpr int kHalf = kTok * kRowB;                 // K or V of one step
   static constexpr int kSlot = 2 * kHalf;
-  static constexpr int kSlots = 2;
-  static constexpr int kRing = 4 * kSlots * kSlot;           // slot s of warp w at (s * 4 + w) * kSlot
+  static constexpr int ring(int slots) { return 4 * slots * kSlot; }           // slot s of warp w at (s * 4 + w) * kSlot
   static constexpr int kCtas = MT > 1 ? (D == 256 ? 1 : 2) : D == 256 ? 1 : 3;
   static constexpr int kQPitch = 2 * D + 16;                 // bytes between query rows in shared memory
 };
@@ -117,10 +118,11 @@ template <int D, bool FP8, int MT>
 __global__ void __launch_bounds__(128, DecodeCfg<D, FP8, MT>::kCtas)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeParams p) {
   using C = DecodeCfg<D, FP8, MT>;
-  constexpr int kSlots = C::kSlots, kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok;
+  constexpr int kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t bars[4 * kSlots];
+  __shared__ __align__(8) uint64_t bars[4 * kMaxSlots];
+  const int slots = p.slots;
   __shared__ int s_last, s_wsum[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   float* s_o = reinterpret_cast<float*>(smem + p.merge_off);                  // [4 warps][rows][D]
@@ -129,13 +131,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   int4* s_len = reinterpret_cast<int4*>(smem + p.len_off);                    // [seqs]: q_len, ctx_len, q_start
   uint8_t* s_q = smem + p.len_off + p.num_seqs * 16;                          // the unit's query rows, as loaded
   if (tid == 0) {
-    for (int i = 0; i < 4 * kSlots; ++i) mb::mbar_init(&bars[i], 1);
+    for (int i = 0; i < 4 * slots; ++i) mb::mbar_init(&bars[i], 1);
     mb::mbar_fence_init();
     mb::tma_prefetch_desc(&tmK);
     mb::tma_prefetch_desc(&tmV);
   }
-  mb::pdl_wait();
-  mb::pdl_launch_dependents();
+  if (!p.early) mb::pdl_wait();
 
   // ---- the list of units: partitions of every sequence in front of it
   auto part_size = [&](int len) { return max(p.part_tokens, ((len + kMaxParts - 1) / kMaxParts + 63) & ~63); };
@@ -244,17 +245,25 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const float sc_log2 = p.scale * kmul * 1.44269504088896f;
   uint32_t phase = 0;                                        // bit s: parity of slot s's next completion
   Unit cur;
-  int u = blockIdx.x;
+  int u = blockIdx.x, begun = 0;
   if (u < units) {
     find(u, cur);
     blocks(cur, 0);
-    for (int i = 0; i < min(cur.slices, kSlots); ++i) issue(cur, i, i);
+    // slices of tokens that were cached before this step travel under the end of the kernel in front, which writes the step's own
+    const int old = max(0, cur.ctx - cur.qlen - cur.begin) / kTok;
+    if (p.early)
+      for (; begun < min(min(cur.slices, slots), (old - warp + 3) >> 2); ++begun) issue(cur, begun, begun);
+  }
+  if (p.early) mb::pdl_wait();
+  mb::pdl_launch_dependents();
+  if (u < units) {
+    for (; begun < min(cur.slices, slots); ++begun) issue(cur, begun, begun);
     fetch_q(cur);
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
   __syncthreads();
   bool ok = true;
-  int started = kSlots;                                      // slices of `cur` that are under way already, at most
+  int started = slots;                                      // slices of `cur` that are under way already, at most
   while (u < units) {
     const int R = p.G * cur.qlen;
     // ---- queries as A fragments: rows g and g + 8 of each 16-row tile
@@ -303,7 +312,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         for (int i = 0; i < 4; ++i) o[mt][n][i] = 0.f;
     }
 
-    for (int i = started; i < min(cur.slices, kSlots); ++i) issue(cur, i, i);
+    for (int i = started; i < min(cur.slices, slots); ++i) issue(cur, i, i);
     int slot = 0;
     for (int i = 0; i < cur.slices; ++i) {
       ok = ok && mb::mbar_wait(&bars[slot * 4 + warp], (phase >> slot) & 1, p.status, MB_ST_TIMEOUT_TMA);
@@ -429,12 +438,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         }
       }
       __syncwarp();                                          // every lane has read the slot
-      const int nx = i + kSlots;
+      const int nx = i + slots;
       if (nx < cur.slices) {
         if (nx * kSub % 32 == 0) blocks(cur, nx);
         issue(cur, nx, slot);
       }
-      slot = slot + 1 == kSlots ? 0 : slot + 1;
+      slot = slot + 1 == slots ? 0 : slot + 1;
     }
 
     // ---- the next unit's first slices travel while this one is merged (slots behind `ahead` hold the merge buffer)
@@ -595,7 +604,7 @@ int parts_of(int max_ctx, int part) {
 int part_tokens_of(const AttnDecodeArgs& a) { return ((a.part_tokens > 0 ? a.part_tokens : a.Hkv >= 8 ? 1024 : 512) + 63) & ~63; }
 
 struct Layout {
-  int ahead, over;
+  int slots, ahead, over;
   uint32_t merge_off, tail_off, len_off;
   size_t smem;
   int per_sm;                                                // CTAs that an SM holds
@@ -605,15 +614,16 @@ struct Layout {
 // units are shared out over it evenly and CTAs beyond would start on theirs when the others are done (e4m3, 40 / 8 heads, 512 sequences
 // of 100 to 1000 tokens 229 -> 172 us, the split-KV kernel 207; bf16, 16 / 2 heads, 1024 of 60 to 700 136 -> 112; 32 rows 225 -> 219).
 template <int D, bool FP8, int MT>
-Layout layout(int rows, int num_seqs) {
+Layout layout(int rows, int num_seqs, int slots = 2) {
   using C = DecodeCfg<D, FP8, MT>;
   Layout l;
+  l.slots = slots;
   // the merge buffer lies over the ring's last slots where it fits in front of the next unit's first ones
   const int merge = 4 * rows * D * 4, behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
-  l.over = behind < C::kSlots;
-  l.ahead = l.over ? C::kSlots - behind : C::kSlots;
-  l.merge_off = l.over ? (uint32_t)(l.ahead * 4 * C::kSlot) : (uint32_t)C::kRing;
-  l.tail_off = l.over ? (uint32_t)C::kRing : (uint32_t)(C::kRing + merge);
+  l.over = behind < slots;
+  l.ahead = l.over ? slots - behind : slots;
+  l.merge_off = l.over ? (uint32_t)(l.ahead * 4 * C::kSlot) : (uint32_t)C::ring(slots);
+  l.tail_off = l.over ? (uint32_t)C::ring(slots) : (uint32_t)(C::ring(slots) + merge);
   l.len_off = (l.tail_off + (uint32_t)(num_seqs + 2) * 4 + 4 * MT * 16 * 8 + 8 + 15) & ~15u;
   l.smem = 1024 + (size_t)l.len_off + (size_t)num_seqs * 16 + (size_t)rows * C::kQPitch;
   const int fit = (int)(228 * 1024 / (l.smem + 1024 + 256));   // a block's own kilobyte, its static arrays
@@ -631,7 +641,18 @@ int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
                                   C::kRowB, (uint64_t)a.Hkv * C::kRowB, 128, 1, kSlice);
     if (rc) return rc;
   }
-  const Layout l = layout<D, FP8, MT>(a.max_q_len * (a.Hq / a.Hkv), a.num_seqs);
+  const int rows = a.max_q_len * (a.Hq / a.Hkv), sms = a.sm_count > 0 ? a.sm_count : 148;
+  const long long most = (long long)a.num_seqs * a.Hkv * p.parts;
+  Layout l = layout<D, FP8, MT>(rows, a.num_seqs);
+  // few units: as deep a ring as leaves each of them a CTA of its own
+  for (int slots = kMaxSlots; slots > 2; --slots) {
+    const Layout deep = layout<D, FP8, MT>(rows, a.num_seqs, slots);
+    if (deep.smem <= 220 * 1024 && (long long)sms * deep.per_sm >= most) {
+      l = deep;
+      break;
+    }
+  }
+  p.slots = l.slots;
   p.ahead = l.ahead;
   p.over = l.over;
   p.merge_off = l.merge_off;
@@ -644,10 +665,9 @@ int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     configured = 220 * 1024;
   }
-  const int sms = a.sm_count > 0 ? a.sm_count : 148;
-  const long long most = (long long)a.num_seqs * a.Hkv * p.parts;
   const int grid = most < (long long)sms * l.per_sm ? (int)most : sms * l.per_sm;
-  return (int)mb::launch_kernel(kern, dim3(grid), dim3(128), l.smem, stream, tm[0], tm[1], p);
+  p.early = a.early && mb_pdl_enabled() == 2;
+  return (int)mb::launch_kernel_ex(kern, dim3(grid), dim3(128), l.smem, stream, 1, p.early || mb_pdl_enabled() == 1, tm[0], tm[1], p);
 }
 
 }  // namespace

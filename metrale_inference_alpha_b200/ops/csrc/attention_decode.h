@@ -30,6 +30,9 @@ struct AttnDecodeArgs {
   size_t ws_bytes;
   int total_rows, part_tokens;   // part_tokens 0 = default
   int sm_count;
+  // the kernel in front wrote q and the cache's rows of this step's tokens (the last q_len of every context) and nothing else that is
+  // read here, and launches its dependents early
+  int early;
   uint32_t* status;
 };
 
