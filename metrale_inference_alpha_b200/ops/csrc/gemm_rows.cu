@@ -774,6 +774,7 @@ int mb_gemm_rows(const MbGemmArgs* a, int tn, cudaStream_t stream) {
     p.n_per_expert = a->tile_expert ? a->n_per_expert : 0;
     const int box_rows = !a->tile_expert || a->force_tn == 128 ? 128 : tn;
     if (box_rows != 16 && box_rows != 32 && box_rows != 64 && box_rows != 128) return MB_ERR_UNSUPPORTED;
+    if (mb_gemm_few_serves(a, box_rows)) return mb_gemm_few(a, box_rows, stream);
     p.a_bytes = box_rows * 128;
     p.m_tiles = a->tile_expert ? a->max_tiles : (a->M + 127) / 128;
     // 256 features a tile read the token rows half as often (at 128 x 128 the operands of 2700 tokens' experts come from L2 at its
