@@ -29,3 +29,5 @@ struct AttnRowsParams {
 };
 
 int mb_attn_rows(const AttnRowsParams& p, int max_q_len, int num_seqs, bool fp8, cudaStream_t stream);
+// the same at head dim 256, bf16 cache and output (attention_rows256.cu)
+int mb_attn_rows256(const AttnRowsParams& p, int max_q_len, int num_seqs, cudaStream_t stream);

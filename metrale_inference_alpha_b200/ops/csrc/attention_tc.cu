@@ -470,10 +470,10 @@ extern "C" int mb_attn_prefill_tc(const MbAttnTcArgs* a, cudaStream_t stream) {
   if (p.gate.mode == mb::GATE_ELEMENT && (a->gate_ld % 8 || (reinterpret_cast<uintptr_t>(a->gate) & 15))) return MB_ERR_UNSUPPORTED;
   if (p.out_ld % 8 || (reinterpret_cast<uintptr_t>(a->out) & 15)) return MB_ERR_BAD_ARG;      // 16-byte stores
   if (a->split_p && a->cache_fp8) return MB_ERR_UNSUPPORTED;
-  if (a->D == 128 && a->v_mn && !a->split_p && !a->sink && a->window <= 0 && !a->gate && !(a->softcap > 0.f) && !a->turn_cos &&
-      p.out_scale == 1.f && a->scale > 0.f) {
-    // the plain case: 256 rows of a head group per CTA (attention_rows.cu), 1.7 - 3 x as fast; what has a sink, a cap, a window,
-    // a gate, turned values or weights in two terms stays here, and head dim 256, whose tiles do not fit twice
+  if ((a->D == 128 || (!a->cache_fp8 && !a->outq)) && a->v_mn && !a->split_p && !a->sink && a->window <= 0 && !a->gate && !(a->softcap > 0.f) &&
+      !a->turn_cos && p.out_scale == 1.f && a->scale > 0.f) {
+    // the plain case: rows of a head group per CTA (attention_rows.cu, attention_rows256.cu), 1.7 - 3 x as fast; what has a sink, a cap, a
+    // window, a gate, turned values or weights in two terms stays here, and head dim 256 with an e4m3 cache
     AttnRowsParams r{};
     r.q = p.q; r.k_cache = p.k_cache; r.v_cache = p.v_cache; r.block_table = p.block_table; r.max_blocks = p.max_blocks;
     r.q_start = p.q_start; r.q_len = p.q_len; r.ctx_len = p.ctx_len;
@@ -487,6 +487,7 @@ extern "C" int mb_attn_prefill_tc(const MbAttnTcArgs* a, cudaStream_t stream) {
       r.outq_sf = reinterpret_cast<uint8_t*>(a->outq_sf); r.outq_sf_k64 = a->outq_sf_k64;
       r.outq_gs = a->outq_gs;
     }
+    if (a->D == 256) return mb_attn_rows256(r, a->max_q_len, a->num_seqs, stream);
     return mb_attn_rows(r, a->max_q_len, a->num_seqs, a->cache_fp8 != 0, stream);
   }
   if (a->outq) return MB_ERR_UNSUPPORTED;
