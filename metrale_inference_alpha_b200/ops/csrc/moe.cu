@@ -22,8 +22,15 @@
 
 namespace {
 
-constexpr int kMaxPerLane = 16;  // 512 experts / 32 lanes
+// Floats as unsigned integers of the same order (NaN aside)
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
+}
 
+// kMaxPerLane: experts of a lane (512 experts: 16). One warp a token, so it is the length of a choice's chain that counts: one
+// maximum over the warp and one over the indices that have it, instead of five exchanges of pairs.
+template <int kMaxPerLane>
 __global__ void __launch_bounds__(128)
 route_kernel(const float* __restrict__ logits, long long ld, int T, int E, int K, int mode,
              const float* __restrict__ bias, int n_group, int topk_group, int renorm, float scaling,
@@ -135,12 +142,9 @@ route_kernel(const float* __restrict__ logits, long long ld, int T, int E, int K
       const int e = j * 32 + lane;
       if (j < per && e < E && (sel[j] > v || (sel[j] == v && e < idx))) { v = sel[j]; idx = e; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-      if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-    }
+    const uint32_t key = order_key(v + 0.f);                 // both zeros are one value
+    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+    idx = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)idx : 0x7fffffffu);
     // owner lane reports the weight and retires the expert
     float w = 0.f;
     if ((idx & 31) == lane) {
@@ -185,9 +189,18 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < num_local; e += nt) cnt[e] = 0;
   __syncthreads();
-  for (int i = tid; i < pairs; i += nt) {
-    const int e = ids[i] - expert_lo;
-    if (e >= 0 && e < num_local) atomicAdd(&cnt[e], 1);
+  // eight ids of a thread on their way together (one CTA: its time is the loads' latencies, 24 us at 24300 pairs one by one)
+  constexpr int kIds = 8;
+  int id[kIds];
+  auto fetch = [&](int i0) {
+#pragma unroll
+    for (int k = 0; k < kIds; ++k) id[k] = i0 + k * nt < pairs ? __ldg(ids + i0 + k * nt) - expert_lo : -1;
+  };
+  for (int i0 = tid; i0 < pairs; i0 += kIds * nt) {
+    fetch(i0);
+#pragma unroll
+    for (int k = 0; k < kIds; ++k)
+      if (id[k] >= 0 && id[k] < num_local) atomicAdd(&cnt[id[k]], 1);
   }
   __syncthreads();
   // offsets and the tile work-list: thread e owns expert e (num_local <= blockDim.x = 1024); an exclusive block
@@ -244,39 +257,57 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
   // the combine reads rows through pair_row in slot order.
   for (int e = tid; e < num_local; e += nt) cnt[e] = 0;         // reused as the running fill of each expert
   __syncthreads();
-  for (int i = tid; i < pairs; i += nt) {
-    const int e = ids[i] - expert_lo;
-    if (e >= 0 && e < num_local) {
-      const int k = atomicAdd(&cnt[e], 1);
-      const int pos = off[e] + (align > 1 ? (k / tile_rows) * align + k % tile_rows : k);
-      pair_row[i] = pos;
-      row_pair[pos] = i;
+  for (int i0 = tid; i0 < pairs; i0 += kIds * nt) {
+    if (pairs > kIds * nt) fetch(i0);                            // otherwise they are still there
+    int pos[kIds];
+#pragma unroll
+    for (int k = 0; k < kIds; ++k) {
+      pos[k] = -1;
+      if (id[k] >= 0 && id[k] < num_local) {
+        const int at = atomicAdd(&cnt[id[k]], 1);
+        pos[k] = off[id[k]] + (align > 1 ? (at / tile_rows) * align + at % tile_rows : at);
+      }
     }
-  }
-  for (int i = tid; i < pairs; i += nt) {
-    const int e = ids[i] - expert_lo;
-    if (e < 0 || e >= num_local) pair_row[i] = -1;
+#pragma unroll
+    for (int k = 0; k < kIds; ++k) {
+      const int i = i0 + k * nt;
+      if (i < pairs) {
+        pair_row[i] = pos[k];
+        if (pos[k] >= 0) row_pair[pos[k]] = i;
+      }
+    }
   }
 }
 
 // ------------------------------------------------------------------ gather / combine
-// dst row r = src row (row_pair[r] / K); 16-byte vectors; rows beyond *total_rows are skipped.
-__global__ void gather_kernel(const uint8_t* __restrict__ src, long long src_ld, uint8_t* __restrict__ dst,
-                              long long dst_ld, int row_bytes, const int* __restrict__ row_pair, int K,
-                              const int* __restrict__ total_rows, int max_rows,
-                              const float* __restrict__ src_scale, float* __restrict__ dst_scale,
-                              int scale_groups, int src_scale_ld, int dst_scale_ld) {
-  const int r = blockIdx.x;
-  if (r >= *total_rows || r >= max_rows) return;
-  const int pr = row_pair[r];
-  uint4* d = reinterpret_cast<uint4*>(dst + (size_t)r * dst_ld);
+// dst row r = src row (row_pair[r] / K); 16-byte vectors; rows beyond *total_rows are skipped. A warp a row, four vectors of a lane on
+// their way together: a CTA a row was bound by the CTAs' lifetimes, two dependent loads and a copy each (24300 rows of 2048 bytes 18 us).
+__global__ void __launch_bounds__(128)
+gather_kernel(const uint8_t* __restrict__ src, long long src_ld, uint8_t* __restrict__ dst,
+              long long dst_ld, int row_bytes, const int* __restrict__ row_pair, int K,
+              const int* __restrict__ total_rows, int max_rows,
+              const float* __restrict__ src_scale, float* __restrict__ dst_scale,
+              int scale_groups, int src_scale_ld, int dst_scale_ld) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= max_rows) return;
+  const int pr = row_pair[r];                     // not written behind *total_rows
+  if (r >= *total_rows) return;
   if (pr < 0) return;                             // padding up to the next expert's aligned first row
-  const int tok = pr / K;
+  uint4* d = reinterpret_cast<uint4*>(dst + (size_t)r * dst_ld);
+  const int tok = pr / K, n = row_bytes / 16;
   const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)tok * src_ld);
-  for (int i = threadIdx.x; i < row_bytes / 16; i += blockDim.x) d[i] = s[i];
+  for (int i0 = lane; i0 < n; i0 += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i0 + 32 * k < n) v[k] = __ldg(s + i0 + 32 * k);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i0 + 32 * k < n) d[i0 + 32 * k] = v[k];
+  }
   if (src_scale) {
     // scales stored [group][row]
-    for (int gI = threadIdx.x; gI < scale_groups; gI += blockDim.x)
+    for (int gI = lane; gI < scale_groups; gI += 32)
       dst_scale[(size_t)gI * dst_scale_ld + r] = src_scale[(size_t)gI * src_scale_ld + tok];
   }
 }
@@ -341,21 +372,22 @@ __global__ void moe_finish_kernel(const float* __restrict__ y, long long y_ld, c
   if (gate_logit) sg = 1.f / (1.f + __expf(-gate_logit[(size_t)tok * gate_ld]));
   __syncthreads();
   if (H % 4 == 0 && y_ld % 4 == 0 && shared_ld % 4 == 0 && aligned) {
-    // four columns a thread, four experts' rows on their way together, summed in slot order
+    // four columns a thread, five experts' rows on their way together, summed in slot order
+    constexpr int kRowsAhead = 5;
     for (int h = (blockIdx.y * blockDim.x + threadIdx.x) * 4; h < H; h += gridDim.y * blockDim.x * 4) {
       float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
       uint2 sv = make_uint2(0, 0), rv = make_uint2(0, 0);
       if (shared) sv = __ldg(reinterpret_cast<const uint2*>(shared + (size_t)tok * shared_ld + h));
       if (residual) rv = __ldg(reinterpret_cast<const uint2*>(residual + (size_t)tok * H + h));
-      for (int j0 = 0; j0 < K; j0 += 4) {
-        float4 v[4];
+      for (int j0 = 0; j0 < K; j0 += kRowsAhead) {
+        float4 v[kRowsAhead];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kRowsAhead; ++i) {
           const int row = j0 + i < K ? s_row[j0 + i] : -1;
           if (row >= 0) v[i] = __ldg(reinterpret_cast<const float4*>(y + (size_t)row * y_ld + h));
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kRowsAhead; ++i) {
           if (j0 + i < K && s_row[j0 + i] >= 0) {
             const float wj = s_w[j0 + i];
             a.x += wj * v[i].x; a.y += wj * v[i].y; a.z += wj * v[i].z; a.w += wj * v[i].w;
@@ -398,6 +430,13 @@ __global__ void moe_finish_kernel(const float* __restrict__ y, long long y_ld, c
   }
 }
 
+int launch_route(const float* logits, long long ld, int T, int E, int K, int mode, const float* bias, int n_group, int topk_group, int renorm, float scaling,
+                 float* out_w, int* out_id, int out_ld, int shared_id, int gate_col, cudaStream_t stream) {
+  auto kern = E <= 128 ? route_kernel<4> : E <= 256 ? route_kernel<8> : route_kernel<16>;
+  kern<<<(T + 3) / 4, 128, 0, stream>>>(logits, ld, T, E, K, mode, bias, n_group, topk_group, renorm, scaling, out_w, out_id, out_ld, shared_id, gate_col);
+  return (int)cudaGetLastError();
+}
+
 }  // namespace
 
 extern "C" {
@@ -423,9 +462,7 @@ int mb_moe_route(const float* logits, long long ld, int T, int E, int K, int mod
   if (!logits || !out_w || !out_id || T <= 0 || E <= 0 || E > 512 || K <= 0 || K > 32 || K > E)
     return MB_ERR_BAD_ARG;
   if (n_group > 1 && (E % n_group || n_group > 32 || topk_group > n_group)) return MB_ERR_BAD_ARG;
-  route_kernel<<<(T + 3) / 4, 128, 0, stream>>>(logits, ld, T, E, K, mode, bias, n_group, topk_group,
-                                               renorm, scaling, out_w, out_id, K, -1, -1);
-  return (int)cudaGetLastError();
+  return launch_route(logits, ld, T, E, K, mode, bias, n_group, topk_group, renorm, scaling, out_w, out_id, K, -1, -1, stream);
 }
 
 // As mb_moe_route, with the outputs [T, K + 1]: slot K of every token is expert `shared_id` with
@@ -436,9 +473,7 @@ int mb_moe_route_shared(const float* logits, long long ld, int T, int E, int K, 
   if (!logits || !out_w || !out_id || T <= 0 || E <= 0 || E > 512 || K <= 0 || K >= 32 || K > E || shared_id < 0)
     return MB_ERR_BAD_ARG;
   if (n_group > 1 && (E % n_group || n_group > 32 || topk_group > n_group)) return MB_ERR_BAD_ARG;
-  route_kernel<<<(T + 3) / 4, 128, 0, stream>>>(logits, ld, T, E, K, mode, bias, n_group, topk_group,
-                                               renorm, scaling, out_w, out_id, K + 1, shared_id, gate_col);
-  return (int)cudaGetLastError();
+  return launch_route(logits, ld, T, E, K, mode, bias, n_group, topk_group, renorm, scaling, out_w, out_id, K + 1, shared_id, gate_col, stream);
 }
 
 // `align` > 1: every tile starts at a multiple of `align` rows; row_pair has `row_cap` entries
@@ -466,7 +501,7 @@ int mb_moe_gather(const void* src, long long src_ld, void* dst, long long dst_ld
                   float* dst_scale, int scale_groups, int src_scale_ld, int dst_scale_ld,
                   cudaStream_t stream) {
   if (!src || !dst || row_bytes % 16 || max_rows <= 0) return MB_ERR_BAD_ARG;
-  gather_kernel<<<max_rows, 128, 0, stream>>>(reinterpret_cast<const uint8_t*>(src), src_ld,
+  gather_kernel<<<(max_rows + 3) / 4, 128, 0, stream>>>(reinterpret_cast<const uint8_t*>(src), src_ld,
                                               reinterpret_cast<uint8_t*>(dst), dst_ld, row_bytes, row_pair, K,
                                               total_rows, max_rows, src_scale, dst_scale, scale_groups,
                                               src_scale_ld, dst_scale_ld);
