@@ -250,14 +250,18 @@ __device__ __forceinline__ void load16(const __nv_bfloat16* src, float* v) {
 // kernel is load -> reduce -> store. amax(y) is taken as max|x w| * inv_rms.
 // The two gated recipes take the same road (GATED; statistics over 128 channels are eight neighbouring threads): through shared memory
 // in 2-byte pieces 2724 rows of 4096 behind a sigmoid gate took 56 us and of 2048 behind the gated norm 24, here 20 and 12.
-template <int BPT, bool GATED>
-__global__ void __launch_bounds__(1024) row_kernel_v2(const RowParams p) {
+// WARP: a warp a row and eight rows a CTA, for many short rows: with a CTA a row an SM holds 32 of them however small they are
+// (24300 rows of 512 behind SiLU, a warp each: 26 us, so 15).
+template <int BPT, bool GATED, bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : 1024) row_kernel_v2(const RowParams p) {
   __shared__ float red[64];
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, nt = WARP ? 32 : blockDim.x;
   const int K = p.K, nblk = K >> 4;
   mb::pdl_wait();
   mb::pdl_launch_dependents();
-  const int m = p.row_index ? p.row_index[blockIdx.x] : (int)blockIdx.x;
+  const int at_row = WARP ? (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) : (int)blockIdx.x;
+  if (WARP && at_row >= p.M) return;
+  const int m = p.row_index ? p.row_index[at_row] : at_row;
   if (m < 0) return;
   float x[BPT][16];
   float ss = 0.f, mx = 0.f;
@@ -379,12 +383,15 @@ __global__ void __launch_bounds__(1024) row_kernel_v2(const RowParams p) {
   if (need_red) {
     ss = mb::warp_sum(ss);
     mx = mb::warp_max(mx);
-    const int w = tid >> 5, l = tid & 31, nw = (nt + 31) >> 5;
-    if (l == 0) { red[w] = ss; red[32 + w] = mx; }
-    __syncthreads();
-    float a = l < nw ? red[l] : 0.f, c = l < nw ? red[32 + l] : 0.f;
-    a = mb::warp_sum(a);
-    c = mb::warp_max(c);
+    float a = ss, c = mx;
+    if constexpr (!WARP) {
+      const int w = tid >> 5, l = tid & 31, nw = (nt + 31) >> 5;
+      if (l == 0) { red[w] = ss; red[32 + w] = mx; }
+      __syncthreads();
+      a = l < nw ? red[l] : 0.f; c = l < nw ? red[32 + l] : 0.f;
+      a = mb::warp_sum(a);
+      c = mb::warp_max(c);
+    }
     if (norm) inv = rsqrtf(a / (float)K + p.eps);
     amax = c * inv;
   }
@@ -476,9 +483,9 @@ __global__ void __launch_bounds__(1024) row_kernel_v2(const RowParams p) {
   }
 }
 
-template <int BPT, bool GATED = false>
+template <int BPT, bool GATED = false, bool WARP = false>
 int launch_row_v2(const RowParams& p, int threads, cudaStream_t stream) {
-  return (int)mb::launch_kernel(row_kernel_v2<BPT, GATED>, dim3(p.M), dim3(threads), 0, stream, p);
+  return (int)mb::launch_kernel(row_kernel_v2<BPT, GATED, WARP>, dim3(WARP ? (p.M + 7) / 8 : p.M), dim3(threads), 0, stream, p);
 }
 
 // Repack row-major ue4m3 scale factors [N, K/16] into the tiled layout
@@ -611,6 +618,8 @@ int mb_row_op(const MbRowArgs* a, cudaStream_t stream) {
       return launch_row_v2<1, true>(p, (nblk + 31) / 32 * 32, stream);
     if (modes && !p.xf32 && !p.residual && !p.residual_out && a->K % 16 == 0 && !(al & 15) && ld_ok &&
         (p.out_mode != OUT_FP8_G128 || a->K % 128 == 0) && nblk <= 4096) {
+      // a warp would take the row anyway; rows of more than a block a lane are faster over a CTA (2700 of 2048: 7.7 us, a warp each 13)
+      if (p.M >= 148 * 8 && nblk <= 32) return launch_row_v2<1, false, true>(p, 256, stream);
       const int bpt = (nblk + 511) / 512;
       int threads = ((nblk + bpt - 1) / bpt + 31) / 32 * 32;
       if (p.out_mode == OUT_FP8_G128) threads = (threads + 7) / 8 * 8;
