@@ -20,6 +20,7 @@ from .. import ops
 from ..config.model_config import KV_KINDS, STATE_KINDS, ModelConfig
 from ..engine.batch import ForwardBatch
 from ..ops import ACT_FOR_WEIGHT, Act
+from ..ops import dense_layer as dense
 from ..ops import reference as ref
 from ..ops import mixers
 from ..weights.loader import AttnW, FfnW, LayerW, ModelW
@@ -284,6 +285,25 @@ class Decoder:
         from .moe import moe_block
         return moe_block(self, x, lw)
 
+    def _dense_layer(self, i: int, x, lw: LayerW, batch: ForwardBatch, caches: LayerCaches):
+        """A plain attention + SwiGLU layer of an NVFP4 model as one native call; None where something of the layer, the batch or
+        the moment (calibration, adapters, traced launches) needs it block by block."""
+        c, w, f = self.cfg, lw.mixer, lw.ffn
+        if (lw.kind != "attention" or lw.ffn_kind != "dense" or type(self.tp) is not TpContext or self.calib is not None or self.kv_cal is not None
+                or w.o_in_scale <= 0.0 or f.down_in_scale <= 0.0 or c.attn_output_gate or c.qk_norm_full or c.residual_multiplier != 1.0
+                or c.ffn_act in ("relu2", "geglu") or c.window_layers or c.sliding_window > 0 or ACT_FOR_WEIGHT["nvfp4"] != "nvfp4"
+                or getattr(batch, "rope_tables", None) is not None or self._lora_for(batch, i) is not None):
+            return None
+        rows = x.table if isinstance(x, TableRows) and x.value is None else self.res(x) if isinstance(x, TableRows) else x
+        if not torch.is_tensor(rows) or not rows.is_cuda or rows.dtype != torch.bfloat16 or not rows.is_contiguous():
+            return None
+        if not dense.serves_weights(lw, c.hidden_size, c.head_dim) or dense.observed():
+            return None
+        j = caches.kv_index[i]
+        kv = caches.kv
+        return dense.dense_layer(rows, lw, batch, kv.k[j], kv.v[j], kv.k_scale[j], kv.v_scale[j], cos=self.cos, sin=self.sin, scale=self.scale,
+                                 eps=c.rms_eps, plus_one=c.norm_plus_one, gather=x.rows if rows is not x and x.value is None else None)
+
     def layer(self, i: int, x, lw: LayerW, batch: ForwardBatch, caches: LayerCaches, kv=None, kv_idx=None, run: Optional[int] = None):
         """`run`: which cache and state this run of the layer has (the layer's own unless it is looped)."""
         if isinstance(x, HyperStream):
@@ -295,6 +315,10 @@ class Decoder:
         if lw.out is not None:
             from .joint import joint_layer
             return joint_layer(self, x, lw, batch, caches, i if run is None else run)
+        if kv is None and kv_idx is None:
+            y = self._dense_layer(i, x, lw, batch, caches)
+            if y is not None:
+                return y
         if lw.kind == "attention":
             kv = kv or caches.kv
             j = caches.kv_index[i] if kv_idx is None else kv_idx

@@ -28,6 +28,7 @@
 // reshape_and_cache.cu, rope.cu, paged_decode_attn{,_fp8,_bf16_gqa,_fp8_gqa}.cu
 // (+ split-K reduce), prefill_paged_compute.cuh and attn_prefill_paged{,_fp8,_batched}.cu.
 #include "common.cuh"
+#include "op_args.h"
 #include "attention_decode.h"
 #include "visible.cuh"
 #include <type_traits>
@@ -1321,31 +1322,6 @@ int dispatch_mt(int mt, const AttnParams& p, int num_seqs, cudaStream_t stream) 
 
 extern "C" {
 
-struct MbRopeKvArgs {
-  int M, Hq, Hkv, D, rot;
-  const void* qkv;
-  long long qkv_ld;
-  int q_head_stride, k_off, v_off;
-  const int* positions;
-  const long long* slots;
-  const void* q_norm_w;
-  const void* k_norm_w;
-  int norm_plus_one;
-  float eps;
-  const float* cos_tab;
-  const float* sin_tab;
-  int max_pos;
-  void* q_out;
-  void* k_cache;
-  void* v_cache;
-  int cache_fp8;
-  const float* k_scale;
-  const float* v_scale;
-  long long num_slots;
-  uint32_t* status;
-  float* amax;             // optional [2] running max |k|, |v| of the written rows
-};
-
 // value * old_scale / *new_scale for every listed slot of an e4m3 cache [num_slots, row_elems]
 int mb_kv_rescale(void* cache, const long long* slots, int n, int row_elems, long long num_slots, float old_scale,
                   const float* new_scale, cudaStream_t stream) {
@@ -1390,55 +1366,6 @@ int mb_qk_norm_rope_kvwrite(const MbRopeKvArgs* a, cudaStream_t stream) {
   }
   return (int)mb::launch_kernel(rope_kv_kernel, dim3(a->M, (Htot + 3) / 4), dim3(128), 0, stream, p);
 }
-
-struct MbAttnArgs {
-  const void* q;
-  const void* k_cache;
-  const void* v_cache;
-  const int* block_table;
-  int max_blocks;
-  const int* q_start;
-  const int* q_len;
-  const int* ctx_len;
-  int num_seqs, max_q_len, max_ctx;
-  int Hq, Hkv, D, block_size;
-  long long num_blocks;
-  float scale;
-  int cache_fp8;
-  const float* k_scale;
-  const float* v_scale;
-  void* out;
-  void* ws;                // split-KV partials
-  size_t ws_bytes;
-  int total_rows;          // query rows (for workspace sizing)
-  int part_tokens;         // 0 = default 512
-  int window;
-  int force_mode;          // 0 auto, 1 split-KV, 2 split-Q
-  uint32_t* status;
-  void* outq;              // optional NVFP4 output (split-KV path only; MB_ERR_UNSUPPORTED otherwise)
-  int ldq;
-  void* outq_sf;
-  int outq_sf_k64;
-  float outq_gs;
-  // separate value head size and softmax variants (all zero = values as wide as keys, plain softmax)
-  int DV;                  // padded value row of the cache (0 = D); bf16 caches
-  int dv;                  // value columns stored per head (0 = DV)
-  long long out_ld;        // elements between output rows (0 = Hq * dv)
-  float out_scale;         // 0 = 1
-  int sink, split_p;
-  const float* sink_w;     // [Hq] sink scores (null: 0), with sink
-  int keep;                // with window: first tokens that stay visible
-  const void* gate;        // logits of sigmoid gates on the output (bf16), or null
-  long long gate_ld;
-  int gate_mode;           // 1 one per head, 2 one per element
-  float softcap;           // 0: off; scores become softcap tanh(score / softcap)
-  const float* turn_cos;   // [turn_max, dv / 2] or null: every output row is turned back by its position
-  const float* turn_sin;
-  int turn_max;
-  int part_fixed;          // partition size that the caller insists on for the plain decode kernel too (0 = its own)
-  int sm_count;
-  int early;               // see AttnDecodeArgs
-};
 
 // the plain decode / verify case that attention_decode.cu may serve (force_mode 1 keeps it on the split-KV kernel here)
 static bool decode_args(const MbAttnArgs* a, AttnDecodeArgs* d) {

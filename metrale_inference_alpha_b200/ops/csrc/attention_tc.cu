@@ -31,6 +31,7 @@
 // Reference behaviour covered: the prefill paged-attention family
 // (kernels/gb10/common/prefill_paged_compute.cuh:3-7,37-41), re-designed for TMEM accumulators.
 #include "common.cuh"
+#include "op_args.h"
 #include "attention_rows.h"
 #include "visible.cuh"
 
@@ -409,41 +410,6 @@ int launch_tc(const TcParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
 }
 
 }  // namespace
-
-struct MbAttnTcArgs {
-  const void* q;
-  const void* k_cache;
-  const void* v_cache;
-  const int* block_table;
-  const int* q_start;
-  const int* q_len;
-  const int* ctx_len;
-  const float* k_scale;
-  const float* v_scale;
-  void* out;
-  uint32_t* status;
-  long long num_blocks;
-  int max_blocks, num_seqs, max_q_len, Hq, Hkv, D, block_size, cache_fp8;
-  float scale;
-  int v_mn;      // 1: V staged as stored and read as an MN-major operand (no transposition)
-  long long out_ld;    // elements between output rows (0 = Hq * D)
-  float out_scale;     // 0 = 1
-  int sink, split_p;
-  const float* sink_w; // [Hq] sink scores (null: 0), with sink
-  int window, keep;    // 0 = no window; the first `keep` tokens stay visible
-  const void* gate;    // logits of sigmoid gates on the output (bf16), or null
-  long long gate_ld;
-  int gate_mode;       // 1 one per head, 2 one per element
-  float softcap;       // 0: off
-  const float* turn_cos;   // [turn_max, D / 2] or null: every output row is turned back by its position
-  const float* turn_sin;
-  int turn_max;
-  void* outq;          // plain attention at head dim 128 only: the output as NVFP4 instead of `out`, see MbGemmArgs
-  int ldq;
-  void* outq_sf;
-  int outq_sf_k64;
-  float outq_gs;
-};
 
 // Causal paged attention for prefill chunks (head dim 128 or 256). Returns 0, MB_ERR_* or a CUDA error.
 extern "C" int mb_attn_prefill_tc(const MbAttnTcArgs* a, cudaStream_t stream) {

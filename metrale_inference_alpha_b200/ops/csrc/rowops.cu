@@ -25,6 +25,7 @@
 // relu_squared.cu, residual_add.cu::sigmoid_gate_mul, quantize_bf16_to_nvfp4.cu,
 // w8a8_act_quant.cu, per_token_group_quant_fp8.
 #include "common.cuh"
+#include "op_args.h"
 #include <cstdlib>
 
 namespace {
@@ -543,36 +544,6 @@ int mb_pdl_enabled() {
   return g_pdl;
 }
 void mb_set_pdl(int mode) { g_pdl = mode < 0 ? 0 : (mode > 2 ? 2 : mode); }
-
-struct MbRowArgs {
-  int M, K, in_mode, out_mode;
-  const void* x;
-  long long x_ld;
-  const void* residual;
-  void* residual_out;
-  const void* w;
-  int w_plus_one;
-  float eps;
-  const void* gate;
-  long long gate_ld;
-  int head_dim, gate_head_stride, gate_head_off, group;
-  const float* xf32;
-  void* out;
-  long long out_ld;
-  void* out_bf16;
-  long long out_bf16_ld;
-  float* scale;
-  int scale_ld;
-  void* sf;
-  int sf_k64;
-  float static_gs;
-  const int* row_index;
-  const void* gather;
-  int gather_wide;
-  long long gather_rows;
-  void* gather_out;
-  uint32_t* status;
-};
 
 int mb_row_op(const MbRowArgs* a, cudaStream_t stream) {
   if (!a || a->M <= 0 || a->K <= 0 || (!a->x && !a->xf32) || !a->out) return MB_ERR_BAD_ARG;
