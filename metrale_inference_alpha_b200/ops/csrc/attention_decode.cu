@@ -11,15 +11,18 @@
 //     The next unit's first slices are under way while this one's warps are merged.
 //   * partitions depend on the sequence's own length only (never on the batch): part_tokens each, but at most 32 of them;
 //     the last to arrive merges them in order.
-// The tensor-core fragments are as in attention.cu: mma.sync m16n8k16, an e4m3 row widened to f16 in registers. So with an e4m3 cache
-// queries and weights are f16 here, as there: a query element beyond 65504 makes its row NaN, weights below 2^-24 of the running
-// maximum vanish.
+// The products are mma.sync m16n8k16 with the cache on the 16-row side: scores are [16 tokens x 8 query rows], outputs [16 dims x 8
+// query rows], so five query rows of a group (40 / 8 heads) waste three columns of eight, not eleven rows of sixteen, and every
+// product, exponential and accumulator register is half of what the other way round takes. Weights pass from the first product's
+// layout to the second's through movmatrix. An e4m3 row is widened to f16 in registers, so with an e4m3 cache queries and weights are
+// f16 as in attention.cu: a query element beyond 65504 makes its row NaN, weights below 2^-24 of the running maximum vanish.
 // Measured against that kernel (us): e4m3, 40 / 8 heads of 128: one sequence of 700 tokens 22.5 -> 13.7, 128 of 129 to 1151 62 -> 50,
 // nine of 4000 to 16000 73 -> 54, eight verify steps of 4 rows 31 -> 22; bf16, 33 of 100 to 2047 57 -> 32; 16 / 2 heads of 256,
 // bf16, sixteen of 200 to 2000 119 -> 22.
 #include "common.cuh"
 #include "attention_decode.h"
 #include "tensormap.h"
+#include <type_traits>
 
 namespace {
 
@@ -94,13 +97,19 @@ __device__ __forceinline__ uint32_t e4m3x2(uint32_t two) {
   asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"((uint16_t)two));
   return r;
 }
+__device__ __forceinline__ uint32_t transposed8x8(uint32_t a) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(a));
+  return r;
+}
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
-template <int D, bool FP8, int MT>
+// NT: tiles of 8 query rows
+template <int D, bool FP8, int NT>
 struct DecodeCfg {
   static constexpr int kRowB = FP8 ? D : 2 * D;              // bytes of a cached row
   static constexpr int kSpans = kRowB / 128;                 // TMA boxes (and swizzled spans) across it
@@ -110,14 +119,15 @@ struct DecodeCfg {
   static constexpr int kHalf = kTok * kRowB;                 // K or V of one step
   static constexpr int kSlot = 2 * kHalf;
   static constexpr int ring(int slots) { return 4 * slots * kSlot; }           // slot s of warp w at (s * 4 + w) * kSlot
-  static constexpr int kCtas = MT > 1 ? (D == 256 ? 1 : 2) : D == 256 ? 1 : 3;
+  static constexpr int kCtas = D == 256 ? 1 : NT > 2 ? 2 : 3;
   static constexpr int kQPitch = 2 * D + 16;                 // bytes between query rows in shared memory
+  static constexpr int kOPitch = D + 4;                      // floats between the merge buffer's rows
 };
 
-template <int D, bool FP8, int MT>
-__global__ void __launch_bounds__(128, DecodeCfg<D, FP8, MT>::kCtas)
+template <int D, bool FP8, int NT>
+__global__ void __launch_bounds__(128, DecodeCfg<D, FP8, NT>::kCtas)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeParams p) {
-  using C = DecodeCfg<D, FP8, MT>;
+  using C = DecodeCfg<D, FP8, NT>;
   constexpr int kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -125,9 +135,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const int slots = p.slots;
   __shared__ int s_last, s_wsum[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  float* s_o = reinterpret_cast<float*>(smem + p.merge_off);                  // [4 warps][rows][D]
+  float* s_o = reinterpret_cast<float*>(smem + p.merge_off);                  // [4 warps][rows][kOPitch]
   int* s_off = reinterpret_cast<int*>(smem + p.tail_off);                     // [seqs + 1]
-  float2* s_ml = reinterpret_cast<float2*>(s_off + ((p.num_seqs + 2) & ~1));  // [4][MT * 16]
+  float2* s_ml = reinterpret_cast<float2*>(s_off + ((p.num_seqs + 2) & ~1));  // [4][NT * 8]
   int4* s_len = reinterpret_cast<int4*>(smem + p.len_off);                    // [seqs]: q_len, ctx_len, q_start
   uint8_t* s_q = smem + p.len_off + p.num_seqs * 16;                          // the unit's query rows, as loaded
   if (tid == 0) {
@@ -266,50 +276,51 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   int started = slots;                                      // slices of `cur` that are under way already, at most
   while (u < units) {
     const int R = p.G * cur.qlen;
-    // ---- queries as A fragments: rows g and g + 8 of each 16-row tile
-    uint32_t qf[MT][D / 16][4];
-    int lim[MT][2], min_limit = 0x7fffffff;
+    // ---- queries as B fragments: row g of each tile of 8; lim: of the rows 2 t and 2 t + 1 whose scores this lane has
+    uint32_t qf[NT][D / 16][2];
+    int lim[NT][2], min_limit = 0x7fffffff;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int nt = 0; nt < NT; ++nt) {
+      const int r = nt * 8 + g;
+      const bool live = r < R;
+      const uint8_t* qrow = s_q + r * C::kQPitch;
 #pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const int r = mt * 16 + g + hr * 8, tq = (r * p.g_magic) >> 16;
-        const bool live = r < R;
-        lim[mt][hr] = live ? cur.ctx - cur.qlen + tq + 1 : 0x7fffffff;        // rows past R are never stored
-        min_limit = min(min_limit, lim[mt][hr]);
-        const uint8_t* qrow = s_q + r * C::kQPitch;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          uint32_t a = 0, b = 0;
-          if (live) {
-            if constexpr (FP8) {                             // four neighbouring dims: the order e4m3 fragments come in
-              const uint2 v = *reinterpret_cast<const uint2*>(qrow + ks * 32 + 8 * t);
-              const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
-              const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
-              a = pack2<true>(f0.x, f0.y);
-              b = pack2<true>(f1.x, f1.y);
-            } else {
-              a = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t);
-              b = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t + 16);
-            }
+      for (int ks = 0; ks < D / 16; ++ks) {
+        uint32_t a = 0, b = 0;
+        if (live) {
+          if constexpr (FP8) {                               // four neighbouring dims: the order e4m3 fragments come in
+            const uint2 v = *reinterpret_cast<const uint2*>(qrow + ks * 32 + 8 * t);
+            const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+            a = pack2<true>(f0.x, f0.y);
+            b = pack2<true>(f1.x, f1.y);
+          } else {
+            a = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t);
+            b = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t + 16);
           }
-          qf[mt][ks][hr] = a;
-          qf[mt][ks][2 + hr] = b;
         }
+        qf[nt][ks][0] = a;
+        qf[nt][ks][1] = b;
       }
-    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 4));
-    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 8));
-    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 16));
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = nt * 8 + 2 * t + e;
+        lim[nt][e] = c < R ? cur.ctx - cur.qlen + ((c * p.g_magic) >> 16) + 1 : 0x7fffffff;      // rows past R are never stored
+        min_limit = min(min_limit, lim[nt][e]);
+      }
+    }
+    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 1));
+    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 2));
 
-    float o[MT][D / 8][4], m_run[MT][2], l_run[MT][2];
+    float o[NT][D / 16][4], m_run[NT][2], l_run[NT][2];      // o: dims (2 g, 2 g + 1 of an e4m3 group of 16, else g, g + 8) x rows (2 t, 2 t + 1)
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      m_run[mt][0] = m_run[mt][1] = -INFINITY;
-      l_run[mt][0] = l_run[mt][1] = 0.f;
+    for (int nt = 0; nt < NT; ++nt) {
+      m_run[nt][0] = m_run[nt][1] = -INFINITY;
+      l_run[nt][0] = l_run[nt][1] = 0.f;
 #pragma unroll
-      for (int n = 0; n < D / 8; ++n)
+      for (int n = 0; n < D / 16; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o[mt][n][i] = 0.f;
+        for (int i = 0; i < 4; ++i) o[nt][n][i] = 0.f;
     }
 
     for (int i = started; i < min(cur.slices, slots); ++i) issue(cur, i, i);
@@ -330,13 +341,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         }
         __syncwarp();
       }
-      float s[MT][2 * kSub][4];
+      float s[NT][kSub][4];                                  // tokens g, g + 8 x rows 2 t, 2 t + 1
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int n = 0; n < 2 * kSub; ++n)
+        for (int b = 0; b < kSub; ++b)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s[mt][n][e] = 0.f;
+          for (int e = 0; e < 4; ++e) s[nt][b][e] = 0.f;
       const int krow = (lane & 7) + ((lane >> 4) << 3), kc = (lane >> 3) & 1, ksw = lane & 7;
       if constexpr (FP8) {
 #pragma unroll
@@ -347,62 +358,64 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             ldsm4(r, kT + (b * kSpans + (kg >> 2)) * (kSlice * 128) + krow * 128 + (((((kg & 3) * 2) + kc) ^ ksw) << 4));
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const uint32_t b00 = e4m3x2(r[h]), b01 = e4m3x2(r[h] >> 16), b10 = e4m3x2(r[2 + h]), b11 = e4m3x2(r[2 + h] >> 16);
+              const uint32_t a[4] = {e4m3x2(r[h]), e4m3x2(r[2 + h]), e4m3x2(r[h] >> 16), e4m3x2(r[2 + h] >> 16)};
 #pragma unroll
-              for (int mt = 0; mt < MT; ++mt) {
-                mma<true>(s[mt][2 * b], qf[mt][kg * 2 + h], b00, b01);
-                mma<true>(s[mt][2 * b + 1], qf[mt][kg * 2 + h], b10, b11);
-              }
+              for (int nt = 0; nt < NT; ++nt) mma<true>(s[nt][b], a, qf[nt][kg * 2 + h][0], qf[nt][kg * 2 + h][1]);
             }
           }
         }
       } else {
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
-          uint32_t b[4];
-          ldsm4(b, kT + (ks >> 2) * (kSlice * 128) + krow * 128 + (((((ks & 3) * 2) + kc) ^ ksw) << 4));
+          uint32_t r[4];
+          ldsm4(r, kT + (ks >> 2) * (kSlice * 128) + krow * 128 + (((((ks & 3) * 2) + kc) ^ ksw) << 4));
+          const uint32_t a[4] = {r[0], r[2], r[1], r[3]};
 #pragma unroll
-          for (int mt = 0; mt < MT; ++mt) {
-            mma<false>(s[mt][0], qf[mt][ks], b[0], b[1]);
-            mma<false>(s[mt][1], qf[mt][ks], b[2], b[3]);
-          }
+          for (int nt = 0; nt < NT; ++nt) mma<false>(s[nt][0], a, qf[nt][ks][0], qf[nt][ks][1]);
         }
       }
       // ---- online softmax; the running maximum moves when the new one is more than 2^8 above it
       const bool mask = pos0 + kTok > min_limit;
-      uint32_t pa[MT][kSub][4];
+      uint32_t pb[NT][kSub][2];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
+      for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
-        for (int hr = 0; hr < 2; ++hr) {
-          float v[4 * kSub], mx = -INFINITY;
+        for (int e = 0; e < 2; ++e) {
+          float mx = -INFINITY;
 #pragma unroll
-          for (int e = 0; e < 4 * kSub; ++e) {
-            v[e] = s[mt][e >> 1][hr * 2 + (e & 1)] * sc_log2;
-            if (mask && pos0 + (e >> 1) * 8 + t * 2 + (e & 1) >= lim[mt][hr]) v[e] = -INFINITY;
-            mx = fmaxf(mx, v[e]);
-          }
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-          if (mx > m_run[mt][hr] + 8.f) {                    // also true on a row's first visible token
-            const float alpha = ex2(m_run[mt][hr] - mx);
-            m_run[mt][hr] = mx;
-            l_run[mt][hr] *= alpha;
+          for (int b = 0; b < kSub; ++b)
 #pragma unroll
-            for (int n = 0; n < D / 8; ++n) {
-              o[mt][n][hr * 2] *= alpha;
-              o[mt][n][hr * 2 + 1] *= alpha;
+            for (int h = 0; h < 2; ++h) {
+              float& v = s[nt][b][2 * h + e];
+              v *= sc_log2;
+              if (mask && pos0 + b * 16 + h * 8 + g >= lim[nt][e]) v = -INFINITY;
+              mx = fmaxf(mx, v);
+            }
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+          if (mx > m_run[nt][e] + 8.f) {                     // also true on a row's first visible token
+            const float alpha = ex2(m_run[nt][e] - mx);
+            m_run[nt][e] = mx;
+            l_run[nt][e] *= alpha;
+#pragma unroll
+            for (int n = 0; n < D / 16; ++n) {
+              o[nt][n][e] *= alpha;
+              o[nt][n][2 + e] *= alpha;
             }
           }
-          const float m_use = m_run[mt][hr] == -INFINITY ? 0.f : m_run[mt][hr];
-#pragma unroll
-          for (int e = 0; e < 4 * kSub; ++e) v[e] = ex2(v[e] - m_use);
+          const float m_use = m_run[nt][e] == -INFINITY ? 0.f : m_run[nt][e];
 #pragma unroll
           for (int b = 0; b < kSub; ++b) {
-            l_run[mt][hr] += (v[4 * b] + v[4 * b + 1]) + (v[4 * b + 2] + v[4 * b + 3]);
-            pa[mt][b][hr] = pack2<FP8>(v[4 * b], v[4 * b + 1]);
-            pa[mt][b][2 + hr] = pack2<FP8>(v[4 * b + 2], v[4 * b + 3]);
+            s[nt][b][e] = ex2(s[nt][b][e] - m_use);
+            s[nt][b][2 + e] = ex2(s[nt][b][2 + e] - m_use);
+            l_run[nt][e] += s[nt][b][e] + s[nt][b][2 + e];
           }
+        }
+#pragma unroll
+        for (int b = 0; b < kSub; ++b) {
+          pb[nt][b][0] = transposed8x8(pack2<FP8>(s[nt][b][0], s[nt][b][1]));
+          pb[nt][b][1] = transposed8x8(pack2<FP8>(s[nt][b][2], s[nt][b][3]));
         }
       }
       const int vrow = (lane & 7) + (((lane >> 3) & 1) << 3), vc = lane >> 4;
@@ -411,30 +424,26 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         for (int d2 = 0; d2 < D / 32; ++d2) {
 #pragma unroll
           for (int b = 0; b < kSub; ++b) {
-          uint32_t r[4];
-          ldsm4t(r, vT + (b * kSpans + (d2 >> 2)) * (kSlice * 128) + vrow * 128 + (((((d2 & 3) * 2) + vc) ^ ksw) << 4));
+            uint32_t r[4];
+            ldsm4t(r, vT + (b * kSpans + (d2 >> 2)) * (kSlice * 128) + vrow * 128 + (((((d2 & 3) * 2) + vc) ^ ksw) << 4));
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint32_t e0 = e4m3x2(__byte_perm(r[2 * h], 0, 0x4420)), e1 = e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4420));
-            const uint32_t o0 = e4m3x2(__byte_perm(r[2 * h], 0, 0x4431)), o1 = e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4431));
+            for (int h = 0; h < 2; ++h) {
+              // even dims of the group of 16 are the tile's first eight rows, odd ones the others
+              const uint32_t a[4] = {e4m3x2(__byte_perm(r[2 * h], 0, 0x4420)), e4m3x2(__byte_perm(r[2 * h], 0, 0x4431)),
+                                     e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4420)), e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4431))};
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-              mma<true>(o[mt][(d2 * 2 + h) * 2], pa[mt][b], e0, e1);        // even dims of the group of 16
-              mma<true>(o[mt][(d2 * 2 + h) * 2 + 1], pa[mt][b], o0, o1);    // odd dims
+              for (int nt = 0; nt < NT; ++nt) mma<true>(o[nt][d2 * 2 + h], a, pb[nt][b][0], pb[nt][b][1]);
             }
-          }
           }
         }
       } else {
 #pragma unroll
         for (int n2 = 0; n2 < D / 16; ++n2) {
-          uint32_t b[4];
-          ldsm4t(b, vT + (n2 >> 2) * (kSlice * 128) + vrow * 128 + (((((n2 & 3) * 2) + vc) ^ ksw) << 4));
+          uint32_t r[4];
+          ldsm4t(r, vT + (n2 >> 2) * (kSlice * 128) + vrow * 128 + (((((n2 & 3) * 2) + vc) ^ ksw) << 4));
+          const uint32_t a[4] = {r[0], r[2], r[1], r[3]};
 #pragma unroll
-          for (int mt = 0; mt < MT; ++mt) {
-            mma<false>(o[mt][n2 * 2], pa[mt][0], b[0], b[1]);
-            mma<false>(o[mt][n2 * 2 + 1], pa[mt][0], b[2], b[3]);
-          }
+          for (int nt = 0; nt < NT; ++nt) mma<false>(o[nt][n2], a, pb[nt][0][0], pb[nt][0][1]);
         }
       }
       __syncwarp();                                          // every lane has read the slot
@@ -461,27 +470,27 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
     if (!p.over) __syncthreads();                            // every warp has its query fragments: the rows may be replaced
     if (un < units) fetch_q(next);
-    const int RP = MT * 16;
+    constexpr int RP = NT * 8;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        const int r = mt * 16 + g + hr * 8;
-        float l = l_run[mt][hr];
-        l += __shfl_xor_sync(0xffffffffu, l, 1);
-        l += __shfl_xor_sync(0xffffffffu, l, 2);
+      for (int e = 0; e < 2; ++e) {
+        const int r = nt * 8 + 2 * t + e;
+        float l = l_run[nt][e];
+        l += __shfl_xor_sync(0xffffffffu, l, 4);
+        l += __shfl_xor_sync(0xffffffffu, l, 8);
+        l += __shfl_xor_sync(0xffffffffu, l, 16);
         if (r < R) {
-          if (t == 0) s_ml[warp * RP + r] = make_float2(m_run[mt][hr], l);
-          float* orow = s_o + (warp * R + r) * D;
-          if constexpr (FP8) {
+          if (g == 0) s_ml[warp * RP + r] = make_float2(m_run[nt][e], l);
+          float* orow = s_o + (warp * R + r) * C::kOPitch;
 #pragma unroll
-            for (int dg = 0; dg < D / 16; ++dg)              // even tile (2t, 2t+1) -> dims 4t, 4t+2; odd tile -> 4t+1, 4t+3
-              *reinterpret_cast<float4*>(orow + dg * 16 + 4 * t) =
-                  make_float4(o[mt][dg * 2][hr * 2], o[mt][dg * 2 + 1][hr * 2], o[mt][dg * 2][hr * 2 + 1], o[mt][dg * 2 + 1][hr * 2 + 1]);
-          } else {
-#pragma unroll
-            for (int n = 0; n < D / 8; ++n)
-              *reinterpret_cast<float2*>(orow + n * 8 + t * 2) = make_float2(o[mt][n][hr * 2], o[mt][n][hr * 2 + 1]);
+          for (int n = 0; n < D / 16; ++n) {
+            if constexpr (FP8) {
+              *reinterpret_cast<float2*>(orow + n * 16 + 2 * g) = make_float2(o[nt][n][e], o[nt][n][2 + e]);
+            } else {
+              orow[n * 16 + g] = o[nt][n][e];
+              orow[n * 16 + 8 + g] = o[nt][n][2 + e];
+            }
           }
         }
       }
@@ -522,7 +531,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const float f = ml[w].x == -INFINITY ? 0.f : ex2(ml[w].x - mx);
-        const float4 ov = *reinterpret_cast<const float4*>(s_o + (w * R + r) * D + c4 * 4);
+        const float4 ov = *reinterpret_cast<const float4*>(s_o + (w * R + r) * C::kOPitch + c4 * 4);
         l += ml[w].y * f;
         acc.x += ov.x * f; acc.y += ov.y * f; acc.z += ov.z * f; acc.w += ov.w * f;
       }
@@ -613,28 +622,28 @@ struct Layout {
 // list of units), so it may leave room for fewer CTAs than the registers do: the grid has as many as are resident, since the
 // units are shared out over it evenly and CTAs beyond would start on theirs when the others are done (e4m3, 40 / 8 heads, 512 sequences
 // of 100 to 1000 tokens 229 -> 172 us, the split-KV kernel 207; bf16, 16 / 2 heads, 1024 of 60 to 700 136 -> 112; 32 rows 225 -> 219).
-template <int D, bool FP8, int MT>
+template <int D, bool FP8, int NT>
 Layout layout(int rows, int num_seqs, int slots = 2) {
-  using C = DecodeCfg<D, FP8, MT>;
+  using C = DecodeCfg<D, FP8, NT>;
   Layout l;
   l.slots = slots;
   // the merge buffer lies over the ring's last slots where it fits in front of the next unit's first ones
-  const int merge = 4 * rows * D * 4, behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
+  const int merge = 4 * rows * C::kOPitch * 4, behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
   l.over = behind < slots;
   l.ahead = l.over ? slots - behind : slots;
   l.merge_off = l.over ? (uint32_t)(l.ahead * 4 * C::kSlot) : (uint32_t)C::ring(slots);
   l.tail_off = l.over ? (uint32_t)C::ring(slots) : (uint32_t)(C::ring(slots) + merge);
-  l.len_off = (l.tail_off + (uint32_t)(num_seqs + 2) * 4 + 4 * MT * 16 * 8 + 8 + 15) & ~15u;
+  l.len_off = (l.tail_off + (uint32_t)(num_seqs + 2) * 4 + 4 * NT * 8 * 8 + 8 + 15) & ~15u;
   l.smem = 1024 + (size_t)l.len_off + (size_t)num_seqs * 16 + (size_t)rows * C::kQPitch;
   const int fit = (int)(228 * 1024 / (l.smem + 1024 + 256));   // a block's own kilobyte, its static arrays
   l.per_sm = fit < 1 ? 1 : fit < C::kCtas ? fit : C::kCtas;
   return l;
 }
 
-template <int D, bool FP8, int MT>
+template <int D, bool FP8, int NT>
 int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
-  using C = DecodeCfg<D, FP8, MT>;
-  auto kern = attn_decode_kernel<D, FP8, MT>;
+  using C = DecodeCfg<D, FP8, NT>;
+  auto kern = attn_decode_kernel<D, FP8, NT>;
   CUtensorMap tm[2];
   for (int i = 0; i < 2; ++i) {
     const int rc = mbh::encode_3d(&tm[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, i ? a.v_cache : a.k_cache, C::kRowB, a.Hkv, (uint64_t)a.num_blocks * a.block_size,
@@ -643,10 +652,10 @@ int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
   }
   const int rows = a.max_q_len * (a.Hq / a.Hkv), sms = a.sm_count > 0 ? a.sm_count : 148;
   const long long most = (long long)a.num_seqs * a.Hkv * p.parts;
-  Layout l = layout<D, FP8, MT>(rows, a.num_seqs);
+  Layout l = layout<D, FP8, NT>(rows, a.num_seqs);
   // few units: as deep a ring as leaves each of them a CTA of its own
   for (int slots = kMaxSlots; slots > 2; --slots) {
-    const Layout deep = layout<D, FP8, MT>(rows, a.num_seqs, slots);
+    const Layout deep = layout<D, FP8, NT>(rows, a.num_seqs, slots);
     if (deep.smem <= 220 * 1024 && (long long)sms * deep.per_sm >= most) {
       l = deep;
       break;
@@ -672,11 +681,30 @@ int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
 
 }  // namespace
 
+namespace {
+
+// f(D, FP8, NT) as types, for rows of either kind
+template <typename F>
+auto by_shape(int D, bool fp8, int rows, F&& f) {
+  auto tiles = [&](auto d, auto eight) {
+    using std::integral_constant;
+    if constexpr (d.value == 256) {
+      return rows <= 8 ? f(d, eight, integral_constant<int, 1>{}) : f(d, eight, integral_constant<int, 2>{});
+    } else {
+      return rows <= 8    ? f(d, eight, integral_constant<int, 1>{})
+             : rows <= 16 ? f(d, eight, integral_constant<int, 2>{})
+             : rows <= 24 ? f(d, eight, integral_constant<int, 3>{})
+                          : f(d, eight, integral_constant<int, 4>{});
+    }
+  };
+  if (D == 256) return fp8 ? tiles(std::integral_constant<int, 256>{}, std::true_type{}) : tiles(std::integral_constant<int, 256>{}, std::false_type{});
+  return fp8 ? tiles(std::integral_constant<int, 128>{}, std::true_type{}) : tiles(std::integral_constant<int, 128>{}, std::false_type{});
+}
+
+}  // namespace
+
 extern "C" int mb_attn_decode_per_sm(int D, int fp8, int rows, int num_seqs, size_t* smem) {
-  const bool two = rows > 16;
-  const Layout l = D == 256 ? (fp8 ? layout<256, true, 1>(rows, num_seqs) : layout<256, false, 1>(rows, num_seqs))
-                   : fp8    ? (two ? layout<128, true, 2>(rows, num_seqs) : layout<128, true, 1>(rows, num_seqs))
-                            : (two ? layout<128, false, 2>(rows, num_seqs) : layout<128, false, 1>(rows, num_seqs));
+  const Layout l = by_shape(D, fp8 != 0, rows, [&](auto d, auto eight, auto nt) { return layout<d.value, eight.value, nt.value>(rows, num_seqs); });
   if (smem) *smem = l.smem;
   return l.per_sm;
 }
@@ -713,8 +741,5 @@ int mb_attn_decode(const AttnDecodeArgs& a, cudaStream_t stream) {
     p.part_o = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a.ws) + kCntBytes);
     p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)a.total_rows * a.Hq * p.parts * a.D);
   }
-  const int mt = a.max_q_len * p.G <= 16 ? 1 : 2;
-  if (a.D == 256) return a.fp8 ? launch<256, true, 1>(a, p, stream) : launch<256, false, 1>(a, p, stream);
-  if (a.fp8) return mt == 1 ? launch<128, true, 1>(a, p, stream) : launch<128, true, 2>(a, p, stream);
-  return mt == 1 ? launch<128, false, 1>(a, p, stream) : launch<128, false, 2>(a, p, stream);
+  return by_shape(a.D, a.fp8 != 0, a.max_q_len * p.G, [&](auto d, auto eight, auto nt) { return launch<d.value, eight.value, nt.value>(a, p, stream); });
 }
