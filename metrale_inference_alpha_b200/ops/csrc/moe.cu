@@ -178,6 +178,9 @@ route_kernel(const float* __restrict__ logits, long long ld, int T, int E, int K
 // factors in blocks of 128 rows, and a token tile must start on such a block): pair i of an expert sits at
 // row off[e] + (i / tile_rows) * align + i % tile_rows. Every row of [0, row_cap) that holds no pair gets
 // row_pair = -1 (nothing is gathered or computed for it); *total_rows is the end of the last tile's slot.
+// CTAS: a cluster shares the pairs out. One CTA's atomic additions in shared memory took 24 us at 24300 pairs (every ninth on the
+// shared expert's counter); a launch of few pairs is over sooner without the cluster's barriers.
+template <int CTAS>
 __global__ void __launch_bounds__(1024)
 sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local, int tile_rows, int align, int row_cap,
             int* __restrict__ pair_row, int* __restrict__ row_pair, int* __restrict__ expert_off,
@@ -187,16 +190,17 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
   int* cnt = sm_i;                       // [num_local]
   int* off = sm_i + num_local;           // [num_local + 1]
   const int tid = threadIdx.x, nt = blockDim.x;
+  const int rank = CTAS > 1 ? (int)mb::cluster_rank() : 0;
+  const int share = (pairs + CTAS - 1) / CTAS, first = rank * share, last = min(pairs, first + share);     // this CTA's pairs
   for (int e = tid; e < num_local; e += nt) cnt[e] = 0;
   __syncthreads();
-  // eight ids of a thread on their way together (one CTA: its time is the loads' latencies, 24 us at 24300 pairs one by one)
-  constexpr int kIds = 8;
+  constexpr int kIds = 8;                // of a thread on their way together
   int id[kIds];
   auto fetch = [&](int i0) {
 #pragma unroll
-    for (int k = 0; k < kIds; ++k) id[k] = i0 + k * nt < pairs ? __ldg(ids + i0 + k * nt) - expert_lo : -1;
+    for (int k = 0; k < kIds; ++k) id[k] = i0 + k * nt < last ? __ldg(ids + i0 + k * nt) - expert_lo : -1;
   };
-  for (int i0 = tid; i0 < pairs; i0 += kIds * nt) {
+  for (int i0 = first + tid; i0 < last; i0 += kIds * nt) {
     fetch(i0);
 #pragma unroll
     for (int k = 0; k < kIds; ++k)
@@ -209,7 +213,22 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
   __shared__ int tot[2];
   {
     const int lane = tid & 31, warp = tid >> 5;
-    const int c = tid < num_local ? cnt[tid] : 0;
+    int c = 0, before = 0;               // rows of the expert: all, and of the CTAs in front
+    if constexpr (CTAS > 1) {
+      mb::cluster_sync_all();
+      if (tid < num_local) {
+#pragma unroll
+        for (int r = 0; r < CTAS; ++r) {
+          int n;
+          asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(n) : "r"(mb::dsmem_addr(mb::smem_u32(cnt + tid), r)) : "memory");
+          c += n;
+          before += r < rank ? n : 0;
+        }
+      }
+      mb::cluster_sync_all();            // the counts have been read
+    } else {
+      c = tid < num_local ? cnt[tid] : 0;
+    }
     const int my_tiles = (c + tile_rows - 1) / tile_rows;
     const int my_rows = align > 1 ? my_tiles * align : c;
     int sr = my_rows, st = my_tiles;
@@ -236,29 +255,38 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
     const int row_base = wsum[0][warp] + sr - my_rows, tile_base = wsum[1][warp] + st - my_tiles;
     if (tid < num_local) {
       off[tid] = row_base;
+      cnt[tid] = before;                                            // from here on the fill of each expert
       const int stride = align > 1 ? align : tile_rows;
-      for (int j = 0; j < my_tiles && tile_base + j < max_tiles; ++j) {
+      for (int j = 0; rank == 0 && j < my_tiles && tile_base + j < max_tiles; ++j) {
         tile_expert[tile_base + j] = tid;
         tile_row0[tile_base + j] = row_base + j * stride;
         tile_nrows[tile_base + j] = min(tile_rows, c - j * tile_rows);
       }
     }
-    if (tid == 0) { off[num_local] = tot[0]; *total_rows = tot[0]; }
-    for (int i = tot[1] + tid; i < max_tiles; i += nt) { tile_expert[i] = -1; tile_row0[i] = 0; tile_nrows[i] = 0; }
+    if (tid == 0) {
+      off[num_local] = tot[0];
+      if (rank == 0) *total_rows = tot[0];
+    }
+    if (rank == 0)
+      for (int i = tot[1] + tid; i < max_tiles; i += nt) { tile_expert[i] = -1; tile_row0[i] = 0; tile_nrows[i] = 0; }
     // rows that end up without a pair keep this -1 (the placement below overwrites the others)
-    if (align > 1)
-      for (int r = tid; r < row_cap; r += nt) row_pair[r] = -1;
+    if (align > 1) {
+      for (int r = rank * nt + tid; r < row_cap; r += CTAS * nt) row_pair[r] = -1;
+      if constexpr (CTAS > 1) {
+        __threadfence();
+        mb::cluster_sync_all();
+      }
+    }
   }
   __syncthreads();
-  for (int e = tid; e <= num_local; e += nt) expert_off[e] = off[e];
+  if (rank == 0)
+    for (int e = tid; e <= num_local; e += nt) expert_off[e] = off[e];
   // placement: every thread takes pairs tid, tid + nt, ... and claims the next free row of its pair's
   // expert with a shared-memory counter. Which row of an expert a pair lands on therefore varies from
   // run to run, the result does not: a row's GEMM output is independent of its place in the tile and
   // the combine reads rows through pair_row in slot order.
-  for (int e = tid; e < num_local; e += nt) cnt[e] = 0;         // reused as the running fill of each expert
-  __syncthreads();
-  for (int i0 = tid; i0 < pairs; i0 += kIds * nt) {
-    if (pairs > kIds * nt) fetch(i0);                            // otherwise they are still there
+  for (int i0 = first + tid; i0 < last; i0 += kIds * nt) {
+    if (share > kIds * nt) fetch(i0);                            // otherwise they are still there
     int pos[kIds];
 #pragma unroll
     for (int k = 0; k < kIds; ++k) {
@@ -271,7 +299,7 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
 #pragma unroll
     for (int k = 0; k < kIds; ++k) {
       const int i = i0 + k * nt;
-      if (i < pairs) {
+      if (i < last) {
         pair_row[i] = pos[k];
         if (pos[k] >= 0) row_pair[pos[k]] = i;
       }
@@ -484,8 +512,12 @@ int mb_moe_sort_aligned(const int* ids, int pairs, int expert_lo, int num_local,
   if (!ids || pairs <= 0 || num_local <= 0 || num_local > 1024 || tile_rows <= 0 || align <= 0 || (align > 1 && (align % tile_rows || row_cap < pairs)))
     return MB_ERR_BAD_ARG;
   const size_t smem = (2 * (size_t)num_local + 1) * sizeof(int);
-  sort_kernel<<<1, 1024, smem, stream>>>(ids, pairs, expert_lo, num_local, tile_rows, align, row_cap, pair_row, row_pair,
-                                         expert_off, tile_expert, tile_row0, tile_nrows, max_tiles, total_rows);
+  constexpr int kCluster = 8;
+  if (pairs >= 4096)
+    return (int)mb::launch_kernel_ex(sort_kernel<kCluster>, dim3(1, 1, kCluster), dim3(1024), smem, stream, kCluster, false, ids, pairs, expert_lo, num_local, tile_rows,
+                                     align, row_cap, pair_row, row_pair, expert_off, tile_expert, tile_row0, tile_nrows, max_tiles, total_rows);
+  sort_kernel<1><<<1, 1024, smem, stream>>>(ids, pairs, expert_lo, num_local, tile_rows, align, row_cap, pair_row, row_pair,
+                                            expert_off, tile_expert, tile_row0, tile_nrows, max_tiles, total_rows);
   return (int)cudaGetLastError();
 }
 
