@@ -33,7 +33,7 @@ namespace {
 constexpr int kC = 64;        // chunk length
 constexpr int kD = 128;       // key dim = value dim
 constexpr int kSlice = 32;    // value columns per scan CTA
-// workspace record of one (sequence, chunk, value head), in floats
+// workspace record of one (sequence, chunk, value head), in floats: W, Kd, Qg and P, operands of the scan's products, rounded to TF32
 constexpr int kOffW = 0, kOffU = kC * kD, kOffKd = 2 * kC * kD, kOffQg = 3 * kC * kD, kOffP = 4 * kC * kD,
               kOffGam = kOffP + kC * kC, kRec = kOffGam + 64;
 
@@ -53,11 +53,14 @@ struct GdnParams {
   uint32_t* status;
 };
 
-__device__ __forceinline__ uint32_t tf32(float f) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(f));
-  return r;
+// The nearest number of 11 significant bits (a TF32 operand), by Veltkamp's splitting: three operations of the multiply-add units. The
+// converter (cvt.rna.tf32.f32) goes through the special function units, 16 cycles of a scheduler a warp, and was what both kernels
+// waited for. Numbers beyond 2^114 have no split (NaN).
+__device__ __forceinline__ float round_tf32(float x) {
+  const float c = __fmul_rn(x, 8193.f);
+  return __fsub_rn(c, __fsub_rn(c, x));
 }
+__device__ __forceinline__ uint32_t bits(float f) { return __float_as_uint(f); }
 __device__ __forceinline__ void mma8(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -65,8 +68,9 @@ __device__ __forceinline__ void mma8(float* c, const uint32_t* a, uint32_t b0, u
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
-  hi = tf32(x);
-  lo = tf32(x - __uint_as_float(hi));
+  const float h = round_tf32(x);
+  hi = bits(h);
+  lo = bits(round_tf32(x - h));
 }
 // two fp32 multiply-adds in one instruction
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -113,13 +117,21 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(const GdnParams p) 
   float* rec = record(p, seq, c, vh);
 
   // unit-norm keys and scaled unit-norm queries, one warp per row
-  for (int i = warp; i < kC; i += 8) {
-    float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f), k4 = q4;
+  float4 q8[kC / 8], k8[kC / 8];                             // a warp's rows travel together
+#pragma unroll
+  for (int r = 0; r < kC / 8; ++r) {
+    const int i = warp + 8 * r;
+    q8[r] = k8[r] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < valid) {
       const float* row = p.conv + (size_t)(tok0 + i) * ld;
-      q4 = *reinterpret_cast<const float4*>(row + kh * kD + lane * 4);
-      k4 = *reinterpret_cast<const float4*>(row + QK + kh * kD + lane * 4);
+      q8[r] = *reinterpret_cast<const float4*>(row + kh * kD + lane * 4);
+      k8[r] = *reinterpret_cast<const float4*>(row + QK + kh * kD + lane * 4);
     }
+  }
+#pragma unroll
+  for (int r = 0; r < kC / 8; ++r) {
+    const int i = warp + 8 * r;
+    const float4 q4 = q8[r], k4 = k8[r];
     const float sq = mb::warp_sum(q4.x * q4.x + q4.y * q4.y + q4.z * q4.z + q4.w * q4.w);
     const float sk = mb::warp_sum(k4.x * k4.x + k4.y * k4.y + k4.z * k4.z + k4.w * k4.w);
     const float nq = rsqrtf(sq + 1e-6f) * rsqrtf((float)kD), nk = rsqrtf(sk + 1e-6f);
@@ -194,7 +206,7 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(const GdnParams p) 
         }
         A[(n0 + 2 * t) * kLdA + i] = -pa[0];               // transposed and negated, as the substitution reads it
         A[(n0 + 2 * t + 1) * kLdA + i] = -pa[1];
-        *reinterpret_cast<float2*>(P + i * kC + n0 + 2 * t) = make_float2(pp[0], pp[1]);
+        *reinterpret_cast<float2*>(P + i * kC + n0 + 2 * t) = make_float2(round_tf32(pp[0]), round_tf32(pp[1]));
       }
     }
   }
@@ -206,8 +218,10 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(const GdnParams p) 
     const float4 k4 = *reinterpret_cast<const float4*>(X + i * kLdX + c4);
     const float4 q4 = *reinterpret_cast<const float4*>(X + i * kLdX + kD + c4);
     const float gi = __expf(sG[i]), gl = i < valid ? __expf(g_last - sG[i]) : 0.f, bi = sBeta[i];
-    *reinterpret_cast<float4*>(rec + kOffQg + i * kD + c4) = make_float4(q4.x * gi, q4.y * gi, q4.z * gi, q4.w * gi);
-    *reinterpret_cast<float4*>(rec + kOffKd + i * kD + c4) = make_float4(k4.x * gl, k4.y * gl, k4.z * gl, k4.w * gl);
+    *reinterpret_cast<float4*>(rec + kOffQg + i * kD + c4) =
+        make_float4(round_tf32(q4.x * gi), round_tf32(q4.y * gi), round_tf32(q4.z * gi), round_tf32(q4.w * gi));
+    *reinterpret_cast<float4*>(rec + kOffKd + i * kD + c4) =
+        make_float4(round_tf32(k4.x * gl), round_tf32(k4.y * gl), round_tf32(k4.z * gl), round_tf32(k4.w * gl));
     const float w = bi * gi;
     *reinterpret_cast<float4*>(X + i * kLdX + c4) = make_float4(k4.x * w, k4.y * w, k4.z * w, k4.w * w);
     float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -239,7 +253,10 @@ __global__ void __launch_bounds__(256) gdn_chunk_prep_kernel(const GdnParams p) 
     }
     float* dst = rec + (col < kD ? kOffW + col : kOffU + col - kD);
 #pragma unroll
-    for (int i = 0; i < kC; ++i) dst[i * kD] = i < valid ? (i & 1 ? x[i / 2].y : x[i / 2].x) : 0.f;
+    for (int i = 0; i < kC; ++i) {
+      const float v = i & 1 ? x[i / 2].y : x[i / 2].x;
+      dst[i * kD] = i < valid ? (col < kD ? round_tf32(v) : v) : 0.f;
+    }
   }
 }
 
@@ -284,12 +301,26 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(const GdnParams p) 
   const int chunks = (n + kC - 1) / kC;
   float* hs = p.state + (((size_t)slot * p.v_heads + vh) * kD) * kD + slice * kSlice;
   const bool fresh = p.positions[q0] == 0;
-  for (int idx = tid; idx < kD * (kSlice / 4); idx += 256) {
-    const int k = idx / (kSlice / 4), c4 = (idx % (kSlice / 4)) * 4;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!fresh) v = *reinterpret_cast<const float4*>(hs + (size_t)k * kD + c4);
-    *reinterpret_cast<float4*>(sS + k * kLdS + c4) = v;
-  }
+  // the state slice: 16 rows a warp in registers, as its update leaves them; rounded in shared memory, as the products read it
+  const int m0 = warp * 16;
+  float st[4][4];
+  auto publish = [&]() {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float2*>(sS + (m0 + g + 8 * h) * kLdS + nt * 8 + 2 * t) = make_float2(round_tf32(st[nt][2 * h]), round_tf32(st[nt][2 * h + 1]));
+  };
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float2 v = make_float2(0.f, 0.f);
+      if (!fresh) v = *reinterpret_cast<const float2*>(hs + (size_t)(m0 + g + 8 * h) * kD + nt * 8 + 2 * t);
+      st[nt][2 * h] = v.x;
+      st[nt][2 * h + 1] = v.y;
+    }
+  publish();
   auto issue_wu = [&](int c) {
     if (c < chunks) {
       const float* rec = record(p, seq, c, vh);
@@ -325,11 +356,11 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(const GdnParams p) 
       for (int k0 = 0; k0 < kD; k0 += 8) {
         uint32_t a[4];
         const float* r0 = sW + (wr + g) * kLdW + k0 + t;
-        a[0] = tf32(r0[0]); a[1] = tf32(r0[8 * kLdW]); a[2] = tf32(r0[4]); a[3] = tf32(r0[8 * kLdW + 4]);
+        a[0] = bits(r0[0]); a[1] = bits(r0[8 * kLdW]); a[2] = bits(r0[4]); a[3] = bits(r0[8 * kLdW + 4]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float* b = sS + (k0 + t) * kLdS + wc + nt * 8 + g;
-          mma8(acc[nt], a, tf32(b[0]), tf32(b[4 * kLdS]));
+          mma8(acc[nt], a, bits(b[0]), bits(b[4 * kLdS]));
         }
       }
 #pragma unroll
@@ -338,7 +369,7 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(const GdnParams p) 
         for (int h = 0; h < 2; ++h) {
           const int o = (wr + g + 8 * h) * kLdS + wc + nt * 8 + 2 * t;
           const float2 u = *reinterpret_cast<const float2*>(sU + o);
-          *reinterpret_cast<float2*>(sV + o) = make_float2(u.x - acc[nt][2 * h], u.y - acc[nt][2 * h + 1]);
+          *reinterpret_cast<float2*>(sV + o) = make_float2(round_tf32(u.x - acc[nt][2 * h]), round_tf32(u.y - acc[nt][2 * h + 1]));
         }
     }
     __syncthreads();
@@ -351,21 +382,21 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(const GdnParams p) 
       for (int k0 = 0; k0 < kD; k0 += 8) {
         uint32_t a[4];
         const float* r0 = sQ + (wr + g) * kLdW + k0 + t;
-        a[0] = tf32(r0[0]); a[1] = tf32(r0[8 * kLdW]); a[2] = tf32(r0[4]); a[3] = tf32(r0[8 * kLdW + 4]);
+        a[0] = bits(r0[0]); a[1] = bits(r0[8 * kLdW]); a[2] = bits(r0[4]); a[3] = bits(r0[8 * kLdW + 4]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float* b = sS + (k0 + t) * kLdS + wc + nt * 8 + g;
-          mma8(acc[nt], a, tf32(b[0]), tf32(b[4 * kLdS]));
+          mma8(acc[nt], a, bits(b[0]), bits(b[4 * kLdS]));
         }
       }
       for (int k0 = 0; k0 <= wr + 8; k0 += 8) {            // P is lower triangular
         uint32_t a[4];
         const float* r0 = sP + (wr + g) * kLdP + k0 + t;
-        a[0] = tf32(r0[0]); a[1] = tf32(r0[8 * kLdP]); a[2] = tf32(r0[4]); a[3] = tf32(r0[8 * kLdP + 4]);
+        a[0] = bits(r0[0]); a[1] = bits(r0[8 * kLdP]); a[2] = bits(r0[4]); a[3] = bits(r0[8 * kLdP + 4]);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const float* b = sV + (k0 + t) * kLdS + wc + nt * 8 + g;
-          mma8(acc[nt], a, tf32(b[0]), tf32(b[4 * kLdS]));
+          mma8(acc[nt], a, bits(b[0]), bits(b[4 * kLdS]));
         }
       }
 #pragma unroll
@@ -384,42 +415,32 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_kernel(const GdnParams p) 
     cp_wait<2>();
     __syncthreads();
     {
-      const int m0 = warp * 16;
-      float acc[4][4];
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float2 s = *reinterpret_cast<const float2*>(sS + (m0 + g + 8 * h) * kLdS + nt * 8 + 2 * t);
-          acc[nt][2 * h] = gam * s.x;
-          acc[nt][2 * h + 1] = gam * s.y;
-        }
+        for (int e = 0; e < 4; ++e) st[nt][e] *= gam;
       for (int k0 = 0; k0 < kC; k0 += 8) {
         uint32_t a[4];
         const float* r0 = sKd + (k0 + t) * kLdKd + m0 + g;
-        a[0] = tf32(r0[0]); a[1] = tf32(r0[8]); a[2] = tf32(r0[4 * kLdKd]); a[3] = tf32(r0[4 * kLdKd + 8]);
+        a[0] = bits(r0[0]); a[1] = bits(r0[8]); a[2] = bits(r0[4 * kLdKd]); a[3] = bits(r0[4 * kLdKd + 8]);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
           const float* b = sV + (k0 + t) * kLdS + nt * 8 + g;
-          mma8(acc[nt], a, tf32(b[0]), tf32(b[4 * kLdS]));
+          mma8(st[nt], a, bits(b[0]), bits(b[4 * kLdS]));
         }
       }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          *reinterpret_cast<float2*>(sS + (m0 + g + 8 * h) * kLdS + nt * 8 + 2 * t) =
-              make_float2(acc[nt][2 * h], acc[nt][2 * h + 1]);
+      publish();
     }
     __syncthreads();
     issue_kd(c + 1);
   }
   cp_wait<0>();
   if (p.write_state) {
-    for (int idx = tid; idx < kD * (kSlice / 4); idx += 256) {
-      const int k = idx / (kSlice / 4), c4 = (idx % (kSlice / 4)) * 4;
-      *reinterpret_cast<float4*>(hs + (size_t)k * kD + c4) = *reinterpret_cast<const float4*>(sS + k * kLdS + c4);
-    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float2*>(hs + (size_t)(m0 + g + 8 * h) * kD + nt * 8 + 2 * t) = make_float2(st[nt][2 * h], st[nt][2 * h + 1]);
   }
 }
 
