@@ -121,7 +121,9 @@ struct DecodeCfg {
   static constexpr int ring(int slots) { return 4 * slots * kSlot; }           // slot s of warp w at (s * 4 + w) * kSlot
   static constexpr int kCtas = D == 256 ? 1 : NT > 2 ? 2 : 3;
   static constexpr int kQPitch = 2 * D + 16;                 // bytes between query rows in shared memory
-  static constexpr int kOPitch = D + 4;                      // floats between the merge buffer's rows
+  // Place of a dim in a row of the merge buffer: a warp writes dims of one group from the rows 2 t, whose banks must differ. (Longer rows
+  // would do too, but at 256 dims and 16 rows the buffer is just what fits over a slot.)
+  static __device__ __forceinline__ int place(int r, int dim) { return dim ^ ((r & 6) << 2); }
 };
 
 template <int D, bool FP8, int NT>
@@ -135,7 +137,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const int slots = p.slots;
   __shared__ int s_last, s_wsum[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  float* s_o = reinterpret_cast<float*>(smem + p.merge_off);                  // [4 warps][rows][kOPitch]
+  float* s_o = reinterpret_cast<float*>(smem + p.merge_off);                  // [4 warps][rows][D], see C::place
   int* s_off = reinterpret_cast<int*>(smem + p.tail_off);                     // [seqs + 1]
   float2* s_ml = reinterpret_cast<float2*>(s_off + ((p.num_seqs + 2) & ~1));  // [4][NT * 8]
   int4* s_len = reinterpret_cast<int4*>(smem + p.len_off);                    // [seqs]: q_len, ctx_len, q_start
@@ -482,14 +484,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         l += __shfl_xor_sync(0xffffffffu, l, 16);
         if (r < R) {
           if (g == 0) s_ml[warp * RP + r] = make_float2(m_run[nt][e], l);
-          float* orow = s_o + (warp * R + r) * C::kOPitch;
+          float* orow = s_o + (warp * R + r) * D;
 #pragma unroll
           for (int n = 0; n < D / 16; ++n) {
             if constexpr (FP8) {
-              *reinterpret_cast<float2*>(orow + n * 16 + 2 * g) = make_float2(o[nt][n][e], o[nt][n][2 + e]);
+              *reinterpret_cast<float2*>(orow + C::place(r, n * 16 + 2 * g)) = make_float2(o[nt][n][e], o[nt][n][2 + e]);
             } else {
-              orow[n * 16 + g] = o[nt][n][e];
-              orow[n * 16 + 8 + g] = o[nt][n][2 + e];
+              orow[C::place(r, n * 16 + g)] = o[nt][n][e];
+              orow[C::place(r, n * 16 + 8 + g)] = o[nt][n][2 + e];
             }
           }
         }
@@ -531,7 +533,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const float f = ml[w].x == -INFINITY ? 0.f : ex2(ml[w].x - mx);
-        const float4 ov = *reinterpret_cast<const float4*>(s_o + (w * R + r) * C::kOPitch + c4 * 4);
+        const float4 ov = *reinterpret_cast<const float4*>(s_o + (w * R + r) * D + C::place(r, c4 * 4));
         l += ml[w].y * f;
         acc.x += ov.x * f; acc.y += ov.y * f; acc.z += ov.z * f; acc.w += ov.w * f;
       }
@@ -628,7 +630,7 @@ Layout layout(int rows, int num_seqs, int slots = 2) {
   Layout l;
   l.slots = slots;
   // the merge buffer lies over the ring's last slots where it fits in front of the next unit's first ones
-  const int merge = 4 * rows * C::kOPitch * 4, behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
+  const int merge = 4 * rows * D * 4, behind = (merge + 4 * C::kSlot - 1) / (4 * C::kSlot);
   l.over = behind < slots;
   l.ahead = l.over ? slots - behind : slots;
   l.merge_off = l.over ? (uint32_t)(l.ahead * 4 * C::kSlot) : (uint32_t)C::ring(slots);
