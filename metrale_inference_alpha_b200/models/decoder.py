@@ -200,7 +200,7 @@ class Decoder:
             qkv, Hq=w.heads, Hkv=w.kv_heads, D=D, positions=rope_pos, slots=batch.slot_mapping,
             k_cache=kc, v_cache=vc, q_norm_w=qn, k_norm_w=kn, plus_one=c.norm_plus_one,
             eps=c.rms_eps, cos=cos, sin=sin, q_head_stride=qhs, k_scale=ks, v_scale=vs,
-            amax=self.kv_cal.amax_for(kv_layer) if (self.kv_cal is not None and kv_layer >= 0) else None)
+            amax=self.kv_cal.amax_for(kv_layer) if (self.kv_cal is not None and kv_layer >= 0) else None, early=kv_layer >= 0)
         fmt = ACT_FOR_WEIGHT[w.o.fmt]
         static = w.o_in_scale if (fmt == "nvfp4" and self.calib is None and not c.attn_output_gate) else 0.0
         if static > 0.0 and lora is None:

@@ -811,10 +811,11 @@ def qk_norm_rope_kvwrite(qkv: torch.Tensor, *, Hq: int, Hkv: int, D: int, positi
                          k_cache, v_cache, q_norm_w=None, k_norm_w=None, plus_one: bool = False,
                          eps: float = 1e-6, cos=None, sin=None, q_head_stride: Optional[int] = None,
                          k_off: Optional[int] = None, v_off: Optional[int] = None,
-                         k_scale=None, v_scale=None, amax=None) -> torch.Tensor:
+                         k_scale=None, v_scale=None, amax=None, early: bool = False) -> torch.Tensor:
     """Per-head q/k RMSNorm (optional) + NeoX RoPE (optional) + K/V scatter into the paged cache.
     qkv [M, *] bf16 row = q heads | k heads | v heads. Returns q [M, Hq, D] bf16. `amax`
-    (fp32 [2]): running max |k| and max |v| of the rows written, for online scale calibration."""
+    (fp32 [2]): running max |k| and max |v| of the rows written, for online scale calibration. `early`: the launch in front wrote qkv
+    and nothing before it in this call chain is still to be waited for."""
     M = qkv.shape[0]
     qhs = q_head_stride or D
     k_off = Hq * qhs if k_off is None else k_off
@@ -854,7 +855,7 @@ def qk_norm_rope_kvwrite(qkv: torch.Tensor, *, Hq: int, Hkv: int, D: int, positi
     a.k_scale, a.v_scale = _ptr(k_scale), _ptr(v_scale)
     a.num_slots = k_cache.shape[0] * k_cache.shape[1]
     a.status = _ptr(runtime(qkv.device).status)
-    a.amax = _ptr(amax)
+    a.amax, a.early = _ptr(amax), int(early)
     _native.check(_native.lib().mb_qk_norm_rope_kvwrite(C.byref(a), _stream()), "rope_kvwrite")
     _count()
     return q_out

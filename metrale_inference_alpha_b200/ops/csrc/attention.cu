@@ -60,6 +60,7 @@ struct RopeKvParams {
   long long num_slots;
   uint32_t* status;
   float* amax;                   // optional [2]: running max |k|, max |v| of the rows written (online scale calibration)
+  int early;                        // see MbRopeKvArgs
 };
 
 // In-place change of an e4m3 cache's per-tensor scale for the listed slots: value * old / new.
@@ -188,7 +189,7 @@ template <int D>
 __global__ void __launch_bounds__(256, 6) rope_kv_vec_kernel(const RopeKvParams p) {
   constexpr int kLanes = D / 8, kHeads = 256 / kLanes;
   const int m = blockIdx.x;
-  mb::pdl_wait();
+  if (!p.early) mb::pdl_wait();
   mb::pdl_launch_dependents();
   const int lane = threadIdx.x & 31, sub = threadIdx.x % kLanes, at = threadIdx.x / kLanes;
   const int Htot = p.Hq + 2 * p.Hkv, half = p.rot / 2;
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(256, 6) rope_kv_vec_kernel(const RopeKvParams 
   const long long slot = p.slots[m];
   const bool write = slot >= 0 && slot < p.num_slots;
   if (slot >= p.num_slots && threadIdx.x == 0 && p.status) atomicCAS(p.status, 0u, MB_ST_BOUNDS);
+  if (p.early) mb::pdl_wait();                               // places and tables stood before the projection began
   const __nv_bfloat16* row = p.qkv + (size_t)m * p.qkv_ld;
   for (int hb = blockIdx.y * kHeads; hb < Htot; hb += gridDim.y * kHeads) {
     const bool live = hb + at < Htot;                        // whole warps go round: the shuffles need every lane
@@ -1360,9 +1362,12 @@ int mb_qk_norm_rope_kvwrite(const MbRopeKvArgs* a, cudaStream_t stream) {
     const int full = (Htot * (a->D / 8) + 255) / 256;
     const int spread = (592 + a->M - 1) / a->M;              // 148 SMs x 4
     const dim3 grid(a->M, spread < full ? spread : full);
-    if (a->D == 64) return (int)mb::launch_kernel(rope_kv_vec_kernel<64>, grid, dim3(256), 0, stream, p);
-    if (a->D == 128) return (int)mb::launch_kernel(rope_kv_vec_kernel<128>, grid, dim3(256), 0, stream, p);
-    return (int)mb::launch_kernel(rope_kv_vec_kernel<256>, grid, dim3(256), 0, stream, p);
+    // few tokens: it comes up under the projection, looks places and tables up and waits for the rows only
+    p.early = a->early && a->M <= 512 && mb_pdl_enabled() == 2;
+    const bool pdl = p.early || mb_pdl_enabled() == 1;
+    if (a->D == 64) return (int)mb::launch_kernel_ex(rope_kv_vec_kernel<64>, grid, dim3(256), 0, stream, 1, pdl, p);
+    if (a->D == 128) return (int)mb::launch_kernel_ex(rope_kv_vec_kernel<128>, grid, dim3(256), 0, stream, 1, pdl, p);
+    return (int)mb::launch_kernel_ex(rope_kv_vec_kernel<256>, grid, dim3(256), 0, stream, 1, pdl, p);
   }
   return (int)mb::launch_kernel(rope_kv_kernel, dim3(a->M, (Htot + 3) / 4), dim3(128), 0, stream, p);
 }

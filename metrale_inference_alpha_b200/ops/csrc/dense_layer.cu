@@ -192,7 +192,7 @@ extern "C" int mb_dense_layer(MbDenseLayerArgs* args, cudaStream_t stream) {
   rk.positions = a.positions; rk.slots = a.slots; rk.q_norm_w = a.q_norm; rk.k_norm_w = a.k_norm; rk.norm_plus_one = a.plus_one; rk.eps = a.eps;
   rk.cos_tab = a.cos_tab; rk.sin_tab = a.sin_tab; rk.max_pos = a.max_pos;
   rk.q_out = s + pl.q; rk.k_cache = a.k_cache; rk.v_cache = a.v_cache; rk.cache_fp8 = a.cache_fp8; rk.k_scale = a.k_scale; rk.v_scale = a.v_scale;
-  rk.num_slots = a.num_blocks * a.block_size; rk.status = a.status;
+  rk.num_slots = a.num_blocks * a.block_size; rk.status = a.status; rk.early = 1;
   ++a.launches;
   if ((rc = mb_qk_norm_rope_kvwrite(&rk, stream))) return rc;
 

@@ -58,6 +58,7 @@ struct MbRopeKvArgs {
   long long num_slots;
   uint32_t* status;
   float* amax;             // optional [2] running max |k|, |v| of the written rows
+  int early;               // the kernel in front wrote qkv and nothing else that is read here, and launches its dependents early
 };
 
 struct MbAttnArgs {
