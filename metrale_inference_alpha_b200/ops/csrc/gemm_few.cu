@@ -133,6 +133,13 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint32_t src = tmem + ((uint32_t)(q * 32) << 16);
     float* sc = s_scale + group * (kChunk * TN);
     auto sync_group = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+    // ... and whether every warp of the group saw its sums: one whose wait ran out takes the others with it
+    auto sync_group_all = [&](bool mine) {
+      int all;
+      asm volatile("{.reg .pred p, q; setp.ne.s32 p, %1, 0; bar.red.and.pred q, %2, 128, p; selp.s32 %0, 1, 0, q;}"
+                   : "=r"(all) : "r"((int)mine), "r"(1 + group) : "memory");
+      return all != 0;
+    };
     int a = 0, turn = 0;                                     // k blocks of this group's tiles so far, tiles of this CTA
     bool ok = true;
     for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
@@ -176,7 +183,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
             }
           }
         }
-        sync_group();                                        // the scales may be replaced
+        ok = sync_group_all(ok);                             // the scales may be replaced
       }
       if (ok) {
         // a lane is a feature: a row's 32 are one piece of a line
