@@ -11,11 +11,16 @@
 //     The next unit's first slices are under way while this one's warps are merged.
 //   * partitions depend on the sequence's own length only (never on the batch): part_tokens each, but at most 32 of them;
 //     the last to arrive merges them in order.
-// The products are mma.sync m16n8k16 with the cache on the 16-row side: scores are [16 tokens x 8 query rows], outputs [16 dims x 8
-// query rows], so five query rows of a group (40 / 8 heads) waste three columns of eight, not eleven rows of sixteen, and every
-// product, exponential and accumulator register is half of what the other way round takes. Weights pass from the first product's
-// layout to the second's through movmatrix. An e4m3 row is widened to f16 in registers, so with an e4m3 cache queries and weights are
-// f16 as in attention.cu: a query element beyond 65504 makes its row NaN, weights below 2^-24 of the running maximum vanish.
+// The products are mma.sync m16n8k16. Up to 8 query rows of a group, and 17 to 24, have the cache on the 16-row side: scores are
+// [16 tokens x 8 query rows], outputs [16 dims x 8 query rows], so five query rows (40 / 8 heads) waste three columns of eight, not
+// eleven rows of sixteen, and every product, exponential and accumulator register is half of what the other way round takes; weights
+// pass from the first product's layout to the second's through movmatrix. 9 to 16 and 25 to 32 rows fill tiles of 16 as well, and
+// without the transpositions and the longer reductions over tokens these are faster with the queries there. Cache / queries on the
+// 16-row side, us, four cache heads, one sequence of 700 tokens and 128 of 129 to 1151:
+//   e4m3  8 rows 9.8, 31.8 / 10.5, 37.4;  10 rows 13.1, 41.6 / 11.9, 38.6;  20 rows 14.9, 80 / 16.8, 88;  32 rows 23.9, 131 / 17.6, 118
+//   bf16  8 rows 11.1, 39.1 / 11.4, 40.4;  10 rows 15.5, 47.0 / 12.5, 41.3;  20 rows 17.7, 105 / 17.4, 106;  32 rows 23.9, 144 / 19.8, 121
+// An e4m3 row is widened to f16 in registers, so with an e4m3 cache queries and weights are f16 as in attention.cu: a query element beyond
+// 65504 makes its row NaN, weights below 2^-24 of the running maximum vanish.
 // Measured against that kernel (us): e4m3, 40 / 8 heads of 128: one sequence of 700 tokens 22.5 -> 13.7, 128 of 129 to 1151 62 -> 50,
 // nine of 4000 to 16000 73 -> 54, eight verify steps of 4 rows 31 -> 22; bf16, 33 of 100 to 2047 57 -> 32; 16 / 2 heads of 256,
 // bf16, sixteen of 200 to 2000 119 -> 22.
@@ -108,9 +113,11 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// NT: tiles of 8 query rows
+// NT: eights of query rows
 template <int D, bool FP8, int NT>
 struct DecodeCfg {
+  static constexpr bool kPairs = NT % 2 == 0;                // queries on the products' 16-row side, else the cache
+  static constexpr int kTiles = kPairs ? NT / 2 : NT;        // tiles of 16 or of 8 query rows
   static constexpr int kRowB = FP8 ? D : 2 * D;              // bytes of a cached row
   static constexpr int kSpans = kRowB / 128;                 // TMA boxes (and swizzled spans) across it
   // slices that a warp takes together: two chains of products in flight, and one maximum and one wait for 32 tokens
@@ -123,14 +130,15 @@ struct DecodeCfg {
   static constexpr int kQPitch = 2 * D + 16;                 // bytes between query rows in shared memory
   // Place of a dim in a row of the merge buffer: a warp writes dims of one group from the rows 2 t, whose banks must differ. (Longer rows
   // would do too, but at 256 dims and 16 rows the buffer is just what fits over a slot.)
-  static __device__ __forceinline__ int place(int r, int dim) { return dim ^ ((r & 6) << 2); }
+  static __device__ __forceinline__ int place(int r, int dim) { return kPairs ? dim : dim ^ ((r & 6) << 2); }
 };
 
 template <int D, bool FP8, int NT>
 __global__ void __launch_bounds__(128, DecodeCfg<D, FP8, NT>::kCtas)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeParams p) {
   using C = DecodeCfg<D, FP8, NT>;
-  constexpr int kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok;
+  constexpr int kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok, kTiles = C::kTiles;
+  constexpr bool kPairs = C::kPairs;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t bars[4 * kMaxSlots];
@@ -278,51 +286,66 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   int started = slots;                                      // slices of `cur` that are under way already, at most
   while (u < units) {
     const int R = p.G * cur.qlen;
-    // ---- queries as B fragments: row g of each tile of 8; lim: of the rows 2 t and 2 t + 1 whose scores this lane has
-    uint32_t qf[NT][D / 16][2];
-    int lim[NT][2], min_limit = 0x7fffffff;
+    // A lane has scores and outputs of two rows of a tile, g and g + 8 or 2 t and 2 t + 1; of row e the elements at(e, 0) and at(e, 1) of
+    // every fragment. The lanes of a row differ in the bits of `t` or in those of `g`.
+    auto row_of = [&](int tile, int e) { return kPairs ? tile * 16 + g + 8 * e : tile * 8 + 2 * t + e; };
+    auto at = [](int e, int j) { return kPairs ? 2 * e + j : 2 * j + e; };
+    auto over_row = [&](auto x, auto&& f) {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int r = nt * 8 + g;
-      const bool live = r < R;
-      const uint8_t* qrow = s_q + r * C::kQPitch;
+      for (int o = kPairs ? 1 : 4; o < (kPairs ? 4 : 32); o <<= 1) x = f(x, __shfl_xor_sync(0xffffffffu, x, o));
+      return x;
+    };
+    // ---- queries as A fragments (rows g and g + 8 of each tile of 16) or B fragments (row g of each tile of 8)
+    uint32_t qf[kTiles][D / 16][kPairs ? 4 : 2];
+    int lim[kTiles][2], min_limit = 0x7fffffff;
 #pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t a = 0, b = 0;
-        if (live) {
-          if constexpr (FP8) {                               // four neighbouring dims: the order e4m3 fragments come in
-            const uint2 v = *reinterpret_cast<const uint2*>(qrow + ks * 32 + 8 * t);
-            const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
-            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
-            a = pack2<true>(f0.x, f0.y);
-            b = pack2<true>(f1.x, f1.y);
-          } else {
-            a = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t);
-            b = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t + 16);
+    for (int tile = 0; tile < kTiles; ++tile) {
+#pragma unroll
+      for (int hr = 0; hr < (kPairs ? 2 : 1); ++hr) {
+        const int r = kPairs ? tile * 16 + g + hr * 8 : tile * 8 + g;
+        const bool live = r < R;
+        const uint8_t* qrow = s_q + r * C::kQPitch;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          uint32_t a = 0, b = 0;
+          if (live) {
+            if constexpr (FP8) {                             // four neighbouring dims: the order e4m3 fragments come in
+              const uint2 v = *reinterpret_cast<const uint2*>(qrow + ks * 32 + 8 * t);
+              const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+              const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+              a = pack2<true>(f0.x, f0.y);
+              b = pack2<true>(f1.x, f1.y);
+            } else {
+              a = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t);
+              b = *reinterpret_cast<const uint32_t*>(qrow + ks * 32 + 4 * t + 16);
+            }
           }
+          qf[tile][ks][hr] = a;
+          qf[tile][ks][kPairs ? 2 + hr : 1] = b;
         }
-        qf[nt][ks][0] = a;
-        qf[nt][ks][1] = b;
       }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int c = nt * 8 + 2 * t + e;
-        lim[nt][e] = c < R ? cur.ctx - cur.qlen + ((c * p.g_magic) >> 16) + 1 : 0x7fffffff;      // rows past R are never stored
-        min_limit = min(min_limit, lim[nt][e]);
+        const int r = row_of(tile, e);
+        lim[tile][e] = r < R ? cur.ctx - cur.qlen + ((r * p.g_magic) >> 16) + 1 : 0x7fffffff;    // rows past R are never stored
+        min_limit = min(min_limit, lim[tile][e]);
       }
     }
-    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 1));
-    min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, 2));
+    // over all rows of the tiles
+#pragma unroll
+    for (int o = kPairs ? 4 : 1; o < (kPairs ? 32 : 4); o <<= 1) min_limit = min(min_limit, __shfl_xor_sync(0xffffffffu, min_limit, o));
 
-    float o[NT][D / 16][4], m_run[NT][2], l_run[NT][2];      // o: dims (2 g, 2 g + 1 of an e4m3 group of 16, else g, g + 8) x rows (2 t, 2 t + 1)
+    // o: 8 dims a fragment, or 16 (dims 2 g, 2 g + 1 of an e4m3 group of 16, else g, g + 8)
+    constexpr int kO = kPairs ? D / 8 : D / 16;
+    float o[kTiles][kO][4], m_run[kTiles][2], l_run[kTiles][2];
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      m_run[nt][0] = m_run[nt][1] = -INFINITY;
-      l_run[nt][0] = l_run[nt][1] = 0.f;
+    for (int tile = 0; tile < kTiles; ++tile) {
+      m_run[tile][0] = m_run[tile][1] = -INFINITY;
+      l_run[tile][0] = l_run[tile][1] = 0.f;
 #pragma unroll
-      for (int n = 0; n < D / 16; ++n)
+      for (int n = 0; n < kO; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o[nt][n][i] = 0.f;
+        for (int i = 0; i < 4; ++i) o[tile][n][i] = 0.f;
     }
 
     for (int i = started; i < min(cur.slices, slots); ++i) issue(cur, i, i);
@@ -343,14 +366,28 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         }
         __syncwarp();
       }
-      float s[NT][kSub][4];                                  // tokens g, g + 8 x rows 2 t, 2 t + 1
+      constexpr int kS = kPairs ? 2 * kSub : kSub;           // fragments of 8 or of 16 tokens
+      float s[kTiles][kS][4];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
+      for (int tile = 0; tile < kTiles; ++tile)
 #pragma unroll
-        for (int b = 0; b < kSub; ++b)
+        for (int n = 0; n < kS; ++n)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) s[nt][b][e] = 0.f;
+          for (int e = 0; e < 4; ++e) s[tile][n][e] = 0.f;
       const int krow = (lane & 7) + ((lane >> 4) << 3), kc = (lane >> 3) & 1, ksw = lane & 7;
+      // keys of 16 tokens at 16 dims: k0, k1 of the first eight tokens, k2, k3 of the others
+      auto score = [&](int b, int ks, uint32_t k0, uint32_t k1, uint32_t k2, uint32_t k3) {
+#pragma unroll
+        for (int tile = 0; tile < kTiles; ++tile) {
+          if constexpr (kPairs) {
+            mma<FP8>(s[tile][2 * b], qf[tile][ks], k0, k1);
+            mma<FP8>(s[tile][2 * b + 1], qf[tile][ks], k2, k3);
+          } else {
+            const uint32_t a[4] = {k0, k2, k1, k3};
+            mma<FP8>(s[tile][b], a, qf[tile][ks][0], qf[tile][ks][1]);
+          }
+        }
+      };
       if constexpr (FP8) {
 #pragma unroll
         for (int kg = 0; kg < D / 32; ++kg) {
@@ -359,11 +396,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             uint32_t r[4];
             ldsm4(r, kT + (b * kSpans + (kg >> 2)) * (kSlice * 128) + krow * 128 + (((((kg & 3) * 2) + kc) ^ ksw) << 4));
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint32_t a[4] = {e4m3x2(r[h]), e4m3x2(r[2 + h]), e4m3x2(r[h] >> 16), e4m3x2(r[2 + h] >> 16)};
-#pragma unroll
-              for (int nt = 0; nt < NT; ++nt) mma<true>(s[nt][b], a, qf[nt][kg * 2 + h][0], qf[nt][kg * 2 + h][1]);
-            }
+            for (int h = 0; h < 2; ++h) score(b, kg * 2 + h, e4m3x2(r[h]), e4m3x2(r[h] >> 16), e4m3x2(r[2 + h]), e4m3x2(r[2 + h] >> 16));
           }
         }
       } else {
@@ -371,56 +404,76 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         for (int ks = 0; ks < D / 16; ++ks) {
           uint32_t r[4];
           ldsm4(r, kT + (ks >> 2) * (kSlice * 128) + krow * 128 + (((((ks & 3) * 2) + kc) ^ ksw) << 4));
-          const uint32_t a[4] = {r[0], r[2], r[1], r[3]};
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) mma<false>(s[nt][0], a, qf[nt][ks][0], qf[nt][ks][1]);
+          score(0, ks, r[0], r[1], r[2], r[3]);
         }
       }
       // ---- online softmax; the running maximum moves when the new one is more than 2^8 above it
       const bool mask = pos0 + kTok > min_limit;
-      uint32_t pb[NT][kSub][2];
+      uint32_t pw[kTiles][kSub][kPairs ? 4 : 2];             // weights, as the second product's operand
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
+      for (int tile = 0; tile < kTiles; ++tile) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           float mx = -INFINITY;
 #pragma unroll
-          for (int b = 0; b < kSub; ++b)
+          for (int n = 0; n < kS; ++n)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float& v = s[nt][b][2 * h + e];
+            for (int j = 0; j < 2; ++j) {
+              float& v = s[tile][n][at(e, j)];
               v *= sc_log2;
-              if (mask && pos0 + b * 16 + h * 8 + g >= lim[nt][e]) v = -INFINITY;
+              if (mask && pos0 + (kPairs ? n * 8 + 2 * t + j : n * 16 + j * 8 + g) >= lim[tile][e]) v = -INFINITY;
               mx = fmaxf(mx, v);
             }
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-          if (mx > m_run[nt][e] + 8.f) {                     // also true on a row's first visible token
-            const float alpha = ex2(m_run[nt][e] - mx);
-            m_run[nt][e] = mx;
-            l_run[nt][e] *= alpha;
+          mx = over_row(mx, [](float x, float y) { return fmaxf(x, y); });
+          if (mx > m_run[tile][e] + 8.f) {                   // also true on a row's first visible token
+            const float alpha = ex2(m_run[tile][e] - mx);
+            m_run[tile][e] = mx;
+            l_run[tile][e] *= alpha;
 #pragma unroll
-            for (int n = 0; n < D / 16; ++n) {
-              o[nt][n][e] *= alpha;
-              o[nt][n][2 + e] *= alpha;
+            for (int n = 0; n < kO; ++n) {
+              o[tile][n][at(e, 0)] *= alpha;
+              o[tile][n][at(e, 1)] *= alpha;
             }
           }
-          const float m_use = m_run[nt][e] == -INFINITY ? 0.f : m_run[nt][e];
+          const float m_use = m_run[tile][e] == -INFINITY ? 0.f : m_run[tile][e];
+#pragma unroll
+          for (int n = 0; n < kS; ++n)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) s[tile][n][at(e, j)] = ex2(s[tile][n][at(e, j)] - m_use);
 #pragma unroll
           for (int b = 0; b < kSub; ++b) {
-            s[nt][b][e] = ex2(s[nt][b][e] - m_use);
-            s[nt][b][2 + e] = ex2(s[nt][b][2 + e] - m_use);
-            l_run[nt][e] += s[nt][b][e] + s[nt][b][2 + e];
+            if constexpr (kPairs) {
+              const float *v0 = s[tile][2 * b] + 2 * e, *v1 = s[tile][2 * b + 1] + 2 * e;
+              l_run[tile][e] += (v0[0] + v0[1]) + (v1[0] + v1[1]);
+              pw[tile][b][e] = pack2<FP8>(v0[0], v0[1]);
+              pw[tile][b][2 + e] = pack2<FP8>(v1[0], v1[1]);
+            } else {
+              l_run[tile][e] += s[tile][b][e] + s[tile][b][2 + e];
+            }
           }
         }
+        if constexpr (!kPairs) {
 #pragma unroll
-        for (int b = 0; b < kSub; ++b) {
-          pb[nt][b][0] = transposed8x8(pack2<FP8>(s[nt][b][0], s[nt][b][1]));
-          pb[nt][b][1] = transposed8x8(pack2<FP8>(s[nt][b][2], s[nt][b][3]));
+          for (int b = 0; b < kSub; ++b) {
+            pw[tile][b][0] = transposed8x8(pack2<FP8>(s[tile][b][0], s[tile][b][1]));
+            pw[tile][b][1] = transposed8x8(pack2<FP8>(s[tile][b][2], s[tile][b][3]));
+          }
         }
       }
       const int vrow = (lane & 7) + (((lane >> 3) & 1) << 3), vc = lane >> 4;
+      // values of 16 tokens at 16 dims: v0, v1 of the first eight dims (of an e4m3 group the even ones), v2, v3 of the others
+      auto weigh = [&](int b, int n, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+#pragma unroll
+        for (int tile = 0; tile < kTiles; ++tile) {
+          if constexpr (kPairs) {
+            mma<FP8>(o[tile][2 * n], pw[tile][b], v0, v1);
+            mma<FP8>(o[tile][2 * n + 1], pw[tile][b], v2, v3);
+          } else {
+            const uint32_t a[4] = {v0, v2, v1, v3};
+            mma<FP8>(o[tile][n], a, pw[tile][b][0], pw[tile][b][1]);
+          }
+        }
+      };
       if constexpr (FP8) {
 #pragma unroll
         for (int d2 = 0; d2 < D / 32; ++d2) {
@@ -429,13 +482,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             uint32_t r[4];
             ldsm4t(r, vT + (b * kSpans + (d2 >> 2)) * (kSlice * 128) + vrow * 128 + (((((d2 & 3) * 2) + vc) ^ ksw) << 4));
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              // even dims of the group of 16 are the tile's first eight rows, odd ones the others
-              const uint32_t a[4] = {e4m3x2(__byte_perm(r[2 * h], 0, 0x4420)), e4m3x2(__byte_perm(r[2 * h], 0, 0x4431)),
-                                     e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4420)), e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4431))};
-#pragma unroll
-              for (int nt = 0; nt < NT; ++nt) mma<true>(o[nt][d2 * 2 + h], a, pb[nt][b][0], pb[nt][b][1]);
-            }
+            for (int h = 0; h < 2; ++h)
+              weigh(b, d2 * 2 + h, e4m3x2(__byte_perm(r[2 * h], 0, 0x4420)), e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4420)),
+                    e4m3x2(__byte_perm(r[2 * h], 0, 0x4431)), e4m3x2(__byte_perm(r[2 * h + 1], 0, 0x4431)));
           }
         }
       } else {
@@ -443,9 +492,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         for (int n2 = 0; n2 < D / 16; ++n2) {
           uint32_t r[4];
           ldsm4t(r, vT + (n2 >> 2) * (kSlice * 128) + vrow * 128 + (((((n2 & 3) * 2) + vc) ^ ksw) << 4));
-          const uint32_t a[4] = {r[0], r[2], r[1], r[3]};
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) mma<false>(o[nt][n2], a, pb[nt][0][0], pb[nt][0][1]);
+          weigh(0, n2, r[0], r[1], r[2], r[3]);
         }
       }
       __syncwarp();                                          // every lane has read the slot
@@ -474,24 +521,28 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     if (un < units) fetch_q(next);
     constexpr int RP = NT * 8;
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int tile = 0; tile < kTiles; ++tile)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int r = nt * 8 + 2 * t + e;
-        float l = l_run[nt][e];
-        l += __shfl_xor_sync(0xffffffffu, l, 4);
-        l += __shfl_xor_sync(0xffffffffu, l, 8);
-        l += __shfl_xor_sync(0xffffffffu, l, 16);
+        const int r = row_of(tile, e);
+        const float l = over_row(l_run[tile][e], [](float x, float y) { return x + y; });
         if (r < R) {
-          if (g == 0) s_ml[warp * RP + r] = make_float2(m_run[nt][e], l);
+          if ((kPairs ? t : g) == 0) s_ml[warp * RP + r] = make_float2(m_run[tile][e], l);
           float* orow = s_o + (warp * R + r) * D;
 #pragma unroll
           for (int n = 0; n < D / 16; ++n) {
-            if constexpr (FP8) {
-              *reinterpret_cast<float2*>(orow + C::place(r, n * 16 + 2 * g)) = make_float2(o[nt][n][e], o[nt][n][2 + e]);
+            if constexpr (kPairs && FP8) {                   // even dims (2 t, 2 t + 1 of their eight), odd ones: dims 4 t to 4 t + 3
+              *reinterpret_cast<float4*>(orow + n * 16 + 4 * t) =
+                  make_float4(o[tile][2 * n][2 * e], o[tile][2 * n + 1][2 * e], o[tile][2 * n][2 * e + 1], o[tile][2 * n + 1][2 * e + 1]);
+            } else if constexpr (kPairs) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float2*>(orow + n * 16 + h * 8 + 2 * t) = make_float2(o[tile][2 * n + h][2 * e], o[tile][2 * n + h][2 * e + 1]);
+            } else if constexpr (FP8) {
+              *reinterpret_cast<float2*>(orow + C::place(r, n * 16 + 2 * g)) = make_float2(o[tile][n][e], o[tile][n][2 + e]);
             } else {
-              orow[C::place(r, n * 16 + g)] = o[nt][n][e];
-              orow[C::place(r, n * 16 + 8 + g)] = o[nt][n][2 + e];
+              orow[C::place(r, n * 16 + g)] = o[tile][n][e];
+              orow[C::place(r, n * 16 + 8 + g)] = o[tile][n][2 + e];
             }
           }
         }
@@ -655,8 +706,9 @@ int launch(const AttnDecodeArgs& a, DecodeParams& p, cudaStream_t stream) {
   const int rows = a.max_q_len * (a.Hq / a.Hkv), sms = a.sm_count > 0 ? a.sm_count : 148;
   const long long most = (long long)a.num_seqs * a.Hkv * p.parts;
   Layout l = layout<D, FP8, NT>(rows, a.num_seqs);
-  // few units: as deep a ring as leaves each of them a CTA of its own
-  for (int slots = kMaxSlots; slots > 2; --slots) {
+  // few units: as deep a ring as leaves each of them a CTA of its own. 25 to 32 rows spill registers, which go through what the ring leaves
+  // of L1: one e4m3 sequence of 700 tokens at 32 rows 17.4 us with two steps, 17.6 with four, 19.4 with six.
+  for (int slots = NT > 3 ? 4 : kMaxSlots; slots > 2; --slots) {
     const Layout deep = layout<D, FP8, NT>(rows, a.num_seqs, slots);
     if (deep.smem <= 220 * 1024 && (long long)sms * deep.per_sm >= most) {
       l = deep;
