@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128, DecodeCfg<D, FP8, NT>::kCtas)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeParams p) {
   using C = DecodeCfg<D, FP8, NT>;
   constexpr int kSpans = C::kSpans, kSub = C::kSub, kTok = C::kTok, kTiles = C::kTiles;
-  constexpr bool kPairs = C::kPairs;
+  constexpr bool kPairs = C::kPairs, kThroughBf16 = NT > 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t bars[4 * kMaxSlots];
@@ -552,13 +552,18 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     auto store = [&](int r, int c4, float4 a) {
       const int tq = (r * p.g_magic) >> 16, head = cur.kvh * p.G + r - tq * p.G;
       const uint32_t m = cur.qs + tq;
+      // 17 rows and more quantise the bf16 value, as the row kernel behind this one did: the same bits as with it. Up to 16 the 32-bit one.
+      if (kThroughBf16 && p.outq) {
+        auto rounded = [](float x) { return __bfloat162float(__float2bfloat16(x)); };
+        a = make_float4(rounded(a.x), rounded(a.y), rounded(a.z), rounded(a.w));
+      }
       if (p.outq) {
         float bmax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)));
         bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
         bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
         const uint8_t sfc = mb::float_to_e4m3(bmax / (6.f * p.outq_gs));
         const float sff = mb::e4m3_to_float(sfc);
-        const float qi = sff > 0.f ? __fdividef(1.f, sff * p.outq_gs) : 0.f;
+        const float qi = sff > 0.f ? (kThroughBf16 ? 1.f / (sff * p.outq_gs) : __fdividef(1.f, sff * p.outq_gs)) : 0.f;
         const uint32_t w = mb::e2m1x2_pack(a.x * qi, a.y * qi) | (mb::e2m1x2_pack(a.z * qi, a.w * qi) << 8);
         const int col = head * D + c4 * 4, kb = col >> 4;
         *reinterpret_cast<uint16_t*>(p.outq + (size_t)m * p.ldq + (col >> 1)) = (uint16_t)w;
