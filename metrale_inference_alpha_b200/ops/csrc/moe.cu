@@ -308,15 +308,18 @@ sort_kernel(const int* __restrict__ ids, int pairs, int expert_lo, int num_local
 }
 
 // ------------------------------------------------------------------ gather / combine
-// dst row r = src row (row_pair[r] / K); 16-byte vectors; rows beyond *total_rows are skipped. A warp a row, four vectors of a lane on
-// their way together: a CTA a row was bound by the CTAs' lifetimes, two dependent loads and a copy each (24300 rows of 2048 bytes 18 us).
+// dst row r = src row (row_pair[r] / K); 16-byte vectors; rows beyond *total_rows are skipped. WARPS warps a row, four vectors of a lane
+// on their way together. A CTA a short row was bound by the CTAs' lifetimes, two dependent loads and a copy each (24300 rows of 2048
+// bytes 18 us); a warp alone takes a long row in several turns, one after the other.
+template <int WARPS>
 __global__ void __launch_bounds__(128)
 gather_kernel(const uint8_t* __restrict__ src, long long src_ld, uint8_t* __restrict__ dst,
               long long dst_ld, int row_bytes, const int* __restrict__ row_pair, int K,
               const int* __restrict__ total_rows, int max_rows,
               const float* __restrict__ src_scale, float* __restrict__ dst_scale,
               int scale_groups, int src_scale_ld, int dst_scale_ld) {
-  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  constexpr int kLanes = 32 * WARPS;
+  const int r = blockIdx.x * (4 / WARPS) + threadIdx.x / kLanes, lane = threadIdx.x % kLanes;
   if (r >= max_rows) return;
   const int pr = row_pair[r];                     // not written behind *total_rows
   if (r >= *total_rows) return;
@@ -324,18 +327,18 @@ gather_kernel(const uint8_t* __restrict__ src, long long src_ld, uint8_t* __rest
   uint4* d = reinterpret_cast<uint4*>(dst + (size_t)r * dst_ld);
   const int tok = pr / K, n = row_bytes / 16;
   const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)tok * src_ld);
-  for (int i0 = lane; i0 < n; i0 += 128) {
+  for (int i0 = lane; i0 < n; i0 += 4 * kLanes) {
     uint4 v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (i0 + 32 * k < n) v[k] = __ldg(s + i0 + 32 * k);
+      if (i0 + kLanes * k < n) v[k] = __ldg(s + i0 + kLanes * k);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (i0 + 32 * k < n) d[i0 + 32 * k] = v[k];
+      if (i0 + kLanes * k < n) d[i0 + kLanes * k] = v[k];
   }
   if (src_scale) {
     // scales stored [group][row]
-    for (int gI = lane; gI < scale_groups; gI += 32)
+    for (int gI = lane; gI < scale_groups; gI += kLanes)
       dst_scale[(size_t)gI * dst_scale_ld + r] = src_scale[(size_t)gI * src_scale_ld + tok];
   }
 }
@@ -533,10 +536,14 @@ int mb_moe_gather(const void* src, long long src_ld, void* dst, long long dst_ld
                   float* dst_scale, int scale_groups, int src_scale_ld, int dst_scale_ld,
                   cudaStream_t stream) {
   if (!src || !dst || row_bytes % 16 || max_rows <= 0) return MB_ERR_BAD_ARG;
-  gather_kernel<<<(max_rows + 3) / 4, 128, 0, stream>>>(reinterpret_cast<const uint8_t*>(src), src_ld,
-                                              reinterpret_cast<uint8_t*>(dst), dst_ld, row_bytes, row_pair, K,
-                                              total_rows, max_rows, src_scale, dst_scale, scale_groups,
-                                              src_scale_ld, dst_scale_ld);
+  // A warp a row / a CTA a row, us. 8 rows of 2048 bytes 2.05 / 1.95, of 4096 2.05 / 1.68, of 7168 3.25 / 2.05, of 16384 4.41 / 2.44; 512 rows of
+  // 2048 2.22 / 2.31, of 4096 2.15 / 2.02; 2400 rows of 4096 3.46 / 3.46, of 5120 3.97 / 3.81; 24300 rows of 2048 12.4 / 17.5, of 4096
+  // 18.8 / 22.6, of 5120 23.9 / 25.8, of 6144 28.7 / 29.4, of 7168 40.2 / 40.6, of 16384 107 / 98.
+  const bool warp_rows = row_bytes <= (max_rows >= 2048 ? 5120 : 2048);
+  auto kern = warp_rows ? gather_kernel<1> : gather_kernel<4>;
+  kern<<<warp_rows ? (max_rows + 3) / 4 : max_rows, 128, 0, stream>>>(reinterpret_cast<const uint8_t*>(src), src_ld, reinterpret_cast<uint8_t*>(dst), dst_ld,
+                                                                      row_bytes, row_pair, K, total_rows, max_rows, src_scale, dst_scale, scale_groups,
+                                                                      src_scale_ld, dst_scale_ld);
   return (int)cudaGetLastError();
 }
 
