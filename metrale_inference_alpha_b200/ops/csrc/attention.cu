@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256, 6) rope_kv_vec_kernel(const RopeKvParams 
     const int kind = head < p.Hq ? 0 : head < p.Hq + p.Hkv ? 1 : 2;
     const int h = kind == 0 ? head : kind == 1 ? head - p.Hq : head - p.Hq - p.Hkv;
     const __nv_bfloat16* src = row + (kind == 0 ? (size_t)h * p.q_head_stride : (size_t)(kind == 1 ? p.k_off : p.v_off) + (size_t)h * D);
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src + sub * 8));
+    const uint4 raw = *reinterpret_cast<const uint4*>(src + sub * 8);        // not __ldg: the projection may write it while this CTA is up
     const __nv_bfloat162* rb = reinterpret_cast<const __nv_bfloat162*>(&raw);
     float v[8];
 #pragma unroll
