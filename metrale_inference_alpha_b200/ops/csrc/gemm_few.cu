@@ -77,7 +77,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   mb::tc_fence_after();
   const uint32_t tmem = tmem_base_s;
   mb::pdl_launch_dependents();
-  mb::pdl_wait();                                            // the work list and the rows come from preceding kernels
+  // The work list, the rows and their scales come from preceding kernels, which may write them while this CTA is up: ordinary loads.
+  mb::pdl_wait();
 
   // item i: entry i / n_tiles, features (i % n_tiles) * 128; entries without rows are passed over by every role alike
   if (warp == 0) {
@@ -85,7 +86,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       int g = 0;
       bool ok = true;
       for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
-        const int mt = i / p.n_tiles, e = __ldg(p.tile_expert + mt), row0 = __ldg(p.tile_row0 + mt);
+        const int mt = i / p.n_tiles, e = p.tile_expert[mt], row0 = p.tile_row0[mt];
         if (e < 0) continue;
         const int w_row0 = e * p.n_per_expert + (i - mt * p.n_tiles) * 128;
         for (int kb = 0; kb < nkb; ++kb, ++g) {
@@ -106,7 +107,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       int g = 0, turn = 0, mine[2] = {0, 0};                 // k blocks so far: all, and of either group's tiles
       bool ok = true;
       for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
-        if (__ldg(p.tile_expert + i / p.n_tiles) < 0) continue;
+        if (p.tile_expert[i / p.n_tiles] < 0) continue;
         const int group = turn++ & 1;
         int a = group ? mine[1] : mine[0];
         for (int kb = 0; kb < nkb; ++kb, ++g, ++a) {
@@ -143,10 +144,10 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     int a = 0, turn = 0;                                     // k blocks of this group's tiles so far, tiles of this CTA
     bool ok = true;
     for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
-      const int mt = i / p.n_tiles, nt = i - mt * p.n_tiles, e = __ldg(p.tile_expert + mt);
+      const int mt = i / p.n_tiles, nt = i - mt * p.n_tiles, e = p.tile_expert[mt];
       if (e < 0) continue;
       if ((turn++ & 1) != group) continue;
-      const int row0 = __ldg(p.tile_row0 + mt), rows = __ldg(p.tile_nrows + mt);
+      const int row0 = p.tile_row0[mt], rows = p.tile_nrows[mt];
       const float* wsp = p.w_scale + (size_t)((e * p.n_per_expert >> 7) + nt) * nkb;
       float acc[TN];
 #pragma unroll
@@ -155,7 +156,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         const int kc = min(kChunk, nkb - k0);
         for (int x = et; x < kc * TN; x += 128) {
           const int kb = x / TN, r = x % TN;
-          sc[x] = r < rows ? __ldg(p.a_scale + (size_t)(k0 + kb) * p.a_ld + row0 + r) * __ldg(wsp + k0 + kb) : 0.f;
+          sc[x] = r < rows ? p.a_scale[(size_t)(k0 + kb) * p.a_ld + row0 + r] * __ldg(wsp + k0 + kb) : 0.f;
         }
         sync_group();
         for (int kb = 0; kb < kc; ++kb, ++a) {
