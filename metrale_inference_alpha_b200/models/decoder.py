@@ -457,12 +457,14 @@ class Decoder:
         [R, vocab / size] (greedy selection then merges per-rank maxima instead)."""
         x = self.backbone(batch, caches)
         if batch.logit_rows.numel() != x.shape[0]:
+            wanted = batch.logit_rows
             if not torch.is_tensor(x) and hasattr(x, "take"):
-                rows = x.take(batch.logit_rows)
-            elif torch.is_tensor(self.w.final_norm) and self.full(x).dtype == torch.bfloat16:
-                rows = TableRows(self.full(x), batch.logit_rows)       # the final norm takes its rows itself
-            else:
-                rows = self.full(x).index_select(0, batch.logit_rows)
+                rows = x.take(wanted)
+            elif (torch.is_tensor(self.w.final_norm) and self.full(x).dtype == torch.bfloat16 and wanted.is_cuda
+                  and wanted.device == self.full(x).device and wanted.dim() == 1 and wanted.is_contiguous() and wanted.dtype in (torch.int32, torch.int64)):
+                rows = TableRows(self.full(x), wanted)                 # the final norm takes its rows itself
+            else:                                                      # strided indices; on the CPU, and what is no index, as index_select has it
+                rows = self.full(x).index_select(0, wanted)
         else:
             rows = self.full(x) if isinstance(x, (CanonStream, HyperStream)) else x
         lg = self.logits(rows, out_f32=out_f32, gather=gather_logits)
