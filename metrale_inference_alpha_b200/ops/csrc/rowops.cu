@@ -589,8 +589,11 @@ int mb_row_op(const MbRowArgs* a, cudaStream_t stream) {
       return launch_row_v2<1, true>(p, (nblk + 31) / 32 * 32, stream);
     if (modes && !p.xf32 && !p.residual && !p.residual_out && a->K % 16 == 0 && !(al & 15) && ld_ok &&
         (p.out_mode != OUT_FP8_G128 || a->K % 128 == 0) && nblk <= 4096) {
-      // a warp would take the row anyway; rows of more than a block a lane are faster over a CTA (2700 of 2048: 7.7 us, a warp each 13)
-      if (p.M >= 148 * 8 && nblk <= 32) return launch_row_v2<1, false, true>(p, 256, stream);
+      // A warp would take the row anyway; rows of more than a block a lane are faster over a CTA (2700 of 2048: 7.7 us, a warp each 13). A CTA /
+      // a warp each, us, 512 channels to nvfp4: copied 1300 rows 2.6 / 2.4, 2700 3.4 / 2.7, 8192 9.1 / 4.5; behind SiLU, twice the loads
+      // and an exponential a value, 1300 2.8 / 2.9 (fp8 groups 2.6 / 2.8), 2700 3.3 / 3.5, 8192 9.2 / 5.7.
+      const int many = 148 * (p.in_mode == IN_SILU_MUL ? 20 : 8);
+      if (p.M >= many && nblk <= 32) return launch_row_v2<1, false, true>(p, 256, stream);
       const int bpt = (nblk + 511) / 512;
       int threads = ((nblk + bpt - 1) / bpt + 31) / 32 * 32;
       if (p.out_mode == OUT_FP8_G128) threads = (threads + 7) / 8 * 8;
