@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "op_args.h"
 #include <cstdlib>
+#include <type_traits>
 
 namespace {
 
@@ -68,21 +69,21 @@ struct RowParams {
 
 // The row of x that output row m is made of. Taking rows of a table (the embedding, the rows that logits are wanted of) and
 // normalising them was a launch of its own in front of the norm's: 3.5 us at 1 to 128 tokens, 20 us at 8192 rows of 5120 (168 MB
-// that the norm then read again).
+// that the norm then read again). A kernel of its own: with the branches in the one of all rows those took 2 to 7 % longer.
 __device__ __forceinline__ long long source_row(const RowParams& p, int m, bool& live) {
-  live = true;
-  if (!p.gather) return m;
   const long long i = p.gather_wide ? reinterpret_cast<const long long*>(p.gather)[m] : reinterpret_cast<const int*>(p.gather)[m];
   live = i >= 0 && i < p.gather_rows;
   if (!live && p.status) atomicCAS(p.status, 0u, MB_ST_BOUNDS);
   return live ? i : 0;
 }
 
-__device__ __forceinline__ float load_x(const RowParams& p, long long m, int k) {
+template <typename Row>
+__device__ __forceinline__ float load_x(const RowParams& p, Row m, int k) {
   if (p.xf32) return p.xf32[(size_t)m * p.x_ld + k];
   return __bfloat162float(p.x[(size_t)m * p.x_ld + k]);
 }
 
+template <bool GATHER>
 __global__ void __launch_bounds__(512) row_kernel(const RowParams p) {
   extern __shared__ float row[];
   __shared__ float red[32];
@@ -96,11 +97,12 @@ __global__ void __launch_bounds__(512) row_kernel(const RowParams p) {
   // ---- stage 1: build the fp32 row
   if (p.in_mode == IN_RMSNORM) {
     float ss = 0.f;
-    bool live;
-    const long long from = source_row(p, m, live);
+    bool live = true;
+    std::conditional_t<GATHER, long long, int> from = m;
+    if constexpr (GATHER) from = source_row(p, m, live);
     for (int k = tid; k < K; k += nt) {
       float h = live ? load_x(p, from, k) : 0.f;
-      if (p.gather_out) p.gather_out[(size_t)m * K + k] = __float2bfloat16(h);
+      if (GATHER && p.gather_out) p.gather_out[(size_t)m * K + k] = __float2bfloat16(h);
       if (p.residual) {
         h += __bfloat162float(p.residual[(size_t)m * K + k]);
         h = __bfloat162float(__float2bfloat16(h));
@@ -253,7 +255,8 @@ __device__ __forceinline__ void load16(const __nv_bfloat16* src, float* v) {
 // in 2-byte pieces 2724 rows of 4096 behind a sigmoid gate took 56 us and of 2048 behind the gated norm 24, here 20 and 12.
 // WARP: a warp a row and eight rows a CTA, for many short rows: with a CTA a row an SM holds 32 of them however small they are
 // (24300 rows of 512 behind SiLU, a warp each: 26 us, so 15).
-template <int BPT, bool GATED, bool WARP>
+// GATHER: row m comes from row gather[m].
+template <int BPT, bool GATED, bool WARP, bool GATHER>
 __global__ void __launch_bounds__(WARP ? 256 : 1024) row_kernel_v2(const RowParams p) {
   __shared__ float red[64];
   const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, nt = WARP ? 32 : blockDim.x;
@@ -267,8 +270,9 @@ __global__ void __launch_bounds__(WARP ? 256 : 1024) row_kernel_v2(const RowPara
   float x[BPT][16];
   float ss = 0.f, mx = 0.f;
   const bool norm = p.in_mode == IN_RMSNORM;
-  bool live;
-  const long long from = source_row(p, m, live);
+  bool live = true;
+  std::conditional_t<GATHER, long long, int> from = m;
+  if constexpr (GATHER) from = source_row(p, m, live);
 #pragma unroll
   for (int j = 0; j < BPT; ++j) {
     const int b = tid + j * nt;
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(WARP ? 256 : 1024) row_kernel_v2(const RowPara
       uint4 v0 = __ldg(reinterpret_cast<const uint4*>(src));
       uint4 v1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
       if (!live) v0 = v1 = make_uint4(0, 0, 0, 0);
-      if (p.gather_out) {
+      if (GATHER && p.gather_out) {
         uint4* d = reinterpret_cast<uint4*>(p.gather_out + (size_t)m * K + b * 16);
         d[0] = v0; d[1] = v1;
       }
@@ -486,7 +490,10 @@ __global__ void __launch_bounds__(WARP ? 256 : 1024) row_kernel_v2(const RowPara
 
 template <int BPT, bool GATED = false, bool WARP = false>
 int launch_row_v2(const RowParams& p, int threads, cudaStream_t stream) {
-  return (int)mb::launch_kernel(row_kernel_v2<BPT, GATED, WARP>, dim3(WARP ? (p.M + 7) / 8 : p.M), dim3(threads), 0, stream, p);
+  const dim3 grid(WARP ? (p.M + 7) / 8 : p.M);
+  if constexpr (!GATED)
+    if (p.gather) return (int)mb::launch_kernel(row_kernel_v2<BPT, GATED, WARP, true>, grid, dim3(threads), 0, stream, p);
+  return (int)mb::launch_kernel(row_kernel_v2<BPT, GATED, WARP, false>, grid, dim3(threads), 0, stream, p);
 }
 
 // Repack row-major ue4m3 scale factors [N, K/16] into the tiled layout
@@ -609,13 +616,14 @@ int mb_row_op(const MbRowArgs* a, cudaStream_t stream) {
   const size_t smem = (size_t)a->K * sizeof(float);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         48 * 1024 * 4);
-    if (e != cudaSuccess) return (int)e;
+    for (auto kern : {row_kernel<false>, row_kernel<true>}) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024 * 4);
+      if (e != cudaSuccess) return (int)e;
+    }
     configured = true;
   }
   int threads = a->K >= 4096 ? 512 : (a->K >= 1024 ? 256 : 128);
-  return (int)mb::launch_kernel(row_kernel, dim3(a->M), dim3(threads), smem, stream, p);
+  return (int)mb::launch_kernel(p.gather ? row_kernel<true> : row_kernel<false>, dim3(a->M), dim3(threads), smem, stream, p);
 }
 
 int mb_sf_repack(const void* src, void* dst, int N, int kblocks, int sf_k64, cudaStream_t stream) {
