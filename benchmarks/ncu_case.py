@@ -7,6 +7,9 @@
     python benchmarks/ncu_case.py --op rowop  [--m 128 --k 5120]
     python benchmarks/ncu_case.py --op mla    [--m 64 --ctx 2048]
     python benchmarks/ncu_case.py --op kda_prefill [--ctx 4096]
+    python benchmarks/ncu_case.py --op prefill_attn256 [--ctx 4096]
+    python benchmarks/ncu_case.py --op gdn_prefill [--ctx 4096]
+    python benchmarks/ncu_case.py --op experts [--m 16]
 """
 import argparse
 import math
@@ -119,6 +122,40 @@ def main():
         b = ForwardBatch.build([dict(tokens=[1] * T, start_pos=0, blocks=list(range(1, T // 16 + 2)), state_slot=1)], 16, device=DEV)
         for _ in range(a.iters):
             rops.kda_recurrence(conv, g_raw, b_raw, A, dtb, -5.0, st, b, heads=H, dim=D, norm=(wn, gate, 1e-6))
+    elif a.op == "prefill_attn256":
+        # one sequence of --ctx query tokens over its own keys, 16 / 2 heads of 256, bf16 cache (csrc/attention_rows256.cu)
+        Hq, Hkv, D, bs, q = 16, 2, 256, 16, a.ctx
+        nblk = (q + bs - 1) // bs
+        kc, vc = (torch.randn(nblk + 1, bs, Hkv, D, device=DEV).to(torch.bfloat16) for _ in range(2))
+        bt = (torch.arange(nblk, device=DEV, dtype=torch.int32) + 1).view(1, nblk).contiguous()
+        qq = torch.randn(q, Hq, D, device=DEV).to(torch.bfloat16)
+        ql, qs = torch.tensor([q], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        for _ in range(a.iters):
+            ops.paged_attention(qq, kc, vc, bt, qs, ql, ql, max_q_len=q, max_ctx=q, scale=1 / math.sqrt(D))
+    elif a.op == "gdn_prefill":
+        # one sequence of --ctx tokens through the chunked gated delta rule, 16 key / 32 value heads x 128
+        from metrale_inference_alpha_b200.engine.batch import ForwardBatch
+        from metrale_inference_alpha_b200.ops import recurrent as rops
+        KH, VH, D, T = 16, 32, 128, a.ctx
+        conv, ba = torch.randn(T, (2 * KH + VH) * D, device=DEV), torch.randn(T, 2 * VH, device=DEV)
+        A, dtb = torch.zeros(VH, device=DEV), torch.zeros(VH, device=DEV)
+        st = torch.zeros(2, VH, D, D, device=DEV)
+        b = ForwardBatch.build([dict(tokens=[1] * T, start_pos=0, blocks=list(range(1, T // 16 + 2)), state_slot=1)], 16, device=DEV)
+        for _ in range(a.iters):
+            rops.gdn_recurrence(conv, ba, A, dtb, st, b, k_heads=KH, v_heads=VH, k_dim=D, v_dim=D)
+    elif a.op == "experts":
+        # --m tokens, each with 8 of 256 experts of 1024 x 2048 in fp8 blocks: sort, gather, grouped GEMM (csrc/moe.cu, gemm_few.cu)
+        from metrale_inference_alpha_b200.ops import moe_cuda
+        E, K, N, top = 256, 2048, 1024, 8
+        w = ops.QuantWeight("fp8_block", E * N, K, torch.randint(0, 0x7e, (E * N, K), dtype=torch.uint8, device=DEV),
+                            torch.rand(E * N // 128, K // 128, device=DEV))
+        x = ops.quantize_act(torch.randn(M, K, device=DEV).to(torch.bfloat16), "fp8_g128")
+        idx = torch.rand(M, E, device=DEV).topk(top, 1).indices.int().contiguous()
+        per = max(1, M * top // E)
+        rows = 16 if per <= 16 else 32 if per <= 32 else 64
+        for _ in range(a.iters):
+            sp = moe_cuda.SortedPairs(idx, 0, E, rows)
+            ops.linear(moe_cuda.gather_act(x, sp), w, out_f32=True, grouped=(sp.tile_expert, sp.tile_row0, sp.tile_nrows, N, sp.max_tiles, rows))
     elif a.op == "rowop":
         x = torch.randn(M, a.k, device=DEV).to(torch.bfloat16)
         w = torch.ones(a.k, device=DEV, dtype=torch.bfloat16)

@@ -909,7 +909,8 @@ def paged_attention(q: torch.Tensor, k_cache, v_cache, block_table, q_start, q_l
     these tokens' cache rows, and nothing before it in this call chain is still to be waited for: the decode kernel then starts on
     the older tokens under it. Caches [num_blocks, block, Hkv, D] bf16 or e4m3 bytes.
     `quant_out` > 0: return the output as an NVFP4 `Act` [T, Hq * D] quantised with that calibrated
-    global scale (inside the decode kernels and the plain head_dim 128 prefill kernel, else by a row kernel)."""
+    global scale (inside the decode kernels and the plain head_dim 128 prefill kernel, else by a row kernel; 17 to 32 query
+    rows of a group quantise the bf16 value inside the kernel, the bits that a row kernel gives)."""
     T, Hq, D = q.shape
     prefill = force_mode == 3 or (force_mode == 0 and _ATTN_TC and D in (128, 256) and window == 0 and max_q_len >= 128)
     if quant_out > 0.0:

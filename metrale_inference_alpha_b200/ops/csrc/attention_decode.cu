@@ -21,9 +21,9 @@
 //   bf16  8 rows 11.1, 39.1 / 11.4, 40.4;  10 rows 15.5, 47.0 / 12.5, 41.3;  20 rows 17.7, 105 / 17.4, 106;  32 rows 23.9, 144 / 19.8, 121
 // An e4m3 row is widened to f16 in registers, so with an e4m3 cache queries and weights are f16 as in attention.cu: a query element beyond
 // 65504 makes its row NaN, weights below 2^-24 of the running maximum vanish.
-// Measured against that kernel (us): e4m3, 40 / 8 heads of 128: one sequence of 700 tokens 22.5 -> 13.7, 128 of 129 to 1151 62 -> 50,
-// nine of 4000 to 16000 73 -> 54, eight verify steps of 4 rows 31 -> 22; bf16, 33 of 100 to 2047 57 -> 32; 16 / 2 heads of 256,
-// bf16, sixteen of 200 to 2000 119 -> 22.
+// Measured against that kernel (us, single calls replayed from a graph): e4m3, 40 / 8 heads of 128: one sequence of 700 tokens 15.4 -> 10.3,
+// 128 of 129 to 1151 70 -> 44, nine of 4000 to 16000 75 -> 48, eight verify steps of 4 rows 27 -> 17; bf16, 33 of 100 to 2047 95 -> 34;
+// 16 / 2 heads of 256, bf16, sixteen of 200 to 2000 63 -> 17.
 #include "common.cuh"
 #include "attention_decode.h"
 #include "tensormap.h"
@@ -662,12 +662,13 @@ int parts_of(int max_ctx, int part) {
 // cache's heads alone, so that a sequence's sums never depend on its batch; a tensor-parallel shard, which has fewer heads, cuts the
 // same sequence finer. Where the line lies, 512 / 1024 tokens, us (e4m3, five heads of 128 a group):
 //                                    8 kv heads     4              2              1
-//   1 sequence of 4000               13.3 / 17.3    12.9 / 17.0    12.7 / 16.8    12.4 / 16.4
-//   16 of 200 to 2000                17.7 / 20.7    14.6 / 18.0    12.8 / 17.4    12.4 / 17.2
-//   33 of 100 to 2047                29.6 / 25.8    17.8 / 20.6    14.6 / 17.8    12.7 / 17.2
-//   128 of 129 to 1151               61.3 / 49.1    36.9 / 32.3    25.2 / 19.2    15.1 / 16.0
-//   9 of 4000 to 16000               72.1 / 50.5    38.0 / 28.8    23.1 / 22.7    19.2 / 19.3
-// Twelve such batches together, time at 1024 over time at 512: e4m3 0.91, 1.01, 1.12, 1.19; bf16 0.95, 1.04, -, 1.26; two heads of 256 1.04.
+//   1 sequence of 4000               12.1 / 14.7    12.0 / 14.4    11.8 / 13.9    10.8 / 14.1
+//   16 of 200 to 2000                14.2 / 16.3    11.3 / 15.1    11.6 / 14.0    11.2 / 14.0
+//   33 of 100 to 2047                24.5 / 19.7    13.6 / 15.9    11.9 / 14.4    11.4 / 14.4
+//   128 of 129 to 1151               57.3 / 45.3    27.3 / 25.3    14.6 / 14.5    12.2 / 12.4
+//   9 of 4000 to 16000               70.5 / 49.8    28.9 / 21.4    18.3 / 17.5    17.0 / 16.9
+// Nine such batches together, time at 1024 over time at 512: e4m3 0.88, 1.03, 1.08, 1.13; bf16 0.97, 1.07, 1.13, 1.27; eight heads of 256 a
+// group e4m3 0.80, 0.88, 1.00, 1.02, bf16 0.81, 0.85, 0.96, 1.03.
 int part_tokens_of(const AttnDecodeArgs& a) { return ((a.part_tokens > 0 ? a.part_tokens : a.Hkv >= 8 ? 1024 : 512) + 63) & ~63; }
 
 struct Layout {
@@ -678,8 +679,9 @@ struct Layout {
 };
 // Shared memory of a launch. What lies beside the ring grows with the rows (the merge buffer, the queries) and with the batch (the
 // list of units), so it may leave room for fewer CTAs than the registers do: the grid has as many as are resident, since the
-// units are shared out over it evenly and CTAs beyond would start on theirs when the others are done (e4m3, 40 / 8 heads, 512 sequences
-// of 100 to 1000 tokens 229 -> 172 us, the split-KV kernel 207; bf16, 16 / 2 heads, 1024 of 60 to 700 136 -> 112; 32 rows 225 -> 219).
+// units are shared out over it evenly and CTAs beyond would start on theirs when the others are done (with all products in the queries'
+// order: e4m3, 40 / 8 heads, 512 sequences of 100 to 1000 tokens 229 -> 172 us, 32 rows 225 -> 219; the former takes 139 now, the split-KV
+// kernel 204).
 template <int D, bool FP8, int NT>
 Layout layout(int rows, int num_seqs, int slots = 2) {
   using C = DecodeCfg<D, FP8, NT>;

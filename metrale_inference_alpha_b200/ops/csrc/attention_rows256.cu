@@ -11,6 +11,8 @@
 // The output is rescaled in TMEM only when a row's maximum has moved by more than 2^8, and then waits for the product before.
 //
 // Bounds: per 64 tokens the two products are 1024 cycles of the tensor cores, 8192 exponentials 512 of the special function units.
+// Measured against attention_tc.cu (us, 16 / 2 heads): one prompt of 128 tokens 21 -> 10, three of 500 to 1300 233 -> 54, 64 of 128 153 -> 71, one
+// of 4096 661 -> 204, 256 tokens behind 4000 281 -> 110.
 #include "common.cuh"
 #include "attention_rows.cuh"
 #include "attention_rows.h"

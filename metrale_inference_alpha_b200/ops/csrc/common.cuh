@@ -294,10 +294,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------- programmatic dependent launch
-// Every kernel of the library starts with pdl_wait() before its first global-memory access
-// and may be launched with the programmatic-stream-serialization attribute (launch_kernel
-// below): the next kernel's CTAs are then scheduled, and run their global-memory-free set-up
-// (barrier init, TMEM alloc, descriptor prefetch), while the previous kernel drains.
+// Every kernel that may be launched with the programmatic-stream-serialization attribute (launch_kernel
+// below) calls pdl_wait() before it touches what preceding kernels of the step write: its CTAs are then
+// scheduled, and run their set-up (barrier init, TMEM alloc, descriptor prefetch), while the previous kernel
+// drains. What stood before the step began may be read in front of the wait: weights (the GEMMs), positions, slots and
+// rotary tables (the rotation), sequence lengths, block tables and older tokens' cache rows (decode attention).
+// What a preceding kernel writes, a kernel that comes up under it reads with ordinary loads: __ldg asks for data that nobody writes while
+// the kernel is up. (The GEMMs but gemm_few.cu still read activations' scales with it, behind the wait.)
 // pdl_wait() returns once the previous grid has completed and its writes are visible; it is
 // a no-op for a kernel launched without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -543,8 +546,9 @@ inline cudaError_t launch_kernel_ex(void (*kern)(KArgs...), dim3 grid, dim3 bloc
   cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
-// METRALE_PDL: 0 = plain launches, 1 = every kernel launches programmatically, 2 (default) = only
-// the GEMMs, whose prologue and first ring of weight tiles then overlap the preceding kernel
+// METRALE_PDL: 0 = plain launches, 1 = every kernel launches programmatically, 2 (default) = the GEMMs, whose prologue and
+// first ring of weight tiles then overlap the preceding kernel, and, where their callers say that the launches in front allow
+// it (`early`), the rotation of up to 512 tokens and decode attention
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                          cudaStream_t stream, int cluster_z, Args&&... args) {

@@ -17,11 +17,11 @@
 //
 // gemm_block_kernel (fp8 with 128 x 128 weight scales, also over the work list of grouped experts): one CTA per tile of
 // 128 tokens x 128 or 256 features. Every 128-deep k block lands in one of four or two TMEM accumulators and is added to registers
-// with its scale, which is one number per thread here (the token's scale times the weight block's). Small work-list entries
-// load boxes of their own 16 to 64 rows: the rest of the tile's rows are whatever was there, and are not stored.
+// with its scale, which is one number per thread here (the token's scale times the weight block's). Work lists of entries of 16 to
+// 64 rows are gemm_few.cu's; only where a residual joins the result do they come here, in boxes of their own rows: the rest of the
+// tile's rows are whatever was there, and are not stored.
 // Measured (2724 tokens x 8 of 256 experts and a shared one; before = 64-token tiles as the UMMA "B" operand): 1024 x 2048 per
-// expert 500 -> 134 us (167 at 128 features a tile), 2048 x 512 417 -> 122 us (144), plain 8192 x 2048 237 -> 64 us (82); 16
-// tokens (rows of 16): 52 -> 49, 48 -> 37 us.
+// expert 500 -> 134 us (167 at 128 features a tile), 2048 x 512 417 -> 122 us (144), plain 8192 x 2048 237 -> 64 us (82).
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "gemm_rows.h"

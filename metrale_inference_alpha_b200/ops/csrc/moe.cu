@@ -171,7 +171,7 @@ route_kernel(const float* __restrict__ logits, long long ld, int T, int E, int K
   }
 }
 
-// ------------------------------------------------------------------ sort (single CTA)
+// ------------------------------------------------------------------ sort (one CTA, or a cluster of eight)
 // pairs = T * K. counts / offsets in shared memory; rows of one expert are independent, so their
 // order inside the expert's range is free. With align > 1 every *tile* starts at a multiple of `align`
 // rows and holds at most tile_rows (<= align) pairs in its first rows (NVFP4 operands carry their scale
